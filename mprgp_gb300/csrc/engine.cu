@@ -1045,13 +1045,210 @@ __device__ double ratio_v(const InstDesc &D, const VCons &C, const double x[3], 
   return r;
 }
 
+// ------------------------------------------- separable vertex constraints --
+// A vertex whose planes all have coordinate-axis normals, each on another
+// axis (floor and walls: nearly every vertex of a body in a box), constrains
+// each coordinate by itself.  Its projector, PHI, BETA, preconditioner and
+// feasibility test then work coordinate by coordinate on three offsets and two
+// bit masks, where VCons with its nine normal components and the support
+// enumeration of the small QPs does not fit the kernels' registers (64 in the
+// engine, 40 in the cluster solver: the candidate phase spilled 1.7 and 4.3 KB
+// a thread).  What a vertex away from contact needs no FP64 work for -- the
+// projection of a feasible point, BETA and the face terms of a vertex with no
+// active plane -- is skipped: GB300 issues an FP64 warp instruction every 64
+// clocks or so per scheduler, so the candidate phase is bound by their number
+// and, before this form, by the spills.  The candidate phase measured 94.3 ->
+// 64.1 us on 348,145 vertices (rows 78 -> 49), 54 -> 34.5 us on 140,481 and
+// 20.4 -> 12.2 us in the cluster solver on 1,760 (mixed).  Every value equals the general path's (a skipped term is an exact
+// zero there, or leaves a finite operand unchanged; operands that are not
+// finite take the terms); only the sign of an exact zero can differ.
+struct VSep {
+  int k, base, axes;  // planes; 2 bits per plane: its coordinate
+  int mask, act;      // coordinates with a plane, and with a plane on the face
+  double c[3];        // x_d >= c_d for d in mask
+};
+
+__device__ __forceinline__ bool finite_bits(double v) {
+  return (__double2hiint(v) & 0x7ff00000) != 0x7ff00000;
+}
+__device__ __forceinline__ bool finite3(const double v[3]) {
+  return finite_bits(v[0]) && finite_bits(v[1]) && finite_bits(v[2]);
+}
+
+// Loads a vertex's constraints in the separable form; false when they do not
+// have it (bounds, a normal off the axes, two planes on one axis).
+__device__ __forceinline__ bool load_cons(const InstDesc &D, int v, VSep &C) {
+  if (D.kind < KIND_DECOUPLED || !D.pl_axis) return false;
+  int b = ldro(D.plane_ptr + v), e = ldro(D.plane_ptr + v + 1);
+  MPRGP_CHECK(b >= 0 && e >= b && e - b <= kMaxPlanes && e <= D.m, D.A.bad, 4, (b = 0, e = 0));
+  C.base = b;
+  C.k = e - b;
+  C.axes = C.mask = C.act = 0;
+  C.c[0] = C.c[1] = C.c[2] = 0.0;
+  bool axis = true;
+#pragma unroll
+  for (int j = 0; j < kMaxPlanes; ++j) {
+    if (j < C.k) {
+      const int a = (int)(__ldg(D.pl_axis + b + j) & 3);
+      const double c = ldro(D.planes + 4 * (size_t)(b + j) + 3);
+      axis &= a != 3;
+      C.axes |= a << (2 * j);
+      C.mask |= 1 << a;
+      if (a == 0) C.c[0] = c;
+      else if (a == 1) C.c[1] = c;
+      else C.c[2] = c;
+    }
+  }
+  return axis && __popc(C.mask) == C.k;
+}
+__device__ __forceinline__ int sep_axis(const VSep &C, int j) { return (C.axes >> (2 * j)) & 3; }
+
+// Reads the face codes into C.act; the returned value is C.act (the other
+// functions take it in place of the general form's packed codes).
+__device__ __forceinline__ int load_face(const InstDesc &D, VSep &C) {
+  C.act = 0;
+#pragma unroll
+  for (int j = 0; j < kMaxPlanes; ++j)
+    if (j < C.k && D.face[C.base + j]) C.act |= 1 << sep_axis(C, j);
+  return C.act;
+}
+__device__ __forceinline__ int decide_face(const InstDesc &D, VSep &C, const double x[3], int &f) {
+  f = 0;
+  int cnt = 0;
+#pragma unroll
+  for (int d = 0; d < 3; ++d)
+    if ((C.mask >> d) & 1 && fabs(x[d] - C.c[d]) < kEps) f |= 1 << d;
+#pragma unroll
+  for (int j = 0; j < kMaxPlanes; ++j) {
+    if (j < C.k) {
+      const int a = (f >> sep_axis(C, j)) & 1;
+      cnt += a;
+      D.face[C.base + j] = (unsigned char)a;
+    }
+  }
+  C.act = f;
+  return cnt;
+}
+// Whether some plane is violated, x_d < c_d (c_d - x_d > 0).
+__device__ __forceinline__ bool violated(const VSep &C, const double x[3]) {
+  bool viol = false;
+#pragma unroll
+  for (int d = 0; d < 3; ++d)
+    if ((C.mask >> d) & 1) viol |= x[d] < C.c[d];
+  return viol;
+}
+// max(q_d, 0) on the coordinates in `on`; the plane kind's QP over several
+// planes (unit_qp3) keeps q_d only above 1e-12 max|q|.
+__device__ __forceinline__ void sep_qp(const InstDesc &D, int on, const double q[3],
+                                       double lam[3]) {
+  double tol = 0.0;
+  if (D.kind == KIND_PLANES && __popc(on) >= 2) {
+    double scale = 1e-300;
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+      if ((on >> d) & 1) scale = fmax(scale, fabs(q[d]));
+    tol = 1e-12 * scale;
+  }
+#pragma unroll
+  for (int d = 0; d < 3; ++d) lam[d] = ((on >> d) & 1 && q[d] > tol) ? q[d] : 0.0;
+}
+__device__ __forceinline__ void project_violated(const InstDesc &D, const VSep &C,
+                                                 const double x[3], double y[3]) {
+  double q[3], lam[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) q[d] = C.c[d] - x[d];
+  sep_qp(D, C.mask, q, lam);
+#pragma unroll
+  for (int d = 0; d < 3; ++d) y[d] = x[d] + lam[d];
+}
+__device__ __forceinline__ void project_v(const InstDesc &D, const VSep &C, const double x[3],
+                                          double y[3]) {
+  y[0] = x[0];
+  y[1] = x[1];
+  y[2] = x[2];
+  if (violated(C, x)) project_violated(D, C, x, y);
+}
+__device__ __forceinline__ void phi_v(const InstDesc &, const VSep &, int f, const double g[3],
+                                      double phi[3]) {
+#pragma unroll
+  for (int d = 0; d < 3; ++d) phi[d] = (f >> d) & 1 ? g[d] + -g[d] : g[d];
+}
+__device__ __forceinline__ void beta_v(const InstDesc &D, const VSep &, int f, const double g[3],
+                                       const double phi[3], double beta[3]) {
+  beta[0] = beta[1] = beta[2] = 0.0;
+  if (!f && finite3(g)) return;  // g - phi = 0
+#pragma unroll
+  for (int d = 0; d < 3; ++d) beta[d] = g[d] - phi[d];
+  if (!f) return;
+  double lam[3];
+  sep_qp(D, f, beta, lam);
+#pragma unroll
+  for (int d = 0; d < 3; ++d) beta[d] -= lam[d];
+}
+__device__ __forceinline__ void precond_v(const InstDesc &D, const VSep &C, int f, int v,
+                                          const double g[3], const double phi[3], double z[3]) {
+  if (D.pre == PRE_NONE || (D.pre == PRE_DECOUPLE && D.m == 0)) {
+    z[0] = phi[0];
+    z[1] = phi[1];
+    z[2] = phi[2];
+    return;
+  }
+  double di[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) di[d] = ldro(D.dinv + 3 * (size_t)v + d);
+  if (D.pre == PRE_INFACE) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) z[d] = phi[d] * di[d];
+    return;
+  }
+#pragma unroll
+  for (int d = 0; d < 3; ++d) z[d] = di[d] * g[d];
+  if (!f && finite3(di)) return;  // t = 0
+  double t[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+  for (int j = 0; j < kMaxPlanes; ++j) {
+    if (j >= C.k) continue;
+    const int a = sep_axis(C, j);
+    if (!((f >> a) & 1)) continue;
+    const double in = ldro(D.pl_indn + C.base + j);
+    if (a == 0) t[0] = in * z[0];
+    else if (a == 1) t[1] = in * z[1];
+    else t[2] = in * z[2];
+  }
+#pragma unroll
+  for (int d = 0; d < 3; ++d) z[d] = fma(-di[d], t[d], z[d]);
+}
+__device__ __forceinline__ double phitphi_v(const InstDesc &D, const VSep &C, double abar,
+                                            const double x[3], const double phi[3]) {
+  const double xa[3] = {x[0] - abar * phi[0], x[1] - abar * phi[1], x[2] - abar * phi[2]};
+  double px[3];
+  project_v(D, C, xa, px);
+  return (x[0] - px[0]) * phi[0] + (x[1] - px[1]) * phi[1] + (x[2] - px[2]) * phi[2];
+}
+__device__ __forceinline__ int infeasible_v(const InstDesc &, const VSep &C, const double y[3]) {
+  int bad = 0;
+#pragma unroll
+  for (int d = 0; d < 3; ++d)
+    if ((C.mask >> d) & 1 && y[d] < C.c[d] - kEps) bad = 1;
+  return bad;
+}
+__device__ __forceinline__ double ratio_v(const InstDesc &, const VSep &C, const double x[3],
+                                          const double p[3]) {
+  double r = DBL_MAX;
+#pragma unroll
+  for (int d = 0; d < 3; ++d)
+    if ((C.mask >> d) & 1 && p[d] > kEps && x[d] > C.c[d]) r = fmin(r, (x[d] - C.c[d]) / p[d]);
+  return r;
+}
+
 __device__ __forceinline__ double *B(const InstDesc &D, int i) { return D.buf[i]; }
 
 // Shared epilogue once g is final for a row and the face is re-decided:
 // DECIDE_FACE(x); PHI(g); z = precond; p = z; then the loop top's BETA and
 // the sums |phi+beta|^2, beta.beta, PHITPHI, z.g, COUNT_CONSTRAINTS.
-__device__ void epilogue_full(const InstDesc &D, const InstState &S, const VCons &C, int v,
-                              const double x[3], const double g[3], double *part) {
+template <typename Cons>
+__device__ __forceinline__ void epilogue_full(const InstDesc &D, const InstState &S, Cons &C, int v,
+                                              const double x[3], const double g[3], double *part) {
   int f;
   const int act = decide_face(D, C, x, f);
   double phi[3], z[3], beta[3];
@@ -1072,6 +1269,27 @@ __device__ void epilogue_full(const InstDesc &D, const InstState &S, const VCons
   part[2] += phitphi_v(D, C, S.alpha_bar, x, phi);
   part[3] += dot3(z, g);
   part[4] += (double)act;
+}
+// The general form on the x and g in the vectors (kept out of line: its
+// registers do not press on the callers' matrix passes).
+__device__ __noinline__ void epilogue_general(const InstDesc &D, const InstState &S, int v,
+                                              double *part) {
+  VCons C;
+  load_cons(D, v, C);
+  double x[3], g[3];
+  ld3(B(D, B_X0 + S.xc), v, x);
+  ld3(B(D, B_G0 + S.gc), v, g);
+  epilogue_full(D, S, C, v, x, g, part);
+}
+__device__ __forceinline__ void epilogue(const InstDesc &D, const InstState &S, int v,
+                                         const double x[3], const double g[3], double *part) {
+  VSep C;
+  if (load_cons(D, v, C)) {
+    epilogue_full(D, S, C, v, x, g, part);
+  } else {
+    st3(B(D, B_G0 + S.gc), v, g);
+    epilogue_general(D, S, v, part);
+  }
 }
 
 // ------------------------------------------------------------- row work --
@@ -1209,15 +1427,31 @@ __device__ __noinline__ void row_power(const InstDesc &D, const InstState &S, in
   row_power64_fin(D, S, v, w, part);
 }
 
-__device__ __noinline__ void row_init(const InstDesc &D, const InstState &S, int v, int slot,
-                                      double *part) {
+// x = P(x) for one row, from x buffer `xin` to `xout`, in the general form.
+__device__ __noinline__ void row_project_general(const InstDesc &D, int xin, int xout, int v) {
   VCons C;
   load_cons(D, v, C);
-  if (S.phase == PH_PROJ0 || S.phase == PH_FINAL) {
+  double x[3], y[3];
+  ld3(B(D, xin), v, x);
+  project_v(D, C, x, y);
+  st3(B(D, xout), v, y);
+}
+__device__ __forceinline__ void row_project(const InstDesc &D, int xin, int xout, int v) {
+  VSep C;
+  if (load_cons(D, v, C)) {
     double x[3], y[3];
-    ld3(B(D, B_X0 + S.xc), v, x);
+    ld3(B(D, xin), v, x);
     project_v(D, C, x, y);
-    st3(B(D, B_X0 + S.xc), v, y);
+    st3(B(D, xout), v, y);
+  } else {
+    row_project_general(D, xin, xout, v);
+  }
+}
+
+__device__ __noinline__ void row_init(const InstDesc &D, const InstState &S, int v, int slot,
+                                      double *part) {
+  if (S.phase == PH_PROJ0 || S.phase == PH_FINAL) {
+    row_project(D, B_X0 + S.xc, B_X0 + S.xc, v);
     return;
   }
   // PH_INIT, PH_EXP_C, PH_PL_EXP_B: g = A x - b, then the full epilogue.
@@ -1235,11 +1469,11 @@ __device__ __noinline__ void row_init(const InstDesc &D, const InstState &S, int
     st3(D.ev, v, t);
   }
   double x[3], ax[3];
-  ld3(B(D, B_X0 + S.xc), v, x);
   spmv_row<double>(D.A, D.A.v64, slot, SrcV{B(D, B_X0 + S.xc)}, ax);
+  ld3(B(D, B_X0 + S.xc), v, x);
   const double g[3] = {ax[0] - ldro(D.b + 3 * (size_t)v), ax[1] - ldro(D.b + 3 * (size_t)v + 1),
                        ax[2] - ldro(D.b + 3 * (size_t)v + 2)};
-  epilogue_full(D, S, C, v, x, g, part);
+  epilogue(D, S, v, x, g, part);
 }
 
 __device__ __noinline__ void row_cg_spmv(const InstDesc &D, const InstState &S, int v, int slot,
@@ -1284,18 +1518,25 @@ __device__ __noinline__ void row_cg_spmv(const InstDesc &D, const InstState &S, 
   part[0] += dot3(p, ap);
   part[1] += dot3(p, g);
   if (S.phase == PH_PL_SPMV) {
-    VCons C;
-    load_cons(D, v, C);
     double x[3];
     ld3(B(D, B_X0 + S.xc), v, x);
-    part[kMinSlot] = fmin(part[kMinSlot], ratio_v(D, C, x, p));
+    VSep C;
+    if (load_cons(D, v, C)) {
+      part[kMinSlot] = fmin(part[kMinSlot], ratio_v(D, C, x, p));
+    } else {
+      VCons G;
+      load_cons(D, v, G);
+      part[kMinSlot] = fmin(part[kMinSlot], ratio_v(D, G, x, p));
+    }
   }
 }
 
 // Candidate y = x - alpha p: feasibility, the f(P(y)) correction terms and
 // the CG state that committing y would produce (CGMonotonicStep, :287-313).
-__device__ __noinline__ void row_cg_yf(const InstDesc &D, const InstState &S, int v, int slot,
-                                       double *part) {
+// The general form, and below it the separable one that nearly every vertex
+// takes.
+__device__ __noinline__ void cg_yf_general(const InstDesc &D, const InstState &S, int v,
+                                           double *part) {
   VCons C;
   load_cons(D, v, C);
   const int f = load_face(D, C);
@@ -1344,6 +1585,71 @@ __device__ __noinline__ void row_cg_yf(const InstDesc &D, const InstState &S, in
   part[7] += phitphi_v(D, C, S.alpha_bar, y, phi);
 }
 
+__device__ __noinline__ void row_cg_yf(const InstDesc &D, const InstState &S, int v, int slot,
+                                       double *part) {
+  (void)slot;
+  VSep C;
+  if (!load_cons(D, v, C)) {
+    cg_yf_general(D, S, v, part);
+    return;
+  }
+  const int f = load_face(D, C);
+  double ap[3], y[3], gy[3];
+  ld3(B(D, B_AP), v, ap);
+  {
+    double x[3], p[3], g[3];
+    ld3(B(D, B_X0 + S.xc), v, x);
+    ld3(B(D, B_P0 + S.pc), v, p);
+    ld3(B(D, B_G0 + S.gc), v, g);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      y[d] = x[d] - S.alpha * p[d];
+      gy[d] = g[d] - S.alpha * ap[d];
+    }
+  }
+  st3(B(D, B_X0 + (S.xc ^ 1)), v, y);
+  st3(B(D, B_G0 + (S.gc ^ 1)), v, gy);
+  double dl[3] = {0.0, 0.0, 0.0};
+  if (violated(C, y) || !finite3(y)) {
+    double py[3];
+    project_v(D, C, y, py);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) dl[d] = py[d] - y[d];
+    if (dl[0] != 0.0 || dl[1] != 0.0 || dl[2] != 0.0) {
+      double gt[3] = {gy[0], gy[1], gy[2]};
+      if (S.e_nz) {
+        double e[3];
+        ld3(B(D, B_E), v, e);
+        gt[0] += e[0];
+        gt[1] += e[1];
+        gt[2] += e[2];
+      }
+      part[0] += dot3(dl, gt);
+      part[1] += 1.0;
+    }
+    if (infeasible_v(D, C, y)) part[2] += 1.0;
+  }
+  st3(B(D, B_W), v, dl);
+  double phi[3], z[3];
+  phi_v(D, C, f, gy, phi);
+  precond_v(D, C, f, v, gy, phi, z);
+  st3(B(D, B_Z0 + (S.zc ^ 1)), v, z);
+  if (D.prec == PREC_MIXED) st3f(D.buf32[F_Z0 + (S.zc ^ 1)], v, z);
+  part[3] += dot3(z, ap);
+  part[4] += dot3(z, gy);
+  part[7] += phitphi_v(D, C, S.alpha_bar, y, phi);
+  double beta[3];
+  beta_v(D, C, f, gy, phi, beta);
+  st3(B(D, B_BT0 + (S.bc ^ 1)), v, beta);
+  if (f || !finite3(gy)) {
+    const double gp[3] = {phi[0] + beta[0], phi[1] + beta[1], phi[2] + beta[2]};
+    part[5] += dot3(gp, gp);
+    part[6] += dot3(beta, beta);
+  } else {  // beta = 0
+    part[5] += dot3(phi, phi);
+  }
+}
+
 // delta^T A delta over the rows where P(y) moved y (rare).
 __device__ __noinline__ void row_cg_dad(const InstDesc &D, const InstState &S, int v, int slot,
                                         double *part) {
@@ -1358,65 +1664,77 @@ __device__ __noinline__ void row_cg_dad(const InstDesc &D, const InstState &S, i
 
 // FP64 residual replacement for the mixed form: g = A64 x - b with the face
 // kept, then phi, z, beta and the sums for the current x.
-__device__ __noinline__ void row_ru(const InstDesc &D, const InstState &S, int v, int slot, double *part) {
-  VCons C;
-  load_cons(D, v, C);
+template <typename Cons>
+__device__ __forceinline__ void ru_epilogue(const InstDesc &D, const InstState &S, Cons &C, int v,
+                                            const double x[3], const double g[3], double *part) {
   const int f = load_face(D, C);
-  double x[3], ax[3], ap[3];
-  ld3(B(D, B_X0 + S.xc), v, x);
-  ld3(B(D, B_AP), v, ap);
-  spmv_row<double>(D.A, D.A.v64, slot, SrcV{B(D, B_X0 + S.xc)}, ax);
-  const double g[3] = {ax[0] - ldro(D.b + 3 * (size_t)v), ax[1] - ldro(D.b + 3 * (size_t)v + 1),
-                       ax[2] - ldro(D.b + 3 * (size_t)v + 2)};
-  double phi[3], z[3], beta[3];
+  double phi[3], z[3], beta[3], ap[3];
   phi_v(D, C, f, g, phi);
   precond_v(D, C, f, v, g, phi, z);
   beta_v(D, C, f, g, phi, beta);
-  st3(B(D, B_G0 + S.gc), v, g);
   st3(B(D, B_Z0 + S.zc), v, z);
   st3f(D.buf32[F_Z0 + S.zc], v, z);  // residual replacement runs in the mixed form only
   st3(B(D, B_BT0 + S.bc), v, beta);
   const double gp[3] = {phi[0] + beta[0], phi[1] + beta[1], phi[2] + beta[2]};
+  ld3(B(D, B_AP), v, ap);
   part[0] += dot3(gp, gp);
   part[1] += dot3(beta, beta);
   part[2] += phitphi_v(D, C, S.alpha_bar, x, phi);
   part[3] += dot3(z, g);
   part[4] += dot3(z, ap);
 }
-
-__device__ __noinline__ void row_exp(const InstDesc &D, const InstState &S, int v, int slot, double *part) {
+__device__ __noinline__ void ru_general(const InstDesc &D, const InstState &S, int v,
+                                        double *part) {
   VCons C;
   load_cons(D, v, C);
-  if (S.phase == PH_EXP_A) {  // y = P(x)
-    double x[3], y[3];
+  double x[3], g[3];
+  ld3(B(D, B_X0 + S.xc), v, x);
+  ld3(B(D, B_G0 + S.gc), v, g);
+  ru_epilogue(D, S, C, v, x, g, part);
+}
+__device__ __noinline__ void row_ru(const InstDesc &D, const InstState &S, int v, int slot, double *part) {
+  double x[3], ax[3];
+  spmv_row<double>(D.A, D.A.v64, slot, SrcV{B(D, B_X0 + S.xc)}, ax);
+  const double g[3] = {ax[0] - ldro(D.b + 3 * (size_t)v), ax[1] - ldro(D.b + 3 * (size_t)v + 1),
+                       ax[2] - ldro(D.b + 3 * (size_t)v + 2)};
+  st3(B(D, B_G0 + S.gc), v, g);
+  VSep C;
+  if (load_cons(D, v, C)) {
     ld3(B(D, B_X0 + S.xc), v, x);
-    project_v(D, C, x, y);
-    st3(B(D, B_X0 + (S.xc ^ 1)), v, y);
-    return;
+    ru_epilogue(D, S, C, v, x, g, part);
+  } else {
+    ru_general(D, S, v, part);
   }
-  if (S.phase == PH_EXP_B) {  // g = A y - b; DECIDE_FACE(y); PHI; x = P(y - abar phi)
-    const double *yb = B(D, B_X0 + (S.xc ^ 1));
-    double y[3], ay[3];
-    ld3(yb, v, y);
-    spmv_row<double>(D.A, D.A.v64, slot, SrcV{yb}, ay);
-    const double g[3] = {ay[0] - ldro(D.b + 3 * (size_t)v),
-                         ay[1] - ldro(D.b + 3 * (size_t)v + 1),
-                         ay[2] - ldro(D.b + 3 * (size_t)v + 2)};
-    st3(B(D, B_G0 + S.gc), v, g);
-    int f;
-    decide_face(D, C, y, f);
-    double phi[3];
-    phi_v(D, C, f, g, phi);
-    const double yn[3] = {y[0] - S.alpha_bar * phi[0], y[1] - S.alpha_bar * phi[1],
-                          y[2] - S.alpha_bar * phi[2]};
-    part[0] += (double)infeasible_v(D, C, yn);
-    double x[3];
-    project_v(D, C, yn, x);
-    st3(B(D, B_X0 + S.xc), v, x);
-    return;
-  }
-  // PH_PL_EXP_A (ExpStep, :196-218): xt = x - af p; g -= af AP;
-  // DECIDE_FACE(xt); PHI(g); x = P(xt - abar phi).
+}
+
+// The rows' work after g in PH_EXP_B: DECIDE_FACE(y); PHI; x = P(y - abar phi).
+template <typename Cons>
+__device__ __forceinline__ void exp_b_tail(const InstDesc &D, const InstState &S, Cons &C, int v,
+                                           const double y[3], const double g[3], double *part) {
+  int f;
+  decide_face(D, C, y, f);
+  double phi[3];
+  phi_v(D, C, f, g, phi);
+  const double yn[3] = {y[0] - S.alpha_bar * phi[0], y[1] - S.alpha_bar * phi[1],
+                        y[2] - S.alpha_bar * phi[2]};
+  part[0] += (double)infeasible_v(D, C, yn);
+  double x[3];
+  project_v(D, C, yn, x);
+  st3(B(D, B_X0 + S.xc), v, x);
+}
+__device__ __noinline__ void exp_b_general(const InstDesc &D, const InstState &S, int v,
+                                           double *part) {
+  VCons C;
+  load_cons(D, v, C);
+  double y[3], g[3];
+  ld3(B(D, B_X0 + (S.xc ^ 1)), v, y);
+  ld3(B(D, B_G0 + S.gc), v, g);
+  exp_b_tail(D, S, C, v, y, g, part);
+}
+// PH_PL_EXP_A (ExpStep, :196-218): xt = x - af p; g -= af AP;
+// DECIDE_FACE(xt); PHI(g); x = P(xt - abar phi).
+template <typename Cons>
+__device__ __forceinline__ void pl_exp_a(const InstDesc &D, const InstState &S, Cons &C, int v) {
   double x[3], p[3], ap[3], g[3];
   ld3(B(D, B_X0 + S.xc), v, x);
   ld3(B(D, B_P0 + S.pc), v, p);
@@ -1438,6 +1756,65 @@ __device__ __noinline__ void row_exp(const InstDesc &D, const InstState &S, int 
   double xn[3];
   project_v(D, C, xt, xn);
   st3(B(D, B_X0 + S.xc), v, xn);
+}
+__device__ __noinline__ void pl_exp_a_general(const InstDesc &D, const InstState &S, int v) {
+  VCons C;
+  load_cons(D, v, C);
+  pl_exp_a(D, S, C, v);
+}
+
+__device__ __noinline__ void row_exp(const InstDesc &D, const InstState &S, int v, int slot, double *part) {
+  if (S.phase == PH_EXP_A) {  // y = P(x)
+    row_project(D, B_X0 + S.xc, B_X0 + (S.xc ^ 1), v);
+    return;
+  }
+  VSep C;
+  if (S.phase == PH_EXP_B) {  // g = A y - b; DECIDE_FACE(y); PHI; x = P(y - abar phi)
+    const double *yb = B(D, B_X0 + (S.xc ^ 1));
+    double y[3], ay[3];
+    spmv_row<double>(D.A, D.A.v64, slot, SrcV{yb}, ay);
+    const double g[3] = {ay[0] - ldro(D.b + 3 * (size_t)v),
+                         ay[1] - ldro(D.b + 3 * (size_t)v + 1),
+                         ay[2] - ldro(D.b + 3 * (size_t)v + 2)};
+    st3(B(D, B_G0 + S.gc), v, g);
+    if (load_cons(D, v, C)) {
+      ld3(yb, v, y);
+      exp_b_tail(D, S, C, v, y, g, part);
+    } else {
+      exp_b_general(D, S, v, part);
+    }
+    return;
+  }
+  if (load_cons(D, v, C)) pl_exp_a(D, S, C, v);
+  else pl_exp_a_general(D, S, v);
+}
+
+// PH_PROP_B (PropStep, :219-243): x = P(x - alpha D); g -= alpha AD.
+template <typename Cons>
+__device__ __forceinline__ void prop_b(const InstDesc &D, const InstState &S, Cons &C, int v,
+                                       double *part) {
+  double x[3], dd[3], ad[3], g[3];
+  ld3(B(D, B_X0 + S.xc), v, x);
+  ld3(B(D, B_BT0 + S.bc), v, dd);
+  ld3(B(D, B_W), v, ad);
+  ld3(B(D, B_G0 + S.gc), v, g);
+  double xt[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    xt[d] = x[d] - S.alpha * dd[d];
+    g[d] -= S.alpha * ad[d];
+  }
+  double xn[3];
+  project_v(D, C, xt, xn);
+  if (xn[0] != xt[0] || xn[1] != xt[1] || xn[2] != xt[2]) part[5] += 1.0;
+  st3(B(D, B_X0 + S.xc), v, xn);
+  epilogue_full(D, S, C, v, xn, g, part);
+}
+__device__ __noinline__ void prop_b_general(const InstDesc &D, const InstState &S, int v,
+                                            double *part) {
+  VCons C;
+  load_cons(D, v, C);
+  prop_b(D, S, C, v, part);
 }
 
 __device__ __noinline__ void row_prop(const InstDesc &D, const InstState &S, int v, int slot,
@@ -1461,32 +1838,15 @@ __device__ __noinline__ void row_prop(const InstDesc &D, const InstState &S, int
     part[1] += dot3(dd, ad);
     return;
   }
-  // PH_PROP_B (PropStep, :219-243): x = P(x - alpha D); g -= alpha AD.
-  VCons C;
-  load_cons(D, v, C);
-  double x[3], dd[3], ad[3], g[3];
-  ld3(B(D, B_X0 + S.xc), v, x);
-  ld3(db, v, dd);
-  ld3(B(D, B_W), v, ad);
-  ld3(B(D, B_G0 + S.gc), v, g);
-  double xt[3];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    xt[d] = x[d] - S.alpha * dd[d];
-    g[d] -= S.alpha * ad[d];
-  }
-  double xn[3];
-  project_v(D, C, xt, xn);
-  if (xn[0] != xt[0] || xn[1] != xt[1] || xn[2] != xt[2]) part[5] += 1.0;
-  st3(B(D, B_X0 + S.xc), v, xn);
-  epilogue_full(D, S, C, v, xn, g, part);
+  VSep C;
+  if (load_cons(D, v, C)) prop_b(D, S, C, v, part);
+  else prop_b_general(D, S, v, part);
 }
 
-__device__ __noinline__ void row_pl_cg(const InstDesc &D, const InstState &S, int v, int slot,
-                                       double *part) {
-  // CGStep (:182-195) then the loop top's BETA and sums.
-  VCons C;
-  load_cons(D, v, C);
+// CGStep (:182-195) then the loop top's BETA and sums.
+template <typename Cons>
+__device__ __forceinline__ void pl_cg(const InstDesc &D, const InstState &S, Cons &C, int v,
+                                      double *part) {
   const int f = load_face(D, C);
   double x[3], p[3], ap[3], g[3];
   ld3(B(D, B_X0 + S.xc), v, x);
@@ -1512,6 +1872,19 @@ __device__ __noinline__ void row_pl_cg(const InstDesc &D, const InstState &S, in
   part[2] += phitphi_v(D, C, S.alpha_bar, x, phi);
   part[3] += dot3(z, g);
   part[5] += dot3(z, ap);
+}
+__device__ __noinline__ void pl_cg_general(const InstDesc &D, const InstState &S, int v,
+                                           double *part) {
+  VCons C;
+  load_cons(D, v, C);
+  pl_cg(D, S, C, v, part);
+}
+__device__ __noinline__ void row_pl_cg(const InstDesc &D, const InstState &S, int v, int slot,
+                                       double *part) {
+  (void)slot;
+  VSep C;
+  if (load_cons(D, v, C)) pl_cg(D, S, C, v, part);
+  else pl_cg_general(D, S, v, part);
 }
 
 __device__ void row_op(const InstDesc &D, const InstState &S, int v, int slot, double *part) {
