@@ -135,15 +135,17 @@ int mprgp_context_counters(mprgp_context *ctx, long long *launches, double *solv
  * (6 CTAs per SM);
  * bit 4 = 1 runs the large instances' phases as a CUDA-graph loop of
  * ordinary launches (one phase per launch) instead of the persistent
- * cooperative engine; bit 5 = 1 runs the power method as one persistent
- * cooperative launch (a grid barrier per phase, state kept on chip) in
- * synchronous runs whose items fit four per resident CTA, the graph loop
- * otherwise.  By default the power kernel runs as the power-step loop: no
- * launch finalizes its own phase -- every CTA of the next launch reduces the
- * item partials and advances its copy of the state with one extra warp while
- * its rows already form their products, and a settle kernel ends each graph
- * body; bit 6 = 1 runs the phase kernel instead, whose last CTA finalizes
- * each launch (bit 2 applies to both loops).  ctas_per_sm
+ * cooperative engine.  By default a synchronous run's power method is one
+ * launch whose CTAs are all resident and wait per instance: with the matrix
+ * slices in shared memory when they fit the SMs', else reading the matrix in
+ * every phase with up to two items a CTA (bit 5 = 1: four), and small
+ * instances with one cluster each (on server lanes too).  Other runs take the
+ * power-step loop: no launch finalizes its own phase -- every CTA of the next
+ * launch reduces the item partials and advances its copy of the state with one
+ * extra warp while its rows already form their products, and a settle kernel
+ * ends each graph body; bit 6 = 1 runs the phase kernel instead, whose last
+ * CTA finalizes each launch (bit 2 applies to both loops; with bits 1, 2 or 6
+ * small instances keep their power method in the cluster solver).  ctas_per_sm
  * caps the persistent grid (0 = every resident CTA).  Every setting gives
  * bitwise the same results. */
 int mprgp_context_set_tuning(mprgp_context *ctx, int stage, int ctas_per_sm);

@@ -9,14 +9,14 @@ the tuner checks that for the setting it picks.
                vertex rows; instances up to that many items take it)
   cluster_items  items per CTA allowed in the largest cluster (larger
                instances then also run as independent clusters)
-  power        the power method's loop: the power-step loop (each launch
-               advances the states the previous one left while its rows form
-               their products; CUDA-graph WHILE loop or plain stream
-               launches; the default), the phase kernel whose last CTA
-               finalizes each launch (graph or stream), phases of the
-               persistent engine, or one persistent cooperative launch of its
-               own (grid barrier per phase; synchronous runs whose items fit,
-               else the power-step graph loop)
+  power        the power method's loop: by default one launch of resident CTAs
+               that wait per instance where a run's items fit, else the
+               power-step loop (each launch advances the states the previous
+               one left while its rows form their products; CUDA-graph WHILE
+               loop); the power-step loop as plain stream launches; the phase
+               kernel whose last CTA finalizes each launch (graph or stream);
+               phases of the persistent engine; or the resident launch with up
+               to four items a CTA (by default two)
   power_regs   the phase kernel's register budget: 40 (6 CTAs per SM) or
                64 (4 CTAs per SM, more loads in flight per thread)
   engine       the large instances' MPRGP phases: the persistent cooperative

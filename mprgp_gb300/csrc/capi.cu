@@ -14,6 +14,7 @@
 #include <deque>
 #include <map>
 #include <string>
+#include <tuple>
 #include <utility>
 #include <vector>
 
@@ -28,9 +29,10 @@ cudaError_t launch_engine(const EngineArgs &args, int grid, cudaStream_t stream)
 cudaError_t build_power_graph(int grid, int variant, const EngineArgs *d_args, PowCtl *d_pc,
                               cudaGraph_t *graph, cudaGraphExec_t *exec);
 cudaError_t power_max_blocks_per_sm(int variant, int *n);
-cudaError_t launch_power_persistent(const EngineArgs &args, PowCtl *d_pc, int limit, int grid,
-                                    cudaStream_t stream);
-cudaError_t power_persistent_max_blocks_per_sm(int *n);
+cudaError_t launch_power_persistent(const SyncArgs &args, int fp32, int grid, cudaStream_t stream);
+cudaError_t power_persistent_max_blocks_per_sm(int fp32, int *n);
+cudaError_t launch_power_clusters(const SyncArgs &args, int fp32, int csize, cudaStream_t stream);
+cudaError_t power_clusters_max_active(int csize, int *n);
 cudaError_t launch_cluster(const ClusterArgs &args, int csize, cudaStream_t stream);
 cudaError_t cluster_max_active(int csize, int *n);
 cudaError_t launch_power_direct(int grid, int variant, int launches, const EngineArgs *d_args,
@@ -44,7 +46,10 @@ void launch_planes_setup(int nv, const int *plane_ptr, const double *in, double 
                          double *indn, const double *dinv, unsigned char *unit, cudaStream_t st);
 void launch_planes_axis(int m, const double *in, unsigned char *axis, cudaStream_t st);
 void launch_state_scatter(const InstDesc *desc, int n, InstState *states, InstState *const *home,
-                          const int *fresh, cudaStream_t st);
+                          const int *fresh, int clear_records, cudaStream_t st);
+cudaError_t power_sync_capacity(int q, int fp32, int smem, int nsm, int *ctas);
+cudaError_t launch_power_sync(const SyncArgs &args, int fp32, int grid, int smem,
+                              cudaStream_t stream);
 void launch_state_gather(const InstDesc *desc, int n, InstState *states, InstState *const *home,
                          cudaStream_t st);
 void launch_spmv(const SellMatrix &A, int nv, bool fp32, const double *x, double *y,
@@ -62,7 +67,9 @@ using namespace mprgp;
 struct LaneRun {
   bool active = false;
   int n = 0, n_large = 0, quantum = 0, cluster_quantum = 0, power_launches = 0;
-  bool power = false, power_graph = false, power_persistent = false, egraph = false;
+  bool power = false, power_graph = false, egraph = false;
+  bool power_sync = false;
+  int class_units[kClusterClasses] = {0, 0, 0, 0, 0};  // of the classes' power loops
   int power_variant = 0;  // the power loop's kernel variant (3: the power-step loop)
   int egraph_stream = 0;  // > 0: the engine loop ran as this many stream launches
   int class_n[kClusterClasses] = {0, 0, 0, 0, 0};
@@ -100,6 +107,8 @@ struct Lane {
   InstState **d_home = nullptr, **h_home = nullptr;
   int *d_fresh = nullptr, *h_fresh = nullptr;
   int *d_item_inst = nullptr, *h_item_inst = nullptr;  // items of the large instances
+  int ucap = 0;
+  SyncItem *d_unit = nullptr, *h_unit = nullptr;       // units of the power sync loop
   HostIO *io = nullptr;
   LaneRun run;
 };
@@ -141,16 +150,18 @@ struct mprgp_context {
   int bps_power_v[4] = {0, 0, 0, 0};  // per power-kernel variant (2: all phases, 3: power steps)
   int power_step = 1;    // power loop as the power-step loop (1, the default; deferred
                          // finalize) or the phase kernel with a finalize per launch (0)
-  int power_persistent = 0;  // power loop as one persistent cooperative launch when the run
-                            // is synchronous and its items fit (1)
+  int power_persistent = 0;  // the persistent power loop whenever its CTAs hold the items (1), or
+                            // up to two items a CTA (0); see persistent_plan
   int bps_power_pp = 0;      // resident CTAs per SM of that kernel
   int engine_graph = 0;  // large instances' phases as a graph loop of the phase kernel (1)
                          // or the persistent cooperative engine (0)
   int cluster = 16;      // largest cluster of the small-instance solver (0 = off)
   int cluster_items = 1; // items per CTA allowed in the largest cluster (1..kClusterItems)
   int cluster_ok[kClusterClasses] = {0, 0, 0, 0, 0};  // cluster sizes 1, 2, 4, 8, 16 usable
+  int power_cluster_ok[kClusterClasses] = {0, 0, 0, 0, 0};  // ... by the power loop's kernel
   int ctas_per_sm = 0;   // persistent CTAs per SM (0 = all resident)
   size_t l2_bytes = 0;   // the device's L2 size
+  std::map<std::tuple<int, int, int>, int> sync_cap;  // resident CTAs of the power sync loop's forms
   cudaMemPool_t pool = nullptr;      // every device array of the context's problems
   mprgp_problem *scratch = nullptr;
   int bps_power = 0;
@@ -194,6 +205,7 @@ struct mprgp_problem {
   size_t stage_nnzb = 0;
   std::vector<int> h_plane_ptr;
   std::vector<int> h_len;     // blocks per row of A
+  int max_len = 0;            // ... and the longest row's
   int *rowmap = nullptr;      // SELL row -> vertex (nullptr: identity)
   unsigned long long layout = 0;
   int want64 = 0, want32 = 0;
@@ -634,6 +646,7 @@ void lane_free(mprgp_context *c, Lane &L) {
   dfree(c, L.d_fresh);
   dfree(c, L.d_home);
   dfree(c, L.d_item_inst);
+  dfree(c, L.d_unit);
   cudaStreamSynchronize(c->stream);
   cudaFreeHost(L.h_desc);
   cudaFreeHost(L.h_prefix);
@@ -642,6 +655,7 @@ void lane_free(mprgp_context *c, Lane &L) {
   cudaFreeHost(L.h_fresh);
   cudaFreeHost(L.h_home);
   cudaFreeHost(L.h_item_inst);
+  cudaFreeHost(L.h_unit);
   cudaFreeHost(L.io);
   for (auto &kv : L.graphs) {
     cudaGraphExecDestroy(kv.second.second);
@@ -709,6 +723,76 @@ int lane_reserve(mprgp_context *c, Lane &L, int n, int items) {
   CK(cudaMallocHost((void **)&L.h_home, sizeof(InstState *) * cap));
   L.cap = cap;
   return MPRGP_OK;
+}
+
+// The same for the units of the power sync loop.
+int lane_reserve_units(mprgp_context *c, Lane &L, int units) {
+  if (units <= L.ucap) return MPRGP_OK;
+  const int ucap = std::max(1024, std::max(units, 2 * L.ucap));
+  dfree(c, L.d_unit);
+  cudaFreeHost(L.h_unit);
+  L.h_unit = nullptr;
+  L.ucap = 0;
+  const int rc = dalloc(c, &L.d_unit, ucap);
+  if (rc) return rc;
+  CK(cudaMallocHost((void **)&L.h_unit, sizeof(SyncItem) * ucap));
+  L.ucap = ucap;
+  return MPRGP_OK;
+}
+
+// How a synchronous run's power method is laid onto the GPU by the power sync
+// loop: q CTAs an item with their matrix slices in shared memory (smem bytes a
+// CTA), or (q == 0) the persistent loop, several items a CTA; grid == 0 when
+// neither applies.
+struct SyncPlan {
+  int q = 0, smem = 0, grid = 0;
+};
+int sync_capacity(mprgp_context *c, int q, int fp32, int smem) {
+  const auto key = std::make_tuple(q, fp32, smem);
+  auto it = c->sync_cap.find(key);
+  if (it == c->sync_cap.end()) {
+    int n = 0;
+    if (power_sync_capacity(q, fp32, smem, c->nsm, &n) != cudaSuccess) {
+      cudaGetLastError();
+      n = 0;
+    }
+    it = c->sync_cap.emplace(key, n).first;
+  }
+  return it->second;
+}
+SyncPlan sync_plan(mprgp_context *c, int units, int max_slots, int fp32) {
+  SyncPlan P;
+  // The fewest CTAs an item whose slices fit shared memory, or twice as many
+  // (three instead of two eighths of an SM's rows a CTA can pack an SM better).
+  // 1,760 vertices mixed: 4.85 us a phase with q = 1, 5.5 with 2, 4 or 8;
+  // 17,856 in FP64: 13.7 with q = 2, 14.2 with 4, 18.3 with 8.
+  const int slice = max_slots * kSlice * (9 * (fp32 ? 4 : 8) + 4);
+  int tried = 0;
+  for (int q = 1; q <= kThreads / kSlice && tried < 2; q *= 2) {
+    const long long bytes = (long long)slice * (kThreads / kSlice / q);
+    const long long smem = (bytes + 4095) / 4096 * 4096;  // few distinct sizes
+    if (smem > kSyncStageBytes) continue;
+    ++tried;
+    if (units * q > sync_capacity(c, q, fp32, (int)smem)) continue;
+    P.q = q;
+    P.smem = (int)smem;
+    P.grid = units * q;
+    break;
+  }
+  return P;
+}
+SyncPlan persistent_plan(mprgp_context *c, int units) {
+  SyncPlan P;
+  const int cap = c->nsm * c->bps_power_pp;
+  // Up to two items a CTA, unless the tuning asks for the persistent loop:
+  // a phase takes 15.8 us against 23.2 as graph launches at 549 items, 29.9
+  // against 31.1 at 833 (two a CTA), but 52.4 against 51.0 at 1,360 (three a
+  // CTA, streaming from DRAM, which more CTAs hide better).
+  if (cap > 0 && units <= cap * (c->power_persistent ? kPowOwn : 2)) {
+    const int per = (units + cap - 1) / cap;  // equally many items a CTA
+    P.grid = (units + per - 1) / per;
+  }
+  return P;
 }
 
 bool other_lanes_active(const mprgp_context *c, int k) {
@@ -891,10 +975,73 @@ int engine_begin(mprgp_context *c, int k, int n, mprgp_problem *const *probs,
     }
   }
   unsigned int in_power = 0;  // large instances in a power phase
-  for (int i = 0; i < n; ++i) {
-    const int ph = probs[i]->phase_host;
-    if (R.pos[i] < n_large)
-      in_power += (ph == PH_POW_RAND || ph == PH_POW || ph == PH_POW_LAST) ? 1u : 0u;
+  for (int i = 0; i < n; ++i)
+    if (R.pos[i] < n_large && engine_in_power(probs[i])) ++in_power;
+  // The power method in the forms whose CTAs wait for each other (unless the
+  // tuning asks for the launch loops): a synchronous run's instances, small
+  // ones too, by the power sync loop when all their CTAs are resident at once;
+  // else its large ones by the persistent loop; small ones, on every lane, by
+  // the persistent loop's kernel with one cluster an instance.
+  const bool waiting = power_launches > 0 && c->power_kernel && c->power_graph && c->power_step;
+  const bool alone = k == 0 && !other_lanes_active(c, k);
+  struct Count {
+    int units = 0, slots = 0, fp32 = 0, n = 0;
+    void add(const mprgp_problem *p, const InstDesc &D) {
+      units += nitems_of(p->nv);
+      slots = std::max(slots, p->max_len);
+      fp32 += D.prec == PREC_MIXED ? 1 : 0;
+      ++n;
+    }
+    bool one() const { return n > 0 && (fp32 == 0 || fp32 == n); }  // of one precision
+  } all, large, cl[kClusterClasses];
+  bool cl_fits[kClusterClasses] = {true, true, true, true, true};
+  for (int i = 0; i < n && waiting; ++i) {
+    if (!engine_in_power(probs[i])) continue;
+    const InstDesc &D = desc[R.pos[i]];
+    if (R.pos[i] < n_large) {
+      all.add(probs[i], D);
+      large.add(probs[i], D);
+    } else if (cluster_quantum == 0) {
+      all.add(probs[i], D);
+      cl[cls[i]].add(probs[i], D);
+      cl_fits[cls[i]] &= D.nitems <= (1 << cls[i]);
+    }
+  }
+  SyncPlan plan;
+  bool small_in_plan = false;
+  if (alone && all.one()) {
+    plan = sync_plan(c, all.units, all.slots, all.fp32 ? 1 : 0);
+    small_in_plan = plan.grid > 0;
+  }
+  if (alone && large.one() && plan.grid == 0) plan = persistent_plan(c, large.units);
+  R.power_sync = plan.grid > 0;
+  const Count &sync = small_in_plan ? all : large;
+  int nunits = 0, class_unit[kClusterClasses];
+  {
+    int want = R.power_sync ? sync.units : 0;
+    for (int q = 0; q < kClusterClasses; ++q) {
+      R.class_units[q] = (!small_in_plan && cl[q].one() && cl_fits[q] && c->power_cluster_ok[q])
+                             ? cl[q].n << q
+                             : 0;
+      want += R.class_units[q];
+    }
+    rc = lane_reserve_units(c, L, want);
+    if (rc) return rc;
+    if (R.power_sync)
+      for (int i = 0; i < n; ++i) {
+        if (!engine_in_power(probs[i]) || !(R.pos[i] < n_large || small_in_plan)) continue;
+        const int limit = R.pos[i] < n_large ? power_launches : INT_MAX;
+        for (int t = 0; t < nitems_of(probs[i]->nv); ++t) L.h_unit[nunits++] = {R.pos[i], t, limit, 0};
+      }
+    for (int q = 0; q < kClusterClasses; ++q) {
+      class_unit[q] = nunits;
+      if (!R.class_units[q]) continue;
+      for (int i = 0; i < n; ++i) {
+        if (cls[i] != q || !engine_in_power(probs[i])) continue;
+        const int ni = nitems_of(probs[i]->nv);
+        for (int t = 0; t < (1 << q); ++t) L.h_unit[nunits++] = {R.pos[i], t, t < ni ? INT_MAX : 0, 0};
+      }
+    }
   }
   cudaStream_t s = L.stream;
   if (s != c->stream) {  // the problems' uploads and setup kernels come first
@@ -911,7 +1058,9 @@ int engine_begin(mprgp_context *c, int k, int n, mprgp_problem *const *probs,
   if (large_items > 0)
     CK(cudaMemcpyAsync(L.d_item_inst, L.h_item_inst, sizeof(int) * large_items,
                        cudaMemcpyHostToDevice, s));
-  launch_state_scatter(L.d_desc, n, L.d_st, L.d_home, L.d_fresh, s);
+  if (nunits > 0)
+    CK(cudaMemcpyAsync(L.d_unit, L.h_unit, sizeof(SyncItem) * nunits, cudaMemcpyHostToDevice, s));
+  launch_state_scatter(L.d_desc, n, L.d_st, L.d_home, L.d_fresh, nunits > 0 ? 1 : 0, s);
   CK(cudaGetLastError());
   HostIO &io = *L.io;
   std::memset(&io.ctl_in, 0, sizeof(Ctl));
@@ -948,21 +1097,12 @@ int engine_begin(mprgp_context *c, int k, int n, mprgp_problem *const *probs,
   // The power method first (at most 1003 phases: the seeded start, 1001
   // iterations, the last difference), as a device-driven loop of launches of
   // the power kernel while any instance is in a power phase; then the engine.
-  R.power = c->power_kernel && in_power > 0 && power_launches > 0;
+  R.power = c->power_kernel && in_power > 0 && power_launches > 0 && !R.power_sync;
   cudaGraphExec_t pexec = nullptr;
   R.power_variant = c->power_step ? 3 : c->power_variant;
   const int pgrid = power_grid(c, prefix[n_large], R.power_variant);
-  // ... or as one persistent cooperative launch: only on lane 0 with no other
-  // lane in flight (its CTAs must all be resident) and when every CTA holds
-  // at most kPowOwn items
-  const int pp_cap = c->nsm * c->bps_power_pp;
-  R.power_persistent = R.power && c->power_persistent && k == 0 && !other_lanes_active(c, k) &&
-                       pp_cap > 0 && prefix[n_large] <= pp_cap * kPowOwn;
-  // equally many items per CTA (the phase waits for the busiest CTA)
-  const int pp_per = pp_cap > 0 ? (prefix[n_large] + pp_cap - 1) / pp_cap : 1;
-  const int pp_grid = std::max(1, (prefix[n_large] + pp_per - 1) / std::max(1, pp_per));
   if (R.power) {
-    if (c->power_graph && !R.power_persistent) {
+    if (c->power_graph) {
       rc = power_graph(L, pgrid, R.power_variant, &pexec);
       if (rc) return rc;
     }
@@ -993,9 +1133,24 @@ int engine_begin(mprgp_context *c, int k, int n, mprgp_problem *const *probs,
   if (R.power || R.egraph)
     CK(cudaMemcpyAsync(L.d_args, &args, sizeof(EngineArgs), cudaMemcpyHostToDevice, s));
   CK(cudaEventRecord(L.e0, s));
+  SyncArgs sa;
+  std::memset(&sa, 0, sizeof(sa));
+  sa.desc = L.d_desc;
+  sa.states = L.d_st;
+  sa.wait_ns = args.wait_ns;
+  sa.ctl = L.ctl;
   // The cluster-size classes run on side streams, concurrently with each
   // other and with the power loop; the engine starts once they are done.
-  if (n - n_large > 0) CK(cudaEventRecord(L.fork_ev, s));
+  if (n - n_large > 0 && !small_in_plan) CK(cudaEventRecord(L.fork_ev, s));
+  if (R.power_sync) {
+    sa.items = L.d_unit;
+    sa.units = sync.units;
+    sa.q = std::max(1, plan.q);
+    if (plan.q > 0) CK(launch_power_sync(sa, sync.fp32 ? 1 : 0, plan.grid, plan.smem, s));
+    else CK(launch_power_persistent(sa, sync.fp32 ? 1 : 0, plan.grid, s));
+    CK(cudaEventRecord(L.e_pow, s));
+  }
+  if (n - n_large > 0 && small_in_plan) CK(cudaEventRecord(L.fork_ev, s));
   for (int q = 0; q < kClusterClasses; ++q) {
     if (!R.class_n[q]) continue;
     ClusterArgs cargs;
@@ -1005,15 +1160,19 @@ int engine_begin(mprgp_context *c, int k, int n, mprgp_problem *const *probs,
         cluster_quantum > 0 ? std::min<long long>(phase_bound, cluster_quantum) : phase_bound,
         INT_MAX);
     CK(cudaStreamWaitEvent(L.side[q], L.fork_ev, 0));
+    if (R.class_units[q]) {
+      sa.items = L.d_unit + class_unit[q];
+      sa.units = R.class_units[q];
+      sa.q = 1;
+      CK(launch_power_clusters(sa, cl[q].fp32 ? 1 : 0, 1 << q, L.side[q]));
+    }
     CK(launch_cluster(cargs, 1 << q, L.side[q]));
     CK(cudaEventRecord(L.join_ev[q], L.side[q]));
   }
-  if (R.power && R.power_persistent)
-    CK(launch_power_persistent(args, L.d_pc, power_launches, pp_grid, s));
-  else if (R.power && pexec) CK(cudaGraphLaunch(pexec, s));
+  if (R.power && pexec) CK(cudaGraphLaunch(pexec, s));
   else if (R.power)
     CK(launch_power_direct(pgrid, R.power_variant, power_launches, L.d_args, L.d_pc, s));
-  CK(cudaEventRecord(L.e_pow, s));  // the lane stream's power loop ends here
+  if (!R.power_sync) CK(cudaEventRecord(L.e_pow, s));  // the lane stream's power loop ends here
   for (int q = 0; q < kClusterClasses; ++q)
     if (R.class_n[q]) CK(cudaStreamWaitEvent(s, L.join_ev[q], 0));
   if (R.egraph && R.egraph_stream)
@@ -1079,13 +1238,13 @@ int engine_end(mprgp_context *c, int k, mprgp_stats *stats, int *done) {
   const HostIO &io = *L.io;
   float ms = 0.f, pms = 0.f;
   CK(cudaEventElapsedTime(&ms, L.e0, L.e1));
-  if (R.power) CK(cudaEventElapsedTime(&pms, L.e0, L.e_pow));
+  if (R.power || R.power_sync) CK(cudaEventElapsedTime(&pms, L.e0, L.e_pow));
   c->power_ms += pms;
   // every body of a loop graph issues kPowerUnroll launches, the stream form
   // all `power_launches` (those after the last working one return at once)
   // (the power-step loop adds its settle kernel to every body)
   const long long body = kPowerUnroll + (R.power_variant == 3 ? 1 : 0);
-  if (R.power && R.power_persistent)
+  if (R.power_sync)
     c->launches += 1;
   else if (R.power && R.power_graph)
     c->launches += body * ((io.pc_out[0].launches + kPowerUnroll - 1) / kPowerUnroll);
@@ -1093,7 +1252,8 @@ int engine_end(mprgp_context *c, int k, mprgp_stats *stats, int *done) {
     c->launches += body * ((R.power_launches + kPowerUnroll - 1) / kPowerUnroll);
   else if (R.power)
     c->launches += R.power_launches;
-  for (int q = 0; q < kClusterClasses; ++q) c->launches += R.class_n[q] ? 1 : 0;
+  for (int q = 0; q < kClusterClasses; ++q)
+    c->launches += (R.class_n[q] ? 1 : 0) + (R.class_units[q] ? 1 : 0);
   if (R.egraph && R.egraph_stream)
     c->launches += R.egraph_stream;
   else if (R.egraph)
@@ -1104,6 +1264,8 @@ int engine_end(mprgp_context *c, int k, mprgp_stats *stats, int *done) {
   c->solver_ms += ms;
   const Ctl &ctl1 = io.ctl_out;
   int worst = MPRGP_OK;
+  bool small_power = false;  // small instances' power loops share the error word
+  for (int q = 0; q < kClusterClasses; ++q) small_power |= R.class_units[q] > 0;
   for (int i = 0; i < n; ++i) {
     mprgp_problem *p = R.probs[i];
     InstState x = L.h_st_out[R.pos[i]];
@@ -1112,7 +1274,7 @@ int engine_end(mprgp_context *c, int k, mprgp_stats *stats, int *done) {
     const bool large = R.pos[i] < n_large;
     // an engine error concerns the engine's instances; an instance left
     // unfinished by a run that had no phase limit hit the hard phase bound
-    const bool err = large && ctl1.err;
+    const bool err = (large || R.power_sync || small_power) && ctl1.err;
     const bool unbounded = (large ? R.quantum : R.cluster_quantum) == 0;
     if (err) x.code = ctl1.err;
     else if (!finished && unbounded) x.code = MPRGP_TIMEOUT;
@@ -1264,7 +1426,12 @@ int mprgp_context_create(int device, mprgp_context **out) {
   CK(power_max_blocks_per_sm(1, &c->bps_power_v[1]));
   CK(power_max_blocks_per_sm(2, &c->bps_power_v[2]));
   CK(power_max_blocks_per_sm(3, &c->bps_power_v[3]));
-  CK(power_persistent_max_blocks_per_sm(&c->bps_power_pp));
+  {
+    int b32 = 0, b64 = 0;
+    CK(power_persistent_max_blocks_per_sm(1, &b32));
+    CK(power_persistent_max_blocks_per_sm(0, &b64));
+    c->bps_power_pp = std::min(b32, b64);
+  }
   c->bps_power = c->bps_power_v[0];
   {
     int largest = 0;
@@ -1273,6 +1440,8 @@ int mprgp_context_create(int device, mprgp_context **out) {
       c->cluster_ok[q] = cluster_max_active(1 << q, &nc) == cudaSuccess && nc >= 1;
       cudaGetLastError();
       if (c->cluster_ok[q]) largest = 1 << q;
+      c->power_cluster_ok[q] = power_clusters_max_active(1 << q, &nc) == cudaSuccess && nc >= 1;
+      cudaGetLastError();
     }
     c->cluster = std::min(c->cluster, largest);
   }
@@ -1453,6 +1622,7 @@ int mprgp_problem_set_matrix(mprgp_problem *p, int nnzb, const int *row_ptr, con
   CK(cudaMemcpyAsync(p->stage_vals, vals, sizeof(double) * 9 * nnzb, kind, s));
   p->h_len.resize(nv);
   for (int r = 0; r < nv; ++r) p->h_len[r] = h_ptr[r + 1] - h_ptr[r];
+  p->max_len = *std::max_element(p->h_len.begin(), p->h_len.end());
   p->nnzb = nnzb;
   p->want64 = precisions & 1;
   p->want32 = (precisions >> 1) & 1;

@@ -183,6 +183,9 @@ __device__ __forceinline__ unsigned long long atom_add_acq_rel(unsigned long lon
                : "=l"(old) : "l"(p), "l"(v) : "memory");
   return old;
 }
+__device__ __forceinline__ void red_add_release(unsigned int *p, unsigned int v) {
+  asm volatile("red.release.gpu.global.add.u32 [%0], %1;" : : "l"(p), "r"(v) : "memory");
+}
 __device__ __forceinline__ void st_release(unsigned int *p, unsigned int v) {
   asm volatile("st.release.gpu.global.u32 [%0], %1;" : : "l"(p), "r"(v) : "memory");
 }
@@ -2011,22 +2014,24 @@ __device__ void cg_decide(const InstDesc &D, InstState &S, double dfy, double co
 }
 
 // Transitions of the power method (specRad, MPRGPSolver.h:42-79), shared by
-// the persistent engine and the dedicated power kernel.
-__device__ void advance_power(const InstDesc &D, InstState &S, const double *s) {
+// every form of the power loop.  R gives the roots of the phase's two sums and
+// their reciprocals: dif = sqrt(s0), nrm = sqrt(s1).
+template <typename Roots>
+__device__ __forceinline__ void advance_power_roots(const InstDesc &D, InstState &S, const Roots &r) {
   const double eps = D.tol;  // specRad(A, ev, tol): eps = tol (MPRGPSolver.h:28)
   switch (S.phase) {
     case PH_POW_RAND:
       S.pow_k = 0;
       S.pow_src = B_W1;
-      S.pow_scale = 1.0 / sqrt(s[0]);  // tmp.normalize()
+      S.pow_scale = r.inv_dif();  // tmp.normalize()
       S.phase = PH_POW;
       break;
     case PH_POW: {
       const int k = S.pow_k;
-      const double nrm = sqrt(s[1]);
+      const double nrm = r.nrm();
       if (D.prec == PREC_MIXED) S.spmv32++; else S.spmv64++;
       S.pow_spmv++;
-      if (k >= 1 && sqrt(s[0]) <= eps) {  // iteration k-1 converged
+      if (k >= 1 && r.dif() <= eps) {  // iteration k-1 converged
         S.spec_rad = S.pow_nrm_prev;
         S.ev_upd = 1;
         S.ev_src = B_T0 + ((k - 1) & 1);
@@ -2043,7 +2048,7 @@ __device__ void advance_power(const InstDesc &D, InstState &S, const double *s) 
         break;
       }
       S.pow_nrm_prev = nrm;
-      S.pow_scale = 1.0 / nrm;
+      S.pow_scale = r.inv_nrm();
       S.pow_src = (k & 1) ? B_W1 : B_W;
       if (k == 1000) {
         S.pow_k = 1001;
@@ -2055,7 +2060,7 @@ __device__ void advance_power(const InstDesc &D, InstState &S, const double *s) 
     }
     case PH_POW_LAST:
       S.spec_rad = S.pow_nrm_prev;
-      if (sqrt(s[0]) <= eps) {
+      if (r.dif() <= eps) {
         S.ev_upd = 1;
         S.ev_src = B_T0 + (1000 & 1);
         S.power_iters = 1000;
@@ -2071,6 +2076,23 @@ __device__ void advance_power(const InstDesc &D, InstState &S, const double *s) 
     S.alpha_bar = 2.0 / S.spec_rad;  // MPRGPSolver.h:28
     if (D.project_x0) S.phase = PH_PROJ0;
   }
+}
+struct RootsOfSums {  // taken when asked for
+  const double *s;
+  __device__ __forceinline__ double dif() const { return sqrt(s[0]); }
+  __device__ __forceinline__ double nrm() const { return sqrt(s[1]); }
+  __device__ __forceinline__ double inv_dif() const { return 1.0 / sqrt(s[0]); }
+  __device__ __forceinline__ double inv_nrm() const { return 1.0 / sqrt(s[1]); }
+};
+struct RootsTaken {
+  double d, n, id, in;
+  __device__ __forceinline__ double dif() const { return d; }
+  __device__ __forceinline__ double nrm() const { return n; }
+  __device__ __forceinline__ double inv_dif() const { return id; }
+  __device__ __forceinline__ double inv_nrm() const { return in; }
+};
+__device__ void advance_power(const InstDesc &D, InstState &S, const double *s) {
+  advance_power_roots(D, S, RootsOfSums{s});
 }
 
 __device__ void advance(const InstDesc &D, InstState &S, const double *s) {
@@ -2919,173 +2941,38 @@ __global__ void __launch_bounds__(32)
   }
 }
 
-// ------------------------------------------------ persistent power loop -----
-// Every power-method phase of a run's large instances in one cooperative
-// launch, a bounded grid barrier as the phase boundary, with the power-step
-// loop's overlap: a phase's reduction and state update run in one extra warp
-// while the row warps already form the next phase's matrix products.
+// ------------------------------------------------------ power sync loop -----
+// The power method of a synchronous run's instances in one launch whose CTAs
+// are all resident, with no grid barrier: an instance's CTAs wait only for
+// each other, on the item partials they exchange anyway.
 //
-// Each CTA owns up to kPowOwn items (item b, b + grid, ...; the host sizes
-// the grid so that the CTAs own equally many) and keeps their desc and state
-// in shared memory for the whole loop.  Phase t: the reduction warp applies
-// phase t-1's item partials to each owned item's copy of the state (the
-// launch form's finalize order, warp_item_sums) while the row warps form the
-// first owned item's raw product A src with the source the advanced state
-// will name; then each owned item in a power phase finishes its rows with
-// the advanced state (scale, store, partials of phase t, double-buffered by
-// phase parity).  Every copy advances from the same sums in the same order as
-// the launch form, so results are bitwise those of the launch form.  The loop
-// ends after the first phase in which no instance had rows (each CTA with
-// rows publishes the phase with atomicMax before the barrier), or after
-// `limit` phases; then the CTA owning an instance's first item writes its
-// state back.
-// The reduction warp's work for one owned item: S advanced by the partials
-// pp.  Not inlined, so that its sums do not take registers from the rows.
-__device__ __noinline__ void persistent_apply(const InstDesc &D, InstState &S, const double *pp,
-                                              int lane, double2 *stage) {
-  double s2[2];
-  warp_item_sums(pp, D.nitems, lane, stage, s2);
-  __syncwarp();
-  if (lane == 0) advance_power_sums(D, S, s2);
-  __syncwarp();
-}
-
-template <int kMinBlocks>
-__global__ void __launch_bounds__(kStepThreads, kMinBlocks)
-    power_persistent_kernel(EngineArgs args, PowCtl *pc, int limit) {
-  __shared__ InstDesc sD[kPowOwn];
-  __shared__ InstState sS[kPowOwn];
-  __shared__ RedBuf red;
-  __shared__ __align__(16) double2 sItems[kSumStage];
-  if (threadIdx.x == 0) g_staged = 0;
-  const int lane = threadIdx.x & 31;
-  const bool rw = threadIdx.x >= kThreads;  // the reduction warp
-  // owned items: blockIdx.x + o * gridDim.x, o < nown
-  const int nown = min(kPowOwn, (args.total_items - (int)blockIdx.x + (int)gridDim.x - 1) /
-                                    (int)gridDim.x);
-  for (int o = 0; o < nown; ++o) {
-    const int inst = instance_of(args.item_inst, args.item_prefix, args.ninst, (int)(blockIdx.x + o * gridDim.x));
-    const int *srcd = reinterpret_cast<const int *>(args.desc + inst);
-    int *dstd = reinterpret_cast<int *>(&sD[o]);
-    for (int w = threadIdx.x; w < (int)(sizeof(InstDesc) / 4); w += kStepThreads)
-      dstd[w] = ldro(srcd + w);
-    const int *srcs = reinterpret_cast<const int *>(args.states ? args.states + inst : nullptr);
-    int *dsts = reinterpret_cast<int *>(&sS[o]);
-    if (srcs)
-      for (int w = threadIdx.x; w < (int)(sizeof(InstState) / 4); w += kStepThreads)
-        dsts[w] = srcs[w];
-  }
-  __syncthreads();
-  if (!args.states) {  // the states live at the descs' home
-    for (int o = 0; o < nown; ++o) {
-      const int *srcs = reinterpret_cast<const int *>(sD[o].st);
-      int *dsts = reinterpret_cast<int *>(&sS[o]);
-      for (int w = threadIdx.x; w < (int)(sizeof(InstState) / 4); w += kStepThreads)
-        dsts[w] = srcs[w];
-    }
-    __syncthreads();
-  }
-  unsigned int pend = 0u;  // bit o: item o's rows ran in the previous phase
-  int t = 0;
-  for (;; ++t) {
-    const int par = t & 1;
-    // The first owned item's source vector, predicted from its state before
-    // the advance (the previous phase's output when rows ran there).
-    int src0 = kNoSrc;
-    if (nown > 0) {
-      const InstState &S0 = sS[0];
-      if (pend & 1u) {
-        if (S0.phase == PH_POW_RAND) src0 = B_W1;
-        else if (S0.phase == PH_POW) src0 = (S0.pow_k & 1) ? B_W1 : B_W;
-      } else if (S0.phase == PH_POW) {
-        src0 = S0.pow_src;
-      }
-    }
-    float wf[3] = {0.f, 0.f, 0.f};
-    double wd[3] = {0.0, 0.0, 0.0};
-    if (!rw && src0 != kNoSrc) {
-      const int slot = ((int)blockIdx.x - sD[0].item_begin) * kThreads + threadIdx.x;
-      if (slot < sD[0].nv) {
-        if (sD[0].prec == PREC_MIXED) pow_raw32(sD[0], src0, slot, wf);
-        else pow_raw64(sD[0], src0, slot, wd);
-      }
-    }
-    if (rw) {  // apply the previous phase's partials to every owned state
-      for (int o = 0; o < nown; ++o) {
-        if (!((pend >> o) & 1u)) continue;
-        persistent_apply(sD[o], sS[o], sD[o].part + (size_t)(par ^ 1) * sD[o].nitems * 2, lane,
-                         sItems);
-      }
-    }
-    __syncthreads();
-    unsigned int ran = 0u;
-    for (int o = 0; o < nown; ++o) {
-      const int phase = sS[o].phase;
-      if (!power_phase(phase)) continue;
-      ran |= 1u << o;
-      const InstDesc &D = sD[o];
-      const int local = (int)(blockIdx.x + o * gridDim.x) - D.item_begin;
-      const int slot = local * kThreads + threadIdx.x;
-      const bool row = !rw && slot < D.nv;
-      const bool f32 = D.prec == PREC_MIXED;
-      double part[2] = {0.0, 0.0};
-      if (row) {
-        const int v = row_vertex(D.A, slot);
-        if (phase == PH_POW_RAND) {
-          row_power_rand(D, v, part);
-        } else {
-          const int src = sS[o].pow_src;
-          if (phase == PH_POW && (o > 0 || src != src0)) {  // not formed above
-            if (f32) pow_raw32(D, src, slot, wf);
-            else pow_raw64(D, src, slot, wd);
-          }
-          if (f32) row_power32_fin(D, sS[o], v, wf, part);
-          else row_power64_fin(D, sS[o], v, wd, part);
-        }
-      }
-      // the item this CTA takes next: its next owned item, else its first
-      // owned item in the next phase
-      if (o + 1 < nown) prefetch_item_head(sD[o + 1], (int)(blockIdx.x + (o + 1) * gridDim.x) - sD[o + 1].item_begin);
-      else prefetch_item_head(sD[0], (int)blockIdx.x - sD[0].item_begin);
-      const double r = block_reduce_rows(part, red, nslots(phase));
-      if (threadIdx.x < 2) D.part[(size_t)par * D.nitems * 2 + 2 * (size_t)local + threadIdx.x] = r;
-    }
-    pend = ran;
-    if (ran && threadIdx.x == 0) atomicMax(&pc->busy, (unsigned int)(t + 1));
-    int unused;
-    if (!grid_barrier(args.ctl, args.wait_ns, unused)) return;
-    if (*(volatile unsigned int *)&pc->busy < (unsigned int)(t + 1)) break;  // no rows anywhere
-    if (t + 1 >= limit) {  // the last phase's partials, then stop
-      if (rw) {
-        for (int o = 0; o < nown; ++o) {
-          if (!((pend >> o) & 1u)) continue;
-          persistent_apply(sD[o], sS[o], sD[o].part + (size_t)par * sD[o].nitems * 2, lane,
-                           sItems);
-        }
-      }
-      __syncthreads();
-      ++t;
-      break;
-    }
-  }
-  // the working phases run (the launch form's launch count)
-  if (blockIdx.x == 0 && threadIdx.x == 0) pc->launches = (unsigned int)t;
-  for (int o = 0; o < nown; ++o)
-    if ((int)(blockIdx.x + o * gridDim.x) == sD[o].item_begin && threadIdx.x == 0) *sD[o].st = sS[o];
-}
-
-// ---------------------------------------------------- cluster solver -----
-// One thread-block cluster per small instance.  Every CTA of the cluster
-// holds the instance's desc and state in shared memory and advances its own
-// copy of the state from the same sums, so the copies never diverge and no
-// state travels through global memory between phases.  A phase: each CTA runs
-// the per-row work of its items and reduces each item in the block (as the
-// engine does); the item partials stay in shared memory; one cluster barrier
-// (release/acquire, which also orders the phase's global vector writes); then
-// every CTA reads all item partials through distributed shared memory in item
-// order and reduces them exactly as the engine's finalize does -- so results
-// are bitwise those of the persistent engine.  The partials are double
-// buffered by phase parity, so one barrier per phase suffices.
+// What bounds a power phase of a small or medium instance is its chain of
+// dependent latencies (a thousand phases, each a matrix pass, two sums over
+// all rows, a square root and a reciprocal), not bytes: as graph launches a
+// 70-item phase took 17.1 us and the cluster solver 9.7 (1,760 vertices,
+// mixed) to 16.7 us (425 vertices, FP64: eight row warps' 1,080 FP64 FMAs on
+// one SM alone take 8.6).  This loop takes 13.7, 4.8 and 10.4 us.  Here:
+//  * A unit is one item's rows, in one CTA or split over a cluster of q CTAs,
+//    so that few items still use many SMs' FP64 units.  A row belongs to one
+//    thread for the whole loop: its iterate, the previous one and its matrix
+//    row (in shared memory) stay on the SM; per phase it reads only the
+//    neighbours' iterates.
+//  * A phase's two item sums go out as doubles whose sign bit, free in a sum
+//    of squares, is a phase tag: a record tells by itself when it is there,
+//    so waiting for the phase and reading its sums is one round trip to L2.
+//    The partials are double buffered by phase parity and the tag alternates
+//    every second phase.  A CTA overwrites the iterate buffer of phase t - 1
+//    only after every CTA of the instance has published phase t, which it
+//    does after its last read of that buffer.
+//  * One more warp waits for the records, reduces them in the finalize's
+//    order and advances the CTA's copy of the state while the row warps form
+//    the next phase's products, whose source the state before the advance
+//    determines (as in the power-step loop).  The two square roots and
+//    reciprocals are taken by two lanes at once.
+// Each copy of a state advances from the same sums in the same order as the
+// launch form, so the results are its bits.  Every wait is bounded by
+// wait_ns; a CTA whose wait ran out sets the error and leaves, with its
+// cluster, and the others follow when they see the error.
 __device__ __forceinline__ void cluster_sync_acq_rel() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;"
                ::: "memory");
@@ -3118,6 +3005,568 @@ __device__ __forceinline__ double ld_dsmem(unsigned int addr) {
   return v;
 }
 
+
+constexpr unsigned long long kSignBit = 1ull << 63;
+
+__device__ __forceinline__ void fence_acq_rel() {
+  asm volatile("fence.acq_rel.gpu;" ::: "memory");
+}
+__device__ __forceinline__ void ld_record(const double *p, unsigned long long &a,
+                                          unsigned long long &b) {
+  asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
+}
+__device__ __forceinline__ void st_record(double *p, double v, unsigned long long tag) {
+  const unsigned long long w = ((unsigned long long)__double_as_longlong(v) & ~kSignBit) | tag;
+  asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" : : "l"(p), "l"(w) : "memory");
+}
+
+// One warp waits for the instance's records of a phase and sums them in the
+// finalize's order (warp_item_sums): lane l holds the sums of items l + 32 i,
+// + 256, ...  `wait` returns false when the wait ran out or another CTA's
+// did; afterwards every write of the phase is visible to the CTA (after its
+// next barrier).
+struct SyncSums {
+  double t0[kThreads / 32], t1[kThreads / 32];
+  __device__ __forceinline__ bool wait(const double *rec, int nitems, int lane,
+                                       unsigned long long tag, Ctl *ctl, long long wait_ns) {
+    bool ok = true;
+    long long since = 0;
+    for (int base = 0; base < nitems; base += kThreads) {
+      const int ni = min(kThreads / 32, (nitems - base + 31) / 32);  // warp-uniform
+      unsigned int need = 0u;
+#pragma unroll
+      for (int i = 0; i < kThreads / 32; ++i)
+        if (base + lane + 32 * i < nitems) need |= 1u << i;
+      if (base == 0) {
+#pragma unroll
+        for (int i = 0; i < kThreads / 32; ++i) t0[i] = t1[i] = 0.0;
+      }
+      int spins = 0;
+      while (__any_sync(0xffffffffu, need != 0u)) {
+        unsigned long long a[kThreads / 32], b[kThreads / 32];
+#pragma unroll
+        for (int i = 0; i < kThreads / 32; ++i)
+          if (i < ni && (need >> i) & 1u) ld_record(rec + 2 * (size_t)(base + lane + 32 * i), a[i], b[i]);
+#pragma unroll
+        for (int i = 0; i < kThreads / 32; ++i) {
+          if (i < ni && (need >> i) & 1u && (a[i] & kSignBit) == tag && (b[i] & kSignBit) == tag) {
+            const double x = __longlong_as_double((long long)(a[i] & ~kSignBit));
+            const double y = __longlong_as_double((long long)(b[i] & ~kSignBit));
+            t0[i] = base == 0 ? x : t0[i] + x;
+            t1[i] = base == 0 ? y : t1[i] + y;
+            need &= ~(1u << i);
+          }
+        }
+        if (++spins >= 64) {
+          spins = 0;
+          const long long now = gtimer();
+          if (since == 0) since = now;
+          bool give_up = *(volatile int *)&ctl->err != 0;
+          if (now - since > wait_ns) {
+            if (lane == 0) atomicCAS(&ctl->err, 0, -4);  // MPRGP_TIMEOUT
+            give_up = true;
+          }
+          if (__any_sync(0xffffffffu, give_up)) {
+            ok = false;
+            break;
+          }
+        }
+      }
+      if (!ok) break;
+    }
+    fence_acq_rel();
+    return ok;
+  }
+  // The instance's sums, with their roots and reciprocals (valid in lane 0).
+  // Additions of an exact zero -- items and lanes that do not exist -- are
+  // left out.
+  __device__ __forceinline__ RootsTaken roots(int nitems, int lane) const {
+    double a0 = t0[0], a1 = t1[0];
+#pragma unroll
+    for (int i = 1; i < kThreads / 32; ++i) {
+      if (32 * i >= nitems) break;
+      a0 = a0 + t0[i];
+      a1 = a1 + t1[i];
+    }
+    if (nitems > 16) {
+      a0 += __shfl_xor_sync(0xffffffffu, a0, 16);
+      a1 += __shfl_xor_sync(0xffffffffu, a1, 16);
+    } else {  // lanes 16.. hold zeros: slot 1's half-warp takes lanes 0..15's values
+      a1 = __shfl_sync(0xffffffffu, a1, lane & 15);
+    }
+    double v = lane < 16 ? a0 : a1;  // the rest of both trees at once
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1)
+      if (o < nitems) v += __shfl_xor_sync(0xffffffffu, v, o);
+    const double root = sqrt(v), inv = 1.0 / root;
+    return RootsTaken{root, __shfl_sync(0xffffffffu, root, 16), inv,
+                      __shfl_sync(0xffffffffu, inv, 16)};
+  }
+};
+
+// The power loop's product, end of row and vectors (B_W, B_W1, B_T0, B_T1) by
+// the form's value type.
+__device__ __forceinline__ void pow_raw(const InstDesc &D, int src, int slot, float w[3]) {
+  pow_raw32(D, src, slot, w);
+}
+__device__ __forceinline__ void pow_raw(const InstDesc &D, int src, int slot, double w[3]) {
+  pow_raw64(D, src, slot, w);
+}
+__device__ __forceinline__ void pow_fin(const InstDesc &D, const InstState &S, int v,
+                                        const float w[3], double *part) {
+  row_power32_fin(D, S, v, w, part);
+}
+__device__ __forceinline__ void pow_fin(const InstDesc &D, const InstState &S, int v,
+                                        const double w[3], double *part) {
+  row_power64_fin(D, S, v, w, part);
+}
+__device__ __forceinline__ float *pow_vec(const InstDesc &D, int id, float) {
+  return D.buf32[id == B_W ? F_W0 : id == B_W1 ? F_W1 : F_Z0 + (id - B_T0)];
+}
+__device__ __forceinline__ double *pow_vec(const InstDesc &D, int id, double) { return D.buf[id]; }
+// A row's product from the staged copy of its slice: kCh slots' neighbours in
+// flight at a time, accumulated slot by slot.
+template <int kCh, typename VT, typename Src>
+__device__ __forceinline__ void sync_row(const VT *sv, const int *sc, int lane, int j0,
+                                                int j1, const Src &src, VT out[3]) {
+  VT a0 = 0, a1 = 0, a2 = 0;
+  for (int jb = j0; jb < j1; jb += kCh) {
+    VT xv[kCh][3];
+#pragma unroll
+    for (int u = 0; u < kCh; ++u)
+      if (jb + u < j1) src(sc[(jb + u) * kSlice + lane], xv[u]);
+#pragma unroll
+    for (int u = 0; u < kCh; ++u) {
+      if (jb + u >= j1) break;
+      VT m[9];
+      const VT *b = sv + (size_t)(jb + u) * (9 * kSlice);
+      if constexpr (sizeof(VT) == 4) {
+        const float4 p = *reinterpret_cast<const float4 *>(b + 4 * lane);
+        const float4 q = *reinterpret_cast<const float4 *>(b + 128 + 4 * lane);
+        m[0] = p.x; m[1] = p.y; m[2] = p.z; m[3] = p.w;
+        m[4] = q.x; m[5] = q.y; m[6] = q.z; m[7] = q.w;
+      } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const double2 p = *reinterpret_cast<const double2 *>(b + 64 * k + 2 * lane);
+          m[2 * k] = p.x;
+          m[2 * k + 1] = p.y;
+        }
+      }
+      m[8] = b[256 + lane];
+      const VT x0 = xv[u][0], x1 = xv[u][1], x2 = xv[u][2];
+      a0 = fma(m[0], x0, a0); a0 = fma(m[1], x1, a0); a0 = fma(m[2], x2, a0);
+      a1 = fma(m[3], x0, a1); a1 = fma(m[4], x1, a1); a1 = fma(m[5], x2, a1);
+      a2 = fma(m[6], x0, a2); a2 = fma(m[7], x1, a2); a2 = fma(m[8], x2, a2);
+    }
+  }
+  out[0] = a0;
+  out[1] = a1;
+  out[2] = a2;
+}
+
+template <int kCh>
+__device__ __forceinline__ void sync_row_staged(const float *sv, const int *sc, int lane, int j0,
+                                                int j1, const float *src, float out[3]) {
+  sync_row<kCh>(sv, sc, lane, j0, j1, SrcF{src}, out);
+}
+template <int kCh>
+__device__ __forceinline__ void sync_row_staged(const double *sv, const int *sc, int lane, int j0,
+                                                int j1, const double *src, double out[3]) {
+  sync_row<kCh>(sv, sc, lane, j0, j1, SrcV{src}, out);
+}
+// The product of a loop's first phase when it was resumed or starts from ev,
+// from global memory; out of line, and by value, since it runs once.
+template <typename VT>
+struct Row3 {
+  VT w[3];
+};
+template <typename VT>
+__device__ __noinline__ Row3<VT> sync_row_first(const InstDesc &D, int src, int slot) {
+  Row3<VT> r;
+  pow_raw(D, src, slot, r.w);
+  return r;
+}
+
+// Slices of one unit part in shared memory: the values as in global memory,
+// then the columns as vertices.  One pass before the loop.
+template <typename VT>
+__device__ __forceinline__ void sync_stage(const SellMatrix &A, const VT *vals, int s0, int s1,
+                                           int threads) {
+  const int f = ldro(A.slice_off + s0), l = ldro(A.slice_off + s1);
+  const int nv16 = (l - f) * 9 * kSlice * (int)sizeof(VT) / 16;
+  const float4 *src = reinterpret_cast<const float4 *>(vals + (size_t)f * (9 * kSlice));
+  for (int i = threadIdx.x; i < nv16; i += threads) cp_async16(g_stage + 16 * (size_t)i, src + i);
+  int *sc = reinterpret_cast<int *>(g_stage + 16 * (size_t)nv16);
+  for (int i = threadIdx.x; i < (l - f) * kSlice; i += threads)
+    sc[i] = checked_col(A, ldro(A.cols + (size_t)f * kSlice + i));
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
+}
+
+__device__ __forceinline__ double sq3(const float d[3]) {
+  return (double)fmaf(d[0], d[0], fmaf(d[1], d[1], d[2] * d[2]));
+}
+__device__ __forceinline__ double sq3(const double d[3]) { return dot3(d, d); }
+__device__ __forceinline__ void block_bar(int threads) {
+  asm volatile("bar.sync 0, %0;" : : "r"(threads) : "memory");
+}
+
+// The reduction warp's part of a phase: waits for the instance's records,
+// meets the row warps (which then form their products), reduces and advances
+// the state.  Not inlined, so that it takes no registers from the row warps.
+__device__ __noinline__ void sync_reduce(const InstDesc &D, InstState &S, int par,
+                                         unsigned long long tag, Ctl *ctl, long long wait_ns,
+                                         int threads, int *fail) {
+  const int lane = threadIdx.x & 31;
+  SyncSums sums;
+  const bool got = sums.wait(D.part + (size_t)par * D.nitems * 2, D.nitems, lane, tag, ctl, wait_ns);
+  if (!got && lane == 0) *fail = 1;
+  block_bar(threads);
+  const RootsTaken r = sums.roots(D.nitems, lane);
+  if (lane == 0 && got) {
+    S.phases++;
+    advance_power_roots(D, S, r);
+  }
+}
+
+template <typename VT, int kThr, int kMinBlocks, int kCh>
+__global__ void __launch_bounds__(kThr, kMinBlocks) power_sync_kernel(SyncArgs args) {
+  constexpr bool kSplit = kThr < kStepThreads;  // units may be split over a cluster
+  __shared__ InstDesc sD;
+  __shared__ InstState sS;
+  __shared__ double sPart[2][kThreads];
+  __shared__ int sFail[2];
+  const int q = kSplit ? args.q : 1;     // CTAs of a unit (a cluster)
+  const int rank = q > 1 ? (int)cluster_rank() : 0;
+  const int R = kThreads / q;            // rows of this CTA
+  const int threads = R + 32;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const bool rw = (int)threadIdx.x >= R;  // the reduction warp
+  const SyncItem unit = args.items[(int)blockIdx.x / q];
+  if (threadIdx.x == 0) {
+    g_staged = 0;
+    sFail[0] = sFail[1] = 0;
+  }
+  {
+    const int *srcd = reinterpret_cast<const int *>(args.desc + unit.inst);
+    int *dstd = reinterpret_cast<int *>(&sD);
+    for (int w = threadIdx.x; w < (int)(sizeof(InstDesc) / 4); w += threads) dstd[w] = ldro(srcd + w);
+    const int *srcs = reinterpret_cast<const int *>(args.states + unit.inst);
+    int *dsts = reinterpret_cast<int *>(&sS);
+    for (int w = threadIdx.x; w < (int)(sizeof(InstState) / 4); w += threads) dsts[w] = srcs[w];
+  }
+  __syncthreads();
+  const InstDesc &D = sD;
+  InstState &S = sS;
+  // the thread's row, its slots in the staged copy, its vectors
+  const int slot = unit.local * kThreads + rank * R + (int)threadIdx.x;
+  const bool row = !rw && slot < D.nv;
+  const int v = row ? row_vertex(D.A, slot) : 0;
+  int j0 = 0, j1 = 0, voff = 0;
+  VT own[3] = {0, 0, 0};                    // the phase's source at the row
+  VT tk[3] = {0, 0, 0}, tp[3] = {0, 0, 0};  // t_k and t_{k-1}
+  {
+    const int s0 = min(unit.local * (kThreads / kSlice) + rank * (R / kSlice), D.A.nslices);
+    const int s1 = min(s0 + R / kSlice, D.A.nslices);
+    sync_stage(D.A, sizeof(VT) == 4 ? reinterpret_cast<const VT *>(D.A.v32)
+                                    : reinterpret_cast<const VT *>(D.A.v64), s0, s1, threads);
+    const int f = ldro(D.A.slice_off + s0), l = ldro(D.A.slice_off + s1);
+    voff = (l - f) * 9 * kSlice * (int)sizeof(VT);
+    if (row) {
+      j0 = ldro(D.A.slice_off + (slot >> 5)) - f;
+      j1 = ldro(D.A.slice_off + (slot >> 5) + 1) - f;
+      if (S.phase == PH_POW || S.phase == PH_POW_LAST) {  // resumed, or started from ev
+        for (int d = 0; d < 3; ++d) {
+          const size_t i = 3 * (size_t)v + d;
+          own[d] = S.pow_src < 0 ? (VT)D.ev[i] : pow_vec(D, S.pow_src, VT())[i];
+          if (S.pow_k >= 1) tk[d] = pow_vec(D, B_T0 + ((S.pow_k - 1) & 1), VT())[i];
+        }
+      }
+    }
+  }
+  __syncthreads();
+  const VT *sv = reinterpret_cast<const VT *>(g_stage);
+  const int *sc = reinterpret_cast<const int *>(g_stage + voff);
+  int kl = -1;  // the last iteration run here
+  for (int t = 0;; ++t) {
+    const int par = t & 1;
+    const unsigned long long tag = ((t >> 1) & 1) ? 0ull : kSignBit;
+    VT wr[3] = {0, 0, 0};  // the raw product of raw_src
+    int raw_src = kNoSrc;
+    if (t > 0) {
+      if (rw) {
+        sync_reduce(D, S, par ^ 1, (((t - 1) >> 1) & 1) ? 0ull : kSignBit, args.ctl, args.wait_ns,
+                    threads, &sFail[par]);
+      } else {
+        const int phase_in = S.phase, k_in = S.pow_k;
+        block_bar(threads);  // phase t - 1 is complete
+        raw_src = phase_in == PH_POW_RAND ? B_W1
+                  : phase_in == PH_POW    ? ((k_in & 1) ? B_W1 : B_W)
+                                          : kNoSrc;
+        if (row && raw_src != kNoSrc) sync_row_staged<kCh>(sv, sc, lane, j0, j1, pow_vec(D, raw_src, VT()), wr);
+      }
+      block_bar(threads);
+      if (q == 1 && sFail[par]) break;
+    }
+    const int phase = S.phase;
+    if (!power_phase(phase) || t >= unit.limit) break;
+    double p0 = 0.0, p1 = 0.0;
+    if (row) {
+      if (phase == PH_POW_RAND) {
+        double part[2] = {0.0, 0.0};
+        row_power_rand(D, v, part);
+        p0 = part[0];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) own[d] = (VT)seeded_uniform(D.seed, 3ull * v + d);
+      } else {  // row_power32_fin / row_power64_fin from registers
+        if (phase == PH_POW && S.pow_src != raw_src) {  // no product yet
+          const Row3<VT> r = sync_row_first<VT>(D, S.pow_src, slot);
+          wr[0] = r.w[0];
+          wr[1] = r.w[1];
+          wr[2] = r.w[2];
+        }
+        const VT scale = (VT)S.pow_scale;
+        const VT u[3] = {own[0] * scale, own[1] * scale, own[2] * scale};
+        if (phase == PH_POW_LAST || S.pow_k >= 1) {
+          const VT d[3] = {u[0] - tk[0], u[1] - tk[1], u[2] - tk[2]};
+          p0 = sq3(d);
+        }
+        if (phase == PH_POW) {
+          VT *wv = pow_vec(D, (S.pow_k & 1) ? B_W1 : B_W, VT()) + 3 * (size_t)v;
+#pragma unroll
+          for (int d = 0; d < 3; ++d) {
+            tp[d] = tk[d];
+            tk[d] = u[d];
+            own[d] = wr[d] * scale;
+            wv[d] = own[d];
+          }
+          p1 = sq3(own);
+        }
+      }
+    }
+    if (phase == PH_POW) kl = S.pow_k;
+    // the item's sums of phase t, in block_reduce's order
+    if (!rw) {
+      sPart[0][threadIdx.x] = p0;
+      sPart[1][threadIdx.x] = p1;
+    }
+    if (q > 1) {
+      cluster_sync_acq_rel();
+      if (warp == 0 && lane < q && lane != rank) {  // a peer's wait ran out: all leave together
+        unsigned int bad;
+        asm volatile("ld.shared::cluster.u32 %0, [%1];"
+                     : "=r"(bad) : "r"(dsmem_addr(&sFail[par], (unsigned int)lane)) : "memory");
+        if (bad) sFail[par] = 1;
+      }
+    } else {
+      __syncthreads();
+    }
+    if (rank == 0 && warp < 2) {
+      double x[kThreads / 32];
+#pragma unroll
+      for (int i = 0; i < kThreads / 32; ++i) {
+        if (q > 1)
+          x[i] = ld_dsmem(dsmem_addr(&sPart[warp][(lane + 32 * i) & (R - 1)],
+                                     (unsigned int)((32 * i) / R)));
+        else
+          x[i] = sPart[warp][lane + 32 * i];
+      }
+      double acc = x[0];
+#pragma unroll
+      for (int i = 1; i < kThreads / 32; ++i) acc = acc + x[i];
+      acc = warp_sum(acc);
+      if (lane == 0) {
+        fence_acq_rel();
+        st_record(D.part + (size_t)par * D.nitems * 2 + 2 * (size_t)unit.local + warp, acc, tag);
+      }
+    }
+    if (q > 1) {
+      __syncthreads();
+      if (sFail[par]) break;
+    }
+  }
+  if (row && kl >= 0) {  // t_k and t_{k-1}, where PH_INIT looks for ev
+    for (int d = 0; d < 3; ++d) {
+      const size_t i = 3 * (size_t)v + d;
+      pow_vec(D, B_T0 + (kl & 1), VT())[i] = tk[d];
+      if (kl >= 1) pow_vec(D, B_T0 + ((kl - 1) & 1), VT())[i] = tp[d];
+    }
+  }
+  __syncthreads();
+  if (rank == 0 && unit.local == 0 && threadIdx.x == 0) args.states[unit.inst] = S;
+  if (q > 1) cluster_sync_acq_rel();  // no CTA leaves while another may read its partials
+}
+
+// ------------------------------------------------ persistent power loop -----
+// The power sync loop for runs whose matrices do not fit the SMs' shared
+// memory: resident CTAs again, with the matrix read from L2 (or DRAM) in every
+// phase.  Each CTA owns up to kPowOwn items (item b,
+// b + grid, ...; the host sizes the grid so that the CTAs own equally many)
+// and keeps their desc and state in shared memory for the whole loop.  Phase
+// t: the reduction warp waits for phase t - 1 of every owned item's instance,
+// then applies its item partials to each owned state (the launch form's finalize
+// order, warp_item_sums) while the row warps form the first owned item's raw
+// product A src with the source the advanced state will name; then each owned
+// item in a power phase finishes its rows with the advanced state (scale,
+// store, partials of phase t).  A phase of an instance ends when its counter
+// says that all its items have published: one release per CTA and a poll of
+// one word, against the two hops of a grid barrier over every CTA (140,481
+// vertices mixed, 549 CTAs: 15.8 us a phase, 17.4 with the grid barrier, 23.2
+// as graph launches; its matrix pass alone, L2-resident, takes 10.4).
+// Instances do not wait for each other.  With the items of an instance in one
+// cluster the same kernel needs no cooperative launch (the cluster's CTAs are
+// resident together): the small instances of a batch or a server lane, which
+// took 9.7 us a phase in the cluster solver, take about 7.  The results are
+// the launch form's bits.
+// Waits until an instance's items have all counted phase t - 1, `target` in
+// all (bounded as SyncSums::wait).  A counter, not the records: with hundreds
+// of CTAs an instance, polling every record took L2 bandwidth from the CTAs
+// still in their matrix pass (140,481 vertices mixed: 22.6 us a phase).
+__device__ __forceinline__ unsigned int *phase_count(const InstDesc &D) {
+  return reinterpret_cast<unsigned int *>(D.part + 4 * (size_t)D.nitems);
+}
+__device__ __noinline__ bool wait_count(const unsigned int *count, unsigned int target, Ctl *ctl,
+                                        long long wait_ns) {
+  long long since = 0;
+  int spins = 0;
+  while (ld_acquire(count) < target) {
+    if (++spins >= 64) {
+      spins = 0;
+      const long long now = gtimer();
+      if (since == 0) since = now;
+      if (*(volatile int *)&ctl->err != 0) return false;
+      if (now - since > wait_ns) {
+        atomicCAS(&ctl->err, 0, -4);  // MPRGP_TIMEOUT
+        return false;
+      }
+    }
+  }
+  return true;
+}
+// The reduction warp's work for one owned item: S advanced by the partials
+// rec.  Not inlined, so that its sums do not take registers from the rows.
+__device__ __noinline__ void persistent_apply(const InstDesc &D, InstState &S, const double *rec,
+                                              int lane, double2 *stage) {
+  double s2[2];
+  warp_item_sums(rec, D.nitems, lane, stage, s2);
+  __syncwarp();
+  if (lane == 0) advance_power_sums(D, S, s2);
+  __syncwarp();
+}
+
+template <typename VT, int kMinBlocks>
+__global__ void __launch_bounds__(kStepThreads, kMinBlocks)
+    power_persistent_kernel(SyncArgs args) {
+  __shared__ InstDesc sD[kPowOwn];
+  __shared__ SyncItem sItem[kPowOwn];
+  __shared__ int sFail;
+  __shared__ InstState sS[kPowOwn];
+  __shared__ RedBuf red;
+  __shared__ __align__(16) double2 sItems[kSumStage];
+  if (threadIdx.x == 0) g_staged = 0;
+  const int lane = threadIdx.x & 31;
+  const bool rw = threadIdx.x >= kThreads;  // the reduction warp
+  // owned items: blockIdx.x + o * gridDim.x, o < nown
+  const int nown = min(kPowOwn, (args.units - (int)blockIdx.x + (int)gridDim.x - 1) /
+                                    (int)gridDim.x);
+  for (int o = 0; o < nown; ++o) {
+    const SyncItem it = args.items[blockIdx.x + o * gridDim.x];
+    if (threadIdx.x == 0) sItem[o] = it;
+    const int *srcd = reinterpret_cast<const int *>(args.desc + it.inst);
+    int *dstd = reinterpret_cast<int *>(&sD[o]);
+    for (int w = threadIdx.x; w < (int)(sizeof(InstDesc) / 4); w += kStepThreads)
+      dstd[w] = ldro(srcd + w);
+    const int *srcs = reinterpret_cast<const int *>(args.states + it.inst);
+    int *dsts = reinterpret_cast<int *>(&sS[o]);
+    for (int w = threadIdx.x; w < (int)(sizeof(InstState) / 4); w += kStepThreads)
+      dsts[w] = srcs[w];
+  }
+  if (threadIdx.x == 0) sFail = 0;
+  __syncthreads();
+  unsigned int pend = 0u;  // bit o: item o's rows ran in the previous phase
+  for (int t = 0;; ++t) {
+    const int par = t & 1;
+    // The first owned item's source vector, predicted from its state before
+    // the advance (the previous phase's output when rows ran there).
+    int src0 = kNoSrc;
+    if (nown > 0) {
+      const InstState &S0 = sS[0];
+      if (pend & 1u) {
+        if (S0.phase == PH_POW_RAND) src0 = B_W1;
+        else if (S0.phase == PH_POW) src0 = (S0.pow_k & 1) ? B_W1 : B_W;
+      } else if (S0.phase == PH_POW) {
+        src0 = S0.pow_src;
+      }
+    }
+    if (threadIdx.x == kThreads && pend) {  // every owned item's instance is done with phase t - 1
+      for (int o = 0; o < nown; ++o)
+        if ((pend >> o) & 1u && !wait_count(phase_count(sD[o]), (unsigned int)(t * sD[o].nitems),
+                                            args.ctl, args.wait_ns))
+          sFail = 1;
+    }
+    __syncthreads();
+    if (sFail) return;  // a wait ran out, here or elsewhere: the error is set
+    VT wr[3] = {0, 0, 0};
+    if (!rw && src0 != kNoSrc) {
+      const int slot = sItem[0].local * kThreads + threadIdx.x;
+      if (slot < sD[0].nv) pow_raw(sD[0], src0, slot, wr);
+    }
+    if (rw) {  // apply the previous phase's partials to every owned state
+      for (int o = 0; o < nown; ++o) {
+        if (!((pend >> o) & 1u)) continue;
+        persistent_apply(sD[o], sS[o], sD[o].part + (size_t)(par ^ 1) * sD[o].nitems * 2, lane,
+                         sItems);
+      }
+    }
+    __syncthreads();
+    unsigned int ran = 0u;
+    for (int o = 0; o < nown; ++o) {
+      const int phase = sS[o].phase;
+      if (!power_phase(phase) || t >= sItem[o].limit) continue;
+      ran |= 1u << o;
+      const InstDesc &D = sD[o];
+      const int local = sItem[o].local;
+      const int slot = local * kThreads + threadIdx.x;
+      const bool row = !rw && slot < D.nv;
+      double part[2] = {0.0, 0.0};
+      if (row) {
+        const int v = row_vertex(D.A, slot);
+        if (phase == PH_POW_RAND) {
+          row_power_rand(D, v, part);
+        } else {
+          const int src = sS[o].pow_src;
+          if (phase == PH_POW && (o > 0 || src != src0)) pow_raw(D, src, slot, wr);  // not formed above
+          pow_fin(D, sS[o], v, wr, part);
+        }
+      }
+      // the item this CTA takes next: its next owned item, else its first
+      // owned item in the next phase
+      const int on = o + 1 < nown ? o + 1 : 0;
+      prefetch_item_head(sD[on], sItem[on].local);
+      const double r = block_reduce_rows(part, red, nslots(phase));
+      if (threadIdx.x < 2) D.part[(size_t)par * D.nitems * 2 + 2 * (size_t)local + threadIdx.x] = r;
+      if (threadIdx.x < 32) __syncwarp();
+      if (threadIdx.x == 0) red_add_release(phase_count(D), 1u);
+    }
+    pend = ran;
+    if (!ran) break;
+  }
+  for (int o = 0; o < nown; ++o)
+    if (sItem[o].local == 0 && threadIdx.x == 0) args.states[sItem[o].inst] = sS[o];
+}
+
+// ---------------------------------------------------- cluster solver -----
+// One thread-block cluster per small instance.  Every CTA of the cluster
+// holds the instance's desc and state in shared memory and advances its own
+// copy of the state from the same sums, so the copies never diverge and no
+// state travels through global memory between phases.  A phase: each CTA runs
+// the per-row work of its items and reduces each item in the block (as the
+// engine does); the item partials stay in shared memory; one cluster barrier
+// (release/acquire, which also orders the phase's global vector writes); then
+// every CTA reads all item partials through distributed shared memory in item
+// order and reduces them exactly as the engine's finalize does -- so results
+// are bitwise those of the persistent engine.  The partials are double
+// buffered by phase parity, so one barrier per phase suffices.
 __global__ void __launch_bounds__(kThreads, MPRGP_CLUSTER_MIN_BLOCKS) cluster_kernel(ClusterArgs args) {
   __shared__ InstDesc sD;
   __shared__ InstState sS;
@@ -3340,11 +3789,16 @@ __global__ void __launch_bounds__(256, MPRGP_SPMV_MIN_BLOCKS) spmv_kernel(SellMa
 static_assert(sizeof(InstState) % 8 == 0, "InstState is copied as 8-byte words");
 constexpr int kStateWords = (int)(sizeof(InstState) / 8);
 
+// With clear_records the power sync loop's records of every instance (two per
+// item and phase parity; their phase tags then match nothing) and its phase
+// counter behind them are cleared too.
 __global__ void state_scatter_kernel(const InstDesc *__restrict__ desc, int n, InstState *states,
                                      InstState *const *__restrict__ home,
-                                     const int *__restrict__ fresh) {
+                                     const int *__restrict__ fresh, int clear_records) {
   const int j = blockIdx.x;
   if (j >= n) return;
+  if (clear_records)
+    for (int i = threadIdx.x; i <= 4 * desc[j].nitems; i += blockDim.x) desc[j].part[i] = 0.0;
   if (fresh[j]) {
     if (threadIdx.x == 0) *desc[j].cnt = 0u;
     return;
@@ -3369,8 +3823,8 @@ __global__ void state_gather_kernel(const InstDesc *__restrict__ desc, int n, In
 
 // Host-side launch helpers (declared in capi.cu).
 void launch_state_scatter(const InstDesc *desc, int n, InstState *states, InstState *const *home,
-                          const int *fresh, cudaStream_t st) {
-  if (n > 0) state_scatter_kernel<<<n, 64, 0, st>>>(desc, n, states, home, fresh);
+                          const int *fresh, int clear_records, cudaStream_t st) {
+  if (n > 0) state_scatter_kernel<<<n, 64, 0, st>>>(desc, n, states, home, fresh, clear_records);
 }
 void launch_state_gather(const InstDesc *desc, int n, InstState *states, InstState *const *home,
                          cudaStream_t st) {
@@ -3535,15 +3989,113 @@ cudaError_t cluster_max_active(int csize, int *n) {
   cfg.numAttrs = 1;
   return cudaOccupancyMaxActiveClusters(n, cluster_kernel, &cfg);
 }
-cudaError_t launch_power_persistent(const EngineArgs &args, PowCtl *d_pc, int limit, int grid,
-                                    cudaStream_t stream) {
-  void *params[] = {(void *)&args, (void *)&d_pc, (void *)&limit};
-  return cudaLaunchCooperativeKernel((const void *)power_persistent_kernel<4>, dim3(grid),
-                                     dim3(kStepThreads), params, 0, stream);
+static const void *power_persistent_fn(int fp32) {
+  return fp32 ? (const void *)power_persistent_kernel<float, 4>
+              : (const void *)power_persistent_kernel<double, 4>;
 }
-cudaError_t power_persistent_max_blocks_per_sm(int *n) {
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, power_persistent_kernel<4>, kStepThreads,
-                                                       0);
+cudaError_t launch_power_persistent(const SyncArgs &args, int fp32, int grid, cudaStream_t stream) {
+  void *params[] = {(void *)&args};
+  return cudaLaunchCooperativeKernel(power_persistent_fn(fp32), dim3(grid), dim3(kStepThreads),
+                                     params, 0, stream);
+}
+// The same kernel with the items of each instance in one cluster of `csize`
+// CTAs (args.items holds csize units an instance, absent ones with limit 0).
+// A cluster's CTAs are resident together, so no cooperative launch is needed
+// and any number of instances can be queued beside other lanes' kernels.
+static void power_clusters_config(int csize, int grid, cudaStream_t stream, cudaLaunchConfig_t &cfg,
+                                  cudaLaunchAttribute (&at)[1]) {
+  cfg = {};
+  cfg.gridDim = dim3((unsigned int)grid);
+  cfg.blockDim = dim3(kStepThreads);
+  cfg.stream = stream;
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned int)csize;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+}
+cudaError_t launch_power_clusters(const SyncArgs &args, int fp32, int csize, cudaStream_t stream) {
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute at[1];
+  power_clusters_config(csize, args.units, stream, cfg, at);
+  void *params[] = {(void *)&args};
+  return cudaLaunchKernelExC(&cfg, power_persistent_fn(fp32), params);
+}
+// Clusters of `csize` CTAs that can be resident at once (0 if none).
+cudaError_t power_clusters_max_active(int csize, int *n) {
+  *n = 0;
+  for (int fp32 = 0; fp32 < 2; ++fp32) {
+    if (csize > 8) {
+      cudaError_t e = cudaFuncSetAttribute(power_persistent_fn(fp32),
+                                           cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+      if (e != cudaSuccess) return e;
+    }
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute at[1];
+    power_clusters_config(csize, csize, nullptr, cfg, at);
+    cudaError_t e = cudaOccupancyMaxActiveClusters(n, power_persistent_fn(fp32), &cfg);
+    if (e != cudaSuccess || *n < 1) return e;
+  }
+  return cudaSuccess;
+}
+cudaError_t power_persistent_max_blocks_per_sm(int fp32, int *n) {
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, power_persistent_fn(fp32), kStepThreads, 0);
+}
+// The power sync loop's kernel for q CTAs a unit.
+template <typename VT>
+static const void *power_sync_fn(int q) {
+  return q > 1 ? (const void *)power_sync_kernel<VT, kThreads / 2 + 32, 3, 8>
+               : (const void *)power_sync_kernel<VT, kStepThreads, 1, 8>;
+}
+static const void *power_sync_fn(int q, int fp32) {
+  return fp32 ? power_sync_fn<float>(q) : power_sync_fn<double>(q);
+}
+static void power_sync_config(int q, int grid, int smem, cudaStream_t stream, cudaLaunchConfig_t &cfg,
+                              cudaLaunchAttribute (&at)[2]) {
+  cfg = {};
+  cfg.gridDim = dim3((unsigned int)grid);
+  cfg.blockDim = dim3((unsigned int)(kThreads / q + 32));
+  cfg.dynamicSmemBytes = (size_t)smem;
+  cfg.stream = stream;
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = (unsigned int)q;
+  at[1].val.clusterDim.y = 1;
+  at[1].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = q > 1 ? 2 : 1;
+}
+// CTAs of that form that can be resident at once (smem: staged bytes a CTA).
+cudaError_t power_sync_capacity(int q, int fp32, int smem, int nsm, int *ctas) {
+  *ctas = 0;
+  const void *fn = power_sync_fn(q, fp32);
+  // (one value for every query: the attribute is the kernel's, not the launch's)
+  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kSyncStageBytes);
+  if (e != cudaSuccess) return e;
+  int n = 0;
+  if (q == 1) {
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, kStepThreads, (size_t)smem);
+    *ctas = n * nsm;
+    return e;
+  }
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute at[2];
+  power_sync_config(q, q, smem, nullptr, cfg, at);
+  cfg.attrs = at + 1;
+  cfg.numAttrs = 1;
+  e = cudaOccupancyMaxActiveClusters(&n, fn, &cfg);
+  *ctas = n * q;
+  return e;
+}
+cudaError_t launch_power_sync(const SyncArgs &args, int fp32, int grid, int smem,
+                              cudaStream_t stream) {
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute at[2];
+  power_sync_config(args.q, grid, smem, stream, cfg, at);
+  void *params[] = {(void *)&args};
+  return cudaLaunchKernelExC(&cfg, power_sync_fn(args.q, fp32), params);
 }
 cudaError_t power_max_blocks_per_sm(int variant, int *n) {
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, power_kernel_fn(variant),

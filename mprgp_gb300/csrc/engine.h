@@ -143,8 +143,7 @@ struct Ctl {
 struct PowCtl {
   unsigned int active;    // instances in a power phase when the current launch began
   unsigned int fin;       // settle-kernel CTAs done in the current body (power-step loop)
-  unsigned int busy;      // instances still in a power phase (settle kernel) / the last
-                          // phase with one (persistent power loop)
+  unsigned int busy;      // instances still in a power phase (settle kernel)
   unsigned int launches;  // launches that did work so far
   unsigned int limit;     // stop after this many launches
   unsigned int stop;      // set when the loop is over: later launches return at once
@@ -169,6 +168,20 @@ struct ClusterArgs {
   const InstDesc *desc;  // the small instances, one per cluster
   int ninst;
   int max_phases;        // quantum / hard bound on phases
+};
+
+constexpr int kSyncStageBytes = 220 * 1024;  // shared memory of a power sync CTA's slices, at most
+// One item of an instance in the power sync loop (`limit`: its phases there).
+struct SyncItem {
+  int inst, local, limit, pad;
+};
+struct SyncArgs {
+  const InstDesc *desc;
+  InstState *states;
+  const SyncItem *items;
+  int units, q;  // q: CTAs of a unit
+  long long wait_ns;
+  Ctl *ctl;
 };
 
 struct EngineArgs {
