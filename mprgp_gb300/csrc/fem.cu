@@ -11,10 +11,10 @@
 //
 // Layout: the block sparsity pattern (3x3 blocks, one block row per vertex,
 // columns sorted) is built once per mesh on the host; per-tet geometry
-// (volume and shape-function gradients) lives on the device.  Assembly is a
-// gather, one thread per block row over the vertex's incident tets in a
-// fixed order: deterministic, no atomics.  The matrix and b go straight
-// into an mprgp_problem from device memory.
+// (volume and shape-function gradients, 128 bytes a tet) lives on the device.
+// Assembly is a gather, one thread per block row over the vertex's incident
+// tets in a fixed order: deterministic, no atomics.  The matrix and b go
+// straight into an mprgp_problem from device memory.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -36,7 +36,8 @@ struct mprgp_fem {
   int *tets = nullptr;                   // 4 per tet
   int *row_ptr = nullptr, *cols = nullptr;
   int *vt_ptr = nullptr, *vt = nullptr;  // incident (tet << 2 | local corner) per vertex
-  double *geom = nullptr;                // 13 per tet: V, grad N_0..3
+  int max_up = 0;                        // blocks right of the diagonal in a row, at most
+  double *geom = nullptr;                // kGeom per tet: V, grad N_0..3, padding
   double *X = nullptr;                   // rest shape
   double *mass = nullptr, *KX = nullptr;
   double *vals = nullptr, *b = nullptr;
@@ -56,6 +57,8 @@ int fail(int code, const char *what) {
     if (_e != cudaSuccess) return fail(MPRGP_CUDA_ERROR, #call);  \
   } while (0)
 
+constexpr int kGeom = 16;  // one 128-byte line a tet
+
 // Volume and shape-function gradients of each tet from the rest shape:
 // Dm = [X1-X0, X2-X0, X3-X0], grad N_a (a = 1..3) = rows of Dm^-1,
 // grad N_0 = -(sum of the others).  A degenerate tet gets V = 0.
@@ -71,7 +74,7 @@ __global__ void tet_geom_kernel(int ntet, const int *__restrict__ tets,
   const double det = Dm[0][0] * (Dm[1][1] * Dm[2][2] - Dm[1][2] * Dm[2][1]) -
                      Dm[0][1] * (Dm[1][0] * Dm[2][2] - Dm[1][2] * Dm[2][0]) +
                      Dm[0][2] * (Dm[1][0] * Dm[2][1] - Dm[1][1] * Dm[2][0]);
-  double *g = geom + 13 * (size_t)t;
+  double *g = geom + kGeom * (size_t)t;
   if (det == 0.0) {
     for (int k = 0; k < 13; ++k) g[k] = 0.0;
     return;
@@ -107,9 +110,135 @@ __device__ __forceinline__ int find_block(const int *__restrict__ cols, int r0, 
   return lo;
 }
 
-// One thread per vertex a: K_ab = V (lam gNa gNb^T + mu gNb gNa^T + mu (gNa . gNb) I)
-// summed over the tets around a (in incidence order), scaled by h^2 into the
-// block row of A, plus the lumped mass on the diagonal block; K X along the way.
+// A's rows by warps of 32 rows, one row a lane.
+//
+// K_ab = V (lam gNa gNb^T + mu gNb gNa^T + mu (gNa . gNb) I) summed over the
+// tets of an edge is lam P + mu P^T + mu tr(P) I with P = sum V gNa gNb^T, so
+// a tet adds nine products to a block instead of some sixty operations; GB300
+// issues one FP64 warp instruction in 64 clocks or more per scheduler, and
+// these bound the assembly (348,145 vertices, 2M tets: 0.77 ms, against 4.81
+// with a thread per row adding whole element blocks in global memory; the
+// matrix alone takes 0.06 ms to write).  Blocks right of the
+// diagonal are formed once and written with their transposes (K is symmetric;
+// the mirrored position comes from a search in the other row).  K X of the
+// rest shape X needs no blocks: sum_b gNb X_b^T = I in every tet, so
+// (K X)_a = (3 lam + 2 mu) sum V gNa.
+//
+// The lanes' blocks lie side by side in shared memory (entry k of lane l at
+// 33 k + l: no bank conflicts while the lanes add to blocks of their own, nor
+// while the warp copies one row out), the diagonal first, so that each row's
+// upper part leaves as one contiguous piece.
+constexpr int kRowPad = 33;
+constexpr int kUpperSmemMax = 220 * 1024;  // rows of up to 84 blocks right of the diagonal
+__host__ __device__ constexpr int upper_smem(int max_up) {
+  return kRowPad * (max_up + 1) * (9 * 8 + 4 + 4);
+}
+__global__ void __launch_bounds__(32)
+    assemble_upper_kernel(int nv, int max_up, const int4 *__restrict__ tets,
+                          const double *__restrict__ geom, const int *__restrict__ row_ptr,
+                          const int *__restrict__ cols, const int *__restrict__ vt_ptr,
+                          const int *__restrict__ vt, double lam, double mu, double rho, double h2,
+                          double *vals, double *mass, double *KX) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  double *P = reinterpret_cast<double *>(smem);                      // 9 per block
+  int *scol = reinterpret_cast<int *>(P + kRowPad * 9 * (max_up + 1));  // the block's column
+  int *spos = scol + kRowPad * (max_up + 1);                         // its mirror's position
+  const int lane = threadIdx.x;
+  const int a = blockIdx.x * 32 + lane;
+  int d = 0, nup = -1;  // the diagonal block, blocks right of it (-1: no row)
+  if (a < nv) {
+    const int r1 = row_ptr[a + 1];
+    d = find_block(cols, row_ptr[a], r1, a);
+    nup = r1 - d - 1;
+    for (int s = 1; s <= nup; ++s) {
+      const int b = cols[d + s];
+      scol[s * kRowPad + lane] = b;
+      spos[s * kRowPad + lane] = find_block(cols, row_ptr[b], row_ptr[b + 1], a);
+    }
+    for (int k = 9; k < 9 * (nup + 1); ++k) P[k * kRowPad + lane] = 0.0;
+    double m = 0.0, w[3] = {0.0, 0.0, 0.0}, q[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    for (int idx = vt_ptr[a]; idx < vt_ptr[a + 1]; ++idx) {
+      const int t = vt[idx] >> 2, la = vt[idx] & 3;
+      const int4 tv = tets[t];
+      const double *g = geom + kGeom * (size_t)t;
+      const double V = g[0];
+      const double g0 = g[1 + 3 * la], g1 = g[2 + 3 * la], g2 = g[3 + 3 * la];
+      const double w0 = V * g0, w1 = V * g1, w2 = V * g2;
+      m += rho * V / 4.0;
+      w[0] += w0;
+      w[1] += w1;
+      w[2] += w2;
+      q[0] = fma(w0, g0, q[0]);
+      q[1] = fma(w0, g1, q[1]);
+      q[2] = fma(w0, g2, q[2]);
+      q[3] = fma(w1, g1, q[3]);
+      q[4] = fma(w1, g2, q[4]);
+      q[5] = fma(w2, g2, q[5]);
+#pragma unroll
+      for (int lb = 0; lb < 4; ++lb) {
+        const int b = lb == 0 ? tv.x : lb == 1 ? tv.y : lb == 2 ? tv.z : tv.w;
+        if (b <= a) continue;
+        int lo = 1, hi = nup;  // its slot
+        while (lo < hi) {
+          const int mid = (lo + hi) >> 1;
+          if (scol[mid * kRowPad + lane] < b) lo = mid + 1;
+          else hi = mid;
+        }
+        double *p = P + 9 * lo * kRowPad + lane;
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+          const double gb = g[1 + 3 * lb + j];
+          p[j * kRowPad] = fma(w0, gb, p[j * kRowPad]);
+          p[(3 + j) * kRowPad] = fma(w1, gb, p[(3 + j) * kRowPad]);
+          p[(6 + j) * kRowPad] = fma(w2, gb, p[(6 + j) * kRowPad]);
+        }
+      }
+    }
+    const double lh = h2 * lam, mh = h2 * mu, c = 3.0 * lam + 2.0 * mu;
+    for (int s = 1; s <= nup; ++s) {
+      double *p = P + 9 * s * kRowPad + lane;
+      double e[9];
+#pragma unroll
+      for (int k = 0; k < 9; ++k) e[k] = p[k * kRowPad];
+      const double tr = mh * (e[0] + e[4] + e[8]);
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+          const double k = fma(mh, e[3 * j + i], lh * e[3 * i + j]);
+          p[(3 * i + j) * kRowPad] = i == j ? k + tr : k;
+        }
+    }
+    {  // the diagonal block: P is symmetric
+      const double tr = mh * (q[0] + q[3] + q[5]), s = lh + mh;
+      double *p = P + lane;
+      p[0] = fma(s, q[0], tr) + m;
+      p[4 * kRowPad] = fma(s, q[3], tr) + m;
+      p[8 * kRowPad] = fma(s, q[5], tr) + m;
+      p[kRowPad] = p[3 * kRowPad] = s * q[1];
+      p[2 * kRowPad] = p[6 * kRowPad] = s * q[2];
+      p[5 * kRowPad] = p[7 * kRowPad] = s * q[4];
+    }
+    mass[a] = m;
+    for (int i = 0; i < 3; ++i) KX[3 * (size_t)a + i] = c * w[i];
+  }
+  __syncwarp();
+  // Copy out row by row: the upper part, then the mirrored blocks, three at a
+  // time (27 lanes).
+  const int sub = lane / 9, e = lane - 9 * sub, et = 3 * (e % 3) + e / 3;
+  for (int r = 0; r < 32; ++r) {
+    const int dr = __shfl_sync(0xffffffffu, d, r), nr = __shfl_sync(0xffffffffu, nup, r);
+    if (nr < 0) break;
+    for (int k = lane; k < 9 * (nr + 1); k += 32) vals[9 * (size_t)dr + k] = P[k * kRowPad + r];
+    for (int s = 1 + sub; s <= nr; s += 3)
+      if (sub < 3) vals[9 * (size_t)spos[s * kRowPad + r] + e] = P[(9 * s + et) * kRowPad + r];
+  }
+}
+
+// The same for a mesh with a row too wide for shared memory: one thread per
+// vertex a adds the element blocks (in incidence order, scaled by h^2) to its
+// row in global memory, plus the lumped mass on the diagonal block; K X along
+// the way.
 __global__ void assemble_rows_kernel(int nv, const int *__restrict__ tets,
                                      const double *__restrict__ geom,
                                      const int *__restrict__ row_ptr, const int *__restrict__ cols,
@@ -125,7 +254,7 @@ __global__ void assemble_rows_kernel(int nv, const int *__restrict__ tets,
   double m = 0.0, kx[3] = {0.0, 0.0, 0.0};
   for (int idx = vt_ptr[a]; idx < vt_ptr[a + 1]; ++idx) {
     const int t = vt[idx] >> 2, la = vt[idx] & 3;
-    const double *g = geom + 13 * (size_t)t;
+    const double *g = geom + kGeom * (size_t)t;
     const double V = g[0];
     m += rho * V / 4.0;
     const double gA[3] = {g[1 + 3 * la], g[2 + 3 * la], g[3 + 3 * la]};
@@ -219,6 +348,7 @@ int mprgp_fem_create(mprgp_context *ctx, int nv, int ntet, const int *tets, cons
   std::vector<int> row_ptr(nv + 1, 0), cols;
   cols.reserve(16LL * nv);
   std::vector<int> nb;
+  int max_up = 0;
   for (int a = 0; a < nv; ++a) {
     nb.clear();
     nb.push_back(a);
@@ -230,6 +360,7 @@ int mprgp_fem_create(mprgp_context *ctx, int nv, int ntet, const int *tets, cons
     nb.erase(std::unique(nb.begin(), nb.end()), nb.end());
     cols.insert(cols.end(), nb.begin(), nb.end());
     row_ptr[a + 1] = (int)cols.size();
+    max_up = std::max(max_up, (int)(nb.end() - std::upper_bound(nb.begin(), nb.end(), a)));
   }
   auto *f = new mprgp_fem();
   f->ctx = ctx;
@@ -237,6 +368,7 @@ int mprgp_fem_create(mprgp_context *ctx, int nv, int ntet, const int *tets, cons
   f->nv = nv;
   f->ntet = ntet;
   f->nnzb = row_ptr[nv];
+  f->max_up = max_up;
   f->lam = poisson * young / ((1.0 + poisson) * (1.0 - 2.0 * poisson));
   f->mu = young / (2.0 * (1.0 + poisson));
   f->rho = rho;
@@ -246,7 +378,7 @@ int mprgp_fem_create(mprgp_context *ctx, int nv, int ntet, const int *tets, cons
   if (!rc) rc = dmalloc(&f->cols, (size_t)f->nnzb);
   if (!rc) rc = dmalloc(&f->vt_ptr, (size_t)nv + 1);
   if (!rc) rc = dmalloc(&f->vt, 4 * (size_t)ntet);
-  if (!rc) rc = dmalloc(&f->geom, 13 * (size_t)ntet);
+  if (!rc) rc = dmalloc(&f->geom, kGeom * (size_t)ntet);
   if (!rc) rc = dmalloc(&f->X, n);
   if (!rc) rc = dmalloc(&f->mass, (size_t)nv);
   if (!rc) rc = dmalloc(&f->KX, n);
@@ -293,9 +425,19 @@ int mprgp_fem_assemble(mprgp_fem *f, double h, const double gravity[3], const do
   cudaStream_t s = f->stream;
   const double g[3] = {gravity ? gravity[0] : 0.0, gravity ? gravity[1] : 0.0,
                        gravity ? gravity[2] : 0.0};
-  assemble_rows_kernel<<<(f->nv + 127) / 128, 128, 0, s>>>(
-      f->nv, f->tets, f->geom, f->row_ptr, f->cols, f->vt_ptr, f->vt, f->X, f->lam, f->mu,
-      f->rho, h * h, f->vals, f->mass, f->KX);
+  const int smem = upper_smem(f->max_up);
+  if (f->max_up < 1024 && smem <= kUpperSmemMax) {
+    if (smem > 48 * 1024)
+      FK(cudaFuncSetAttribute(assemble_upper_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              kUpperSmemMax));
+    assemble_upper_kernel<<<(f->nv + 31) / 32, 32, smem, s>>>(
+        f->nv, f->max_up, reinterpret_cast<const int4 *>(f->tets), f->geom, f->row_ptr, f->cols,
+        f->vt_ptr, f->vt, f->lam, f->mu, f->rho, h * h, f->vals, f->mass, f->KX);
+  } else {
+    assemble_rows_kernel<<<(f->nv + 127) / 128, 128, 0, s>>>(
+        f->nv, f->tets, f->geom, f->row_ptr, f->cols, f->vt_ptr, f->vt, f->X, f->lam, f->mu,
+        f->rho, h * h, f->vals, f->mass, f->KX);
+  }
   FK(cudaGetLastError());
   f->assembled = 1;
   const double *dx, *dv;

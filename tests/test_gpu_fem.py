@@ -72,3 +72,65 @@ def test_solve_from_gpu_assembly(ctx):
     assert st2.code == 0
     fem.close()
     pr.close()
+
+
+def _assembled(tets, X, E, nu, rho, h):
+    """A of the mesh by element blocks in numpy, dense."""
+    lam, mu = nu * E / ((1 + nu) * (1 - 2 * nu)), E / (2 * (1 + nu))
+    P = X.reshape(-1, 3)
+    A = np.zeros((X.size, X.size))
+    for t in tets:
+        D = (P[t[1:]] - P[t[0]]).T
+        G = np.linalg.inv(D)
+        g = np.vstack([-G.sum(axis=0), G])
+        V = abs(np.linalg.det(D)) / 6
+        for i in range(4):
+            A[3 * t[i]:3 * t[i] + 3, 3 * t[i]:3 * t[i] + 3] += rho * V / 4 * np.eye(3)
+            for j in range(4):
+                K = V * (lam * np.outer(g[i], g[j]) + mu * np.outer(g[j], g[i]) +
+                         mu * (g[i] @ g[j]) * np.eye(3))
+                A[3 * t[i]:3 * t[i] + 3, 3 * t[j]:3 * t[j] + 3] += h * h * K
+    return A
+
+
+@pytest.mark.parametrize("points,hub", [
+    (4, "first"),     # a single tet: one partial warp
+    (33, "last"),     # one row past a warp
+    (84, "first"),    # the widest row that fits shared memory (83 blocks right of the hub's)
+    (86, "first"),    # one that does not: the form in global memory
+    (150, "first"),
+    (150, "last"),    # the hub's row is as wide, its upper part empty
+])
+def test_assembly_of_a_hub(ctx, points, hub):
+    """A vertex joined to every other one, on both sides of the width that
+    shared memory holds.  Bound: a block sums at most 200 element blocks, so
+    200 eps times the largest entry, and ten times that for the gradients'
+    own rounding on random tets."""
+    rng = np.random.default_rng(points)
+    ang = np.arange(points - 1) * 0.37
+    ring = np.stack([np.cos(ang), np.sin(ang), 0.1 * np.arange(points - 1)], axis=1)
+    ring += 0.05 * rng.standard_normal(ring.shape)
+    P = np.vstack([[0.1, 0.2, -1.0], ring])
+    i = np.arange(1, points - 2)
+    tets = np.stack([np.zeros_like(i), i, i + 1, i + 2], axis=1)
+    if hub == "last":
+        P = np.vstack([P[1:], P[:1]])
+        tets = (tets - 1) % points
+    E, nu, rho, h = 1e5, 0.4, 1000.0, 0.01
+    X = P.reshape(-1).copy()
+    fem = M.FemMesh(ctx, tets.astype(np.int32), X, E, nu, rho)
+    fem.assemble(h, (0.0, -9.8, 0.0), X)
+    rp, cols, vals, b, mass = fem.get()
+    A = _assembled(tets, X, E, nu, rho, h)
+    got = np.zeros_like(A)
+    for r in range(points):
+        for k in range(rp[r], rp[r + 1]):
+            got[3 * r:3 * r + 3, 3 * cols[k]:3 * cols[k] + 3] = vals[k].reshape(3, 3)
+    assert np.abs(got - A).max() <= 2000 * 2.2e-16 * np.abs(A).max()
+    K = (A - np.kron(np.diag(mass), np.eye(3)))
+    m3 = np.repeat(mass, 3)
+    g = np.tile([0.0, -9.8, 0.0], points)
+    want = m3 * X + h * h * m3 * g + K @ X
+    scale = np.abs(K).sum(axis=1).max() * np.abs(X).max() + np.abs(want).max()
+    assert np.abs(b - want).max() <= 2000 * 2.2e-16 * scale
+    fem.close()
