@@ -78,3 +78,52 @@ def test_ica_rejects_bad_input(ctx):
     with pytest.raises(M.MPRGPError) as e:
         ctx.ica_solve(bad, qp.x0)
     assert e.value.code == M.INVALID
+
+
+@pytest.mark.parametrize("dims", [
+    (1, 1, 1),                      # 8 vertices, one CTA
+    (7, 7, 15), (4, 4, 40),         # 1,024 and 1,025: the cluster grows
+    (7, 15, 19), (18, 14, 8),       # 2,560 and 2,565: two rounds of vertices
+    (15, 15, 19), (18, 14, 17),     # 5,120 and 5,130: the largest body of the cluster form
+    (40, 40, 1),                    # wide levels: several groups of rows a warp
+])
+def test_ica_cluster_form_edges(ctx, dims):
+    """The one-cluster form at the edges of its range: the oracle's bits."""
+    qp = M.beam(*dims, extra_planes_max=2, extra_planes_min=2, plane_mode=2, seed=4)
+    xo, lo, so = H.oracle_ica(qp, qp.x0, max_it=4, tol=1e-14)
+    xg, lg, sg = ctx.ica_solve(qp, qp.x0, max_it=4, tol=1e-14)
+    assert (sg.iterations, sg.pgs_sweeps) == (so["iterations"], so["pgs_sweeps"])
+    assert np.array_equal(xg, xo) and np.array_equal(lg, lo)
+    assert sg.residual == pytest.approx(so["residual"], rel=1e-12)
+
+
+def test_ica_without_planes_and_without_sweeps(ctx):
+    """No constraint row at all, and no sweep allowed."""
+    qp = M.beam(3, 3, 9, seed=4)
+    free = M.BeamQP(qp.nv, qp.row_ptr, qp.cols, qp.vals, qp.b, qp.x0,
+                    np.zeros(qp.nv + 1, np.int32), np.zeros((0, 4)), {})
+    xo, _, so = H.oracle_ica(free, qp.x0, max_it=200, tol=1e-9)
+    xg, lg, sg = ctx.ica_solve(free, qp.x0, max_it=200, tol=1e-9)
+    assert len(lg) == 0 and np.array_equal(xg, xo)
+    assert (sg.iterations, sg.converged, sg.pgs_sweeps) == \
+        (so["iterations"], so["converged"], so["pgs_sweeps"])
+    _, l0, s0 = ctx.ica_solve(qp, qp.x0, max_it=3, tol=1e-14, gs_max_it=0)
+    assert s0.pgs_sweeps == 0 and not l0.any()
+
+
+def test_ica_unsorted_rows_take_the_grid_form(ctx):
+    """Rows whose lower blocks are not stored first are solved by the grid
+    form; the sums run in stored order, so the iterates agree to rounding: 3
+    iterations of some hundred operations a row, 1e-12 relative."""
+    qp = M.beam(4, 4, 16, extra_planes_max=1, extra_planes_min=1, plane_mode=2, seed=4)
+    rng = np.random.default_rng(1)
+    cols, vals = qp.cols.copy(), qp.vals.copy()
+    for v in range(qp.nv):
+        o = qp.row_ptr[v] + rng.permutation(qp.row_ptr[v + 1] - qp.row_ptr[v])
+        cols[qp.row_ptr[v]:qp.row_ptr[v + 1]] = qp.cols[o]
+        vals[qp.row_ptr[v]:qp.row_ptr[v + 1]] = qp.vals[o]
+    mixed = M.BeamQP(qp.nv, qp.row_ptr, cols, vals, qp.b, qp.x0, qp.plane_ptr, qp.planes, {})
+    xa, la, sa = ctx.ica_solve(qp, qp.x0, max_it=3, tol=1e-14)
+    xb, lb, sb = ctx.ica_solve(mixed, qp.x0, max_it=3, tol=1e-14)
+    assert sa.pgs_sweeps == sb.pgs_sweeps
+    assert np.linalg.norm(xa - xb) <= 1e-12 * np.linalg.norm(xa)
