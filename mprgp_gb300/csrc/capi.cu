@@ -33,6 +33,9 @@ cudaError_t launch_power_persistent(const SyncArgs &args, int fp32, int grid, cu
 cudaError_t power_persistent_max_blocks_per_sm(int fp32, int *n);
 cudaError_t launch_power_clusters(const SyncArgs &args, int fp32, int csize, cudaStream_t stream);
 cudaError_t power_clusters_max_active(int csize, int *n);
+cudaError_t launch_engine_sync(const EngineSyncArgs &args, int groups, int grid,
+                               cudaStream_t stream);
+cudaError_t engine_sync_capacity(int q, int nsm, int *ctas);
 cudaError_t launch_cluster(const ClusterArgs &args, int csize, cudaStream_t stream);
 cudaError_t cluster_max_active(int csize, int *n);
 cudaError_t launch_power_direct(int grid, int variant, int launches, const EngineArgs *d_args,
@@ -68,7 +71,7 @@ struct LaneRun {
   bool active = false;
   int n = 0, n_large = 0, quantum = 0, cluster_quantum = 0, power_launches = 0;
   bool power = false, power_graph = false, egraph = false;
-  bool power_sync = false;
+  bool power_sync = false, engine_sync = false, engine_small = false;
   int class_units[kClusterClasses] = {0, 0, 0, 0, 0};  // of the classes' power loops
   int power_variant = 0;  // the power loop's kernel variant (3: the power-step loop)
   int egraph_stream = 0;  // > 0: the engine loop ran as this many stream launches
@@ -160,6 +163,7 @@ struct mprgp_context {
   int cluster_ok[kClusterClasses] = {0, 0, 0, 0, 0};  // cluster sizes 1, 2, 4, 8, 16 usable
   int power_cluster_ok[kClusterClasses] = {0, 0, 0, 0, 0};  // ... by the power loop's kernel
   int ctas_per_sm = 0;   // persistent CTAs per SM (0 = all resident)
+  int engine_cap[2] = {0, 0};  // resident CTAs of the waiting engine (whole units, split units)
   size_t l2_bytes = 0;   // the device's L2 size
   std::map<std::tuple<int, int, int>, int> sync_cap;  // resident CTAs of the power sync loop's forms
   cudaMemPool_t pool = nullptr;      // every device array of the context's problems
@@ -745,7 +749,7 @@ int lane_reserve_units(mprgp_context *c, Lane &L, int units) {
 // CTA), or (q == 0) the persistent loop, several items a CTA; grid == 0 when
 // neither applies.
 struct SyncPlan {
-  int q = 0, smem = 0, grid = 0;
+  int q = 0, smem = 0, grid = 0, groups = 1;
 };
 int sync_capacity(mprgp_context *c, int q, int fp32, int smem) {
   const auto key = std::make_tuple(q, fp32, smem);
@@ -790,6 +794,31 @@ SyncPlan persistent_plan(mprgp_context *c, int units) {
   // CTA, streaming from DRAM, which more CTAs hide better).
   if (cap > 0 && units <= cap * (c->power_persistent ? kPowOwn : 2)) {
     const int per = (units + cap - 1) / cap;  // equally many items a CTA
+    P.grid = (units + per - 1) / per;
+  }
+  return P;
+}
+
+// The waiting engine's layout; grid == 0 when it does not apply.
+SyncPlan engine_plan(mprgp_context *c, int units, bool fp64, bool beside) {
+  SyncPlan P;
+  // FP64 items while two CTAs of each have an SM of their own: an item's eight
+  // row warps take 135 FP64 FMAs each, two warps a scheduler in one CTA
+  // (6,720 vertices with box bounds 22.6 -> 21.0 ms, 17,856 16.6 -> 16.1).
+  if (fp64 && 2 * units <= std::min(c->nsm, c->engine_cap[1])) {
+    P.q = 2;
+    P.grid = 2 * units;
+    return P;
+  }
+  // One CTA an SM with equally many items, in as few rounds as four groups
+  // give; beside cluster solves, smaller CTAs of one group, which find room as
+  // those finish (a batch of 48 takes 25.6 ms so, 28.8 with one CTA an SM).
+  const int ctas = std::min(c->nsm, c->engine_cap[0]) * (beside ? 4 : 1);
+  const int per = ctas > 0 ? (units + ctas - 1) / ctas : kEngOwn + 1;
+  if (per <= kEngOwn) {
+    const int rounds = beside ? per : (per + 3) / 4;
+    P.q = 1;
+    P.groups = (per + rounds - 1) / rounds;
     P.grid = (units + per - 1) / per;
   }
   return P;
@@ -1016,7 +1045,27 @@ int engine_begin(mprgp_context *c, int k, int n, mprgp_problem *const *probs,
   if (alone && large.one() && plan.grid == 0) plan = persistent_plan(c, large.units);
   R.power_sync = plan.grid > 0;
   const Count &sync = small_in_plan ? all : large;
-  int nunits = 0, class_unit[kClusterClasses];
+  // The instances' other phases: the waiting engine for the large ones of a
+  // synchronous run, and for small ones too when they are FP64 and few enough
+  // for split units (425 vertices: 14.2 -> 13.8 ms).
+  Count eng;
+  for (int i = 0; i < n; ++i) eng.add(probs[i], desc[R.pos[i]]);
+  const bool eng_on = alone && quantum >= 0 && !c->engine_graph && !c->stage && c->power_kernel &&
+                      c->ctas_per_sm == 0;
+  SyncPlan eplan;
+  if (eng_on && n_large == 0 && quantum == 0 && cluster_quantum == 0 && eng.fp32 == 0 &&
+      (all.n == 0 || small_in_plan))
+    eplan = engine_plan(c, eng.units, true, false);
+  if (eplan.q < 2) eplan = SyncPlan();
+  R.engine_small = eplan.grid > 0;
+  if (eng_on && n_large > 0) {
+    eng = Count();
+    for (int i = 0; i < n; ++i)
+      if (R.pos[i] < n_large) eng.add(probs[i], desc[R.pos[i]]);
+    eplan = engine_plan(c, eng.units, eng.fp32 == 0, n > n_large);
+  }
+  R.engine_sync = eplan.grid > 0;
+  int nunits = 0, class_unit[kClusterClasses], engine_unit = 0;
   {
     int want = R.power_sync ? sync.units : 0;
     for (int q = 0; q < kClusterClasses; ++q) {
@@ -1025,6 +1074,7 @@ int engine_begin(mprgp_context *c, int k, int n, mprgp_problem *const *probs,
                              : 0;
       want += R.class_units[q];
     }
+    want += eplan.grid > 0 ? eng.units : 0;
     rc = lane_reserve_units(c, L, want);
     if (rc) return rc;
     if (R.power_sync)
@@ -1042,6 +1092,11 @@ int engine_begin(mprgp_context *c, int k, int n, mprgp_problem *const *probs,
         for (int t = 0; t < (1 << q); ++t) L.h_unit[nunits++] = {R.pos[i], t, t < ni ? INT_MAX : 0, 0};
       }
     }
+    engine_unit = nunits;
+    if (R.engine_sync)
+      for (int i = 0; i < n; ++i)
+        if (R.pos[i] < n_large || R.engine_small)
+          for (int t = 0; t < nitems_of(probs[i]->nv); ++t) L.h_unit[nunits++] = {R.pos[i], t, 0, 0};
   }
   cudaStream_t s = L.stream;
   if (s != c->stream) {  // the problems' uploads and setup kernels come first
@@ -1153,6 +1208,7 @@ int engine_begin(mprgp_context *c, int k, int n, mprgp_problem *const *probs,
   if (n - n_large > 0 && small_in_plan) CK(cudaEventRecord(L.fork_ev, s));
   for (int q = 0; q < kClusterClasses; ++q) {
     if (!R.class_n[q]) continue;
+    if (R.engine_small) continue;
     ClusterArgs cargs;
     cargs.desc = L.d_desc + class_off[q];
     cargs.ninst = R.class_n[q];
@@ -1173,9 +1229,25 @@ int engine_begin(mprgp_context *c, int k, int n, mprgp_problem *const *probs,
   else if (R.power)
     CK(launch_power_direct(pgrid, R.power_variant, power_launches, L.d_args, L.d_pc, s));
   if (!R.power_sync) CK(cudaEventRecord(L.e_pow, s));  // the lane stream's power loop ends here
+  if (R.engine_sync) {
+    EngineSyncArgs ea;
+    std::memset(&ea, 0, sizeof(ea));
+    ea.desc = L.d_desc;
+    ea.states = L.d_st;
+    ea.items = L.d_unit + engine_unit;
+    ea.units = eng.units;
+    ea.q = eplan.q;
+    ea.max_phases = args.max_phases;
+    ea.wait_ns = args.wait_ns;
+    ea.total_ns = args.total_ns;
+    ea.ctl = L.ctl;
+    CK(launch_engine_sync(ea, eplan.groups, eplan.grid, s));
+  }
   for (int q = 0; q < kClusterClasses; ++q)
-    if (R.class_n[q]) CK(cudaStreamWaitEvent(s, L.join_ev[q], 0));
-  if (R.egraph && R.egraph_stream)
+    if (R.class_n[q] && !R.engine_small) CK(cudaStreamWaitEvent(s, L.join_ev[q], 0));
+  if (R.engine_sync) {
+    // launched above, beside the cluster classes
+  } else if (R.egraph && R.egraph_stream)
     CK(launch_power_direct(egrid, 2, R.egraph_stream, L.d_args, L.d_pc2, s));
   else if (R.egraph) CK(cudaGraphLaunch(eexec, s));
   else if (n_large > 0 && quantum >= 0) CK(launch_engine(args, grid, s));
@@ -1253,13 +1325,13 @@ int engine_end(mprgp_context *c, int k, mprgp_stats *stats, int *done) {
   else if (R.power)
     c->launches += R.power_launches;
   for (int q = 0; q < kClusterClasses; ++q)
-    c->launches += (R.class_n[q] ? 1 : 0) + (R.class_units[q] ? 1 : 0);
+    c->launches += (R.class_n[q] && !R.engine_small ? 1 : 0) + (R.class_units[q] ? 1 : 0);
   if (R.egraph && R.egraph_stream)
     c->launches += R.egraph_stream;
   else if (R.egraph)
     c->launches += (long long)kPowerUnroll * ((io.pc_out[1].launches + kPowerUnroll - 1) / kPowerUnroll);
   else
-    c->launches += (n_large > 0 && R.quantum >= 0) ? 1 : 0;
+    c->launches += ((n_large > 0 && R.quantum >= 0) || R.engine_small) ? 1 : 0;
   c->launches += 2;  // state scatter and gather
   c->solver_ms += ms;
   const Ctl &ctl1 = io.ctl_out;
@@ -1274,7 +1346,7 @@ int engine_end(mprgp_context *c, int k, mprgp_stats *stats, int *done) {
     const bool large = R.pos[i] < n_large;
     // an engine error concerns the engine's instances; an instance left
     // unfinished by a run that had no phase limit hit the hard phase bound
-    const bool err = (large || R.power_sync || small_power) && ctl1.err;
+    const bool err = (large || R.power_sync || R.engine_small || small_power) && ctl1.err;
     const bool unbounded = (large ? R.quantum : R.cluster_quantum) == 0;
     if (err) x.code = ctl1.err;
     else if (!finished && unbounded) x.code = MPRGP_TIMEOUT;
@@ -1422,6 +1494,11 @@ int mprgp_context_create(int device, mprgp_context **out) {
   CK(cudaMemPoolCreate(&c->pool, &props));
   unsigned long long keep = ~0ULL;  // never trim: freed blocks serve the next problem
   CK(cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &keep));
+  CK(engine_sync_capacity(1, c->nsm, &c->engine_cap[0]));
+  if (engine_sync_capacity(2, c->nsm, &c->engine_cap[1]) != cudaSuccess) {
+    cudaGetLastError();
+    c->engine_cap[1] = 0;
+  }
   CK(power_max_blocks_per_sm(0, &c->bps_power_v[0]));
   CK(power_max_blocks_per_sm(1, &c->bps_power_v[1]));
   CK(power_max_blocks_per_sm(2, &c->bps_power_v[2]));

@@ -28,9 +28,6 @@ constexpr double kEps = 1e-9;  // ScalarUtil<double>::scalar_eps (MathBasic.cpp:
 #ifndef MPRGP_PREFETCH_DIST  // chunks ahead that a streaming matrix pass prefetches into L2
 #define MPRGP_PREFETCH_DIST 1  // (0: none)
 #endif
-#ifndef MPRGP_SPMV_CHUNK
-#define MPRGP_SPMV_CHUNK 4
-#endif
 #ifndef MPRGP_SPMV_MIN_BLOCKS  // resident CTAs per SM the standalone SpMV is compiled for
 #define MPRGP_SPMV_MIN_BLOCKS 4
 #endif
@@ -263,10 +260,12 @@ __device__ __forceinline__ double seeded_uniform(unsigned long long seed, unsign
 // is one coalesced line; x is gathered per neighbour vertex.  VT is the value
 // type of A and of the accumulator (FP32 accumulation for the FP32 copy).
 struct SrcV {
+  static constexpr int kChunk = 4;
   const double *p;
   __device__ __forceinline__ void operator()(int c, double o[3]) const { ld3(p, c, o); }
 };
-struct SrcPNew {  // z - beta p   (CGStep's p = z - beta*p)
+struct SrcPNew {
+  static constexpr int kChunk = 3;  // z - beta p   (CGStep's p = z - beta*p)
   const double *z, *p;
   double beta;
   __device__ __forceinline__ void operator()(int c, double o[3]) const {
@@ -282,6 +281,7 @@ struct SrcPNew {  // z - beta p   (CGStep's p = z - beta*p)
 // FP32 sources for the mixed form: the FP32 shadow of a vector, or the CG
 // direction z - beta p formed from the shadows in FP32.
 struct SrcF {
+  static constexpr int kChunk = 3;
   const float *p;
   __device__ __forceinline__ void operator()(int c, float o[3]) const {
     const float *q = p + 3 * (size_t)c;
@@ -291,6 +291,7 @@ struct SrcF {
   }
 };
 struct SrcPNewF {
+  static constexpr int kChunk = 2;
   const float *z, *p;
   float beta;
   __device__ __forceinline__ void operator()(int c, float o[3]) const {
@@ -300,7 +301,8 @@ struct SrcPNewF {
     o[2] = fmaf(-beta, pq[2], zq[2]);
   }
 };
-struct SrcVtoF {  // FP64 vector read by an FP32 pass (standalone y = A32 x)
+struct SrcVtoF {
+  static constexpr int kChunk = 4;  // FP64 vector read by an FP32 pass (standalone y = A32 x)
   const double *p;
   __device__ __forceinline__ void operator()(int c, float o[3]) const {
     const double *q = p + 3 * (size_t)c;
@@ -341,13 +343,14 @@ __device__ __forceinline__ void prefetch_slots(const SellMatrix &A, const VT *va
 // it for the item it takes next (the next item of this launch, or its first
 // item again for the next phase) while the current item reduces, so that
 // the next item's rows do not start with a DRAM round trip.
+constexpr int kHeadSlots = 4;
 template <typename VT>
 __device__ __forceinline__ void prefetch_slice_head(const SellMatrix &A, const VT *vals, int slice,
                                                     unsigned long long pol) {
   const int j0 = ldro(A.slice_off + slice), j1 = ldro(A.slice_off + slice + 1);
   if (j1 <= j0) return;
-  if (A.cols16 && ldro(A.c16ok)) prefetch_slots<true>(A, vals, j0, min(MPRGP_SPMV_CHUNK, j1 - j0), pol);
-  else prefetch_slots<false>(A, vals, j0, min(MPRGP_SPMV_CHUNK, j1 - j0), pol);
+  if (A.cols16 && ldro(A.c16ok)) prefetch_slots<true>(A, vals, j0, min(kHeadSlots, j1 - j0), pol);
+  else prefetch_slots<false>(A, vals, j0, min(kHeadSlots, j1 - j0), pol);
 }
 __device__ __forceinline__ void prefetch_item_head(const InstDesc &D, int local_item) {
 #if MPRGP_PREFETCH_DIST > 0
@@ -384,37 +387,23 @@ __device__ __forceinline__ int col_of(const SellMatrix &A, size_t j, int lane, i
 }
 
 // Every slot below j1 is valid (padding blocks are zero and point at a real
-// row), so whole chunks of MPRGP_SPMV_CHUNK slots carry no per-slot condition
-// and all their column, value and neighbour loads can be in flight together
-// (0: columns of 8 slots fetched together, then one slot at a time).  The
+// row), so whole chunks of Src::kChunk slots carry no per-slot condition and
+// all their column, value and neighbour loads can be in flight together.  The
 // products are accumulated slot by slot in order either way, so the results
-// are the same -- and the same whichever column form is read.
+// are the same -- and the same whichever column form is read.  The chunk
+// follows from the registers a slot takes: three for the FP32 power pass
+// (48.2 us a phase on 348,145 vertices, 50.6 with four, 56.5 with five: spills;
+// and a tetrahedral grid's 15 blocks a row leave no rest), two for the CG pass,
+// which gathers two vectors (a timestep's solve 86.2 ms, 90.5 with four), four
+// for the rest (the standalone FP64 product: two 95, three and four 89 us).
 template <bool k16, typename VT, typename Src>
 __device__ __forceinline__ void spmv_row_body(const SellMatrix &A, const VT *__restrict__ vals,
                                               int lane, int vrow, int j0, int j1,
                                               unsigned long long pol, const Src &src, VT &a0,
                                               VT &a1, VT &a2) {
   int jb = j0;
-#if MPRGP_SPMV_CHUNK == 0
-  for (; jb < j1; jb += 8) {
-    int cc[8];
-#pragma unroll
-    for (int u = 0; u < 8; ++u) cc[u] = (jb + u < j1) ? col_of<k16>(A, (size_t)(jb + u), lane, vrow, pol) : -1;
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      if (cc[u] < 0) break;
-      VT m[9];
-      ld_block(vals, (size_t)(jb + u), lane, m, pol);
-      VT xv[3];
-      src(cc[u], xv);
-      a0 = fma(m[0], xv[0], a0); a0 = fma(m[1], xv[1], a0); a0 = fma(m[2], xv[2], a0);
-      a1 = fma(m[3], xv[0], a1); a1 = fma(m[4], xv[1], a1); a1 = fma(m[5], xv[2], a1);
-      a2 = fma(m[6], xv[0], a2); a2 = fma(m[7], xv[1], a2); a2 = fma(m[8], xv[2], a2);
-    }
-  }
-#else
-  for (; jb + MPRGP_SPMV_CHUNK <= j1; jb += MPRGP_SPMV_CHUNK) {
-    constexpr int K = MPRGP_SPMV_CHUNK;
+  constexpr int K = Src::kChunk;
+  for (; jb + K <= j1; jb += K) {
 #if MPRGP_PREFETCH_DIST > 0
     if (A.stream_l2 && lane == 0) {  // the slots this warp reads MPRGP_PREFETCH_DIST chunks on
       const int jp = jb + K * MPRGP_PREFETCH_DIST;
@@ -448,7 +437,6 @@ __device__ __forceinline__ void spmv_row_body(const SellMatrix &A, const VT *__r
     a1 = fma(m[3], xv[0], a1); a1 = fma(m[4], xv[1], a1); a1 = fma(m[5], xv[2], a1);
     a2 = fma(m[6], xv[0], a2); a2 = fma(m[7], xv[1], a2); a2 = fma(m[8], xv[2], a2);
   }
-#endif
 }
 
 // One row's product with a source vector; v is the row's SELL slot.  The
@@ -2974,6 +2962,7 @@ __global__ void __launch_bounds__(32)
 // wait_ns; a CTA whose wait ran out sets the error and leaves, with its
 // cluster, and the others follow when they see the error.
 __device__ __forceinline__ void cluster_sync_acq_rel() {
+  __syncwarp();  // the barrier is .aligned: the warp arrives together
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;"
                ::: "memory");
 }
@@ -3057,19 +3046,18 @@ struct SyncSums {
             need &= ~(1u << i);
           }
         }
+        if (!__any_sync(0xffffffffu, need != 0u)) break;
+        const long long now = gtimer();
+        if (since == 0) since = now;
+        bool give_up = __any_sync(0xffffffffu, now - since > wait_ns);
+        if (give_up && lane == 0) atomicCAS(&ctl->err, 0, -4);  // MPRGP_TIMEOUT
         if (++spins >= 64) {
           spins = 0;
-          const long long now = gtimer();
-          if (since == 0) since = now;
-          bool give_up = *(volatile int *)&ctl->err != 0;
-          if (now - since > wait_ns) {
-            if (lane == 0) atomicCAS(&ctl->err, 0, -4);  // MPRGP_TIMEOUT
-            give_up = true;
-          }
-          if (__any_sync(0xffffffffu, give_up)) {
-            ok = false;
-            break;
-          }
+          give_up |= *(volatile int *)&ctl->err != 0;
+        }
+        if (__any_sync(0xffffffffu, give_up)) {
+          ok = false;
+          break;
         }
       }
       if (!ok) break;
@@ -3207,6 +3195,9 @@ __device__ __forceinline__ double sq3(const float d[3]) {
   return (double)fmaf(d[0], d[0], fmaf(d[1], d[1], d[2] * d[2]));
 }
 __device__ __forceinline__ double sq3(const double d[3]) { return dot3(d, d); }
+__device__ __forceinline__ void group_bar(int g) {  // 256 threads of a larger CTA
+  asm volatile("bar.sync %0, %1;" : : "r"(1 + g), "n"(kThreads) : "memory");
+}
 __device__ __forceinline__ void block_bar(int threads) {
   asm volatile("bar.sync 0, %0;" : : "r"(threads) : "memory");
 }
@@ -3235,7 +3226,7 @@ __global__ void __launch_bounds__(kThr, kMinBlocks) power_sync_kernel(SyncArgs a
   __shared__ InstDesc sD;
   __shared__ InstState sS;
   __shared__ double sPart[2][kThreads];
-  __shared__ int sFail[2];
+  __shared__ int sFail[2], sLeave;       // this CTA's wait ran out (by phase parity); a peer's did
   const int q = kSplit ? args.q : 1;     // CTAs of a unit (a cluster)
   const int rank = q > 1 ? (int)cluster_rank() : 0;
   const int R = kThreads / q;            // rows of this CTA
@@ -3245,7 +3236,7 @@ __global__ void __launch_bounds__(kThr, kMinBlocks) power_sync_kernel(SyncArgs a
   const SyncItem unit = args.items[(int)blockIdx.x / q];
   if (threadIdx.x == 0) {
     g_staged = 0;
-    sFail[0] = sFail[1] = 0;
+    sFail[0] = sFail[1] = sLeave = 0;
   }
   {
     const int *srcd = reinterpret_cast<const int *>(args.desc + unit.inst);
@@ -3352,11 +3343,15 @@ __global__ void __launch_bounds__(kThr, kMinBlocks) power_sync_kernel(SyncArgs a
     }
     if (q > 1) {
       cluster_sync_acq_rel();
-      if (warp == 0 && lane < q && lane != rank) {  // a peer's wait ran out: all leave together
+      // A CTA whose wait ran out reads nothing of its peers, which may have
+      // left the power method and be gone; it waits for those that have not
+      // at the barrier after the loop.  They read its flag and leave too.
+      if (sFail[par]) break;
+      if (warp == 0 && lane < q && lane != rank) {
         unsigned int bad;
         asm volatile("ld.shared::cluster.u32 %0, [%1];"
                      : "=r"(bad) : "r"(dsmem_addr(&sFail[par], (unsigned int)lane)) : "memory");
-        if (bad) sFail[par] = 1;
+        if (bad) sLeave = 1;
       }
     } else {
       __syncthreads();
@@ -3382,7 +3377,7 @@ __global__ void __launch_bounds__(kThr, kMinBlocks) power_sync_kernel(SyncArgs a
     }
     if (q > 1) {
       __syncthreads();
-      if (sFail[par]) break;
+      if (sLeave) break;
     }
   }
   if (row && kl >= 0) {  // t_k and t_{k-1}, where PH_INIT looks for ev
@@ -3430,15 +3425,15 @@ __device__ __noinline__ bool wait_count(const unsigned int *count, unsigned int 
   long long since = 0;
   int spins = 0;
   while (ld_acquire(count) < target) {
+    const long long now = gtimer();
+    if (since == 0) since = now;
+    if (now - since > wait_ns) {
+      atomicCAS(&ctl->err, 0, -4);  // MPRGP_TIMEOUT
+      return false;
+    }
     if (++spins >= 64) {
       spins = 0;
-      const long long now = gtimer();
-      if (since == 0) since = now;
       if (*(volatile int *)&ctl->err != 0) return false;
-      if (now - since > wait_ns) {
-        atomicCAS(&ctl->err, 0, -4);  // MPRGP_TIMEOUT
-        return false;
-      }
     }
   }
   return true;
@@ -3553,6 +3548,295 @@ __global__ void __launch_bounds__(kStepThreads, kMinBlocks)
   }
   for (int o = 0; o < nown; ++o)
     if (sItem[o].local == 0 && threadIdx.x == 0) args.states[sItem[o].inst] = sS[o];
+}
+
+// ------------------------------------------------ waiting engine ----------
+// Every phase of a run's instances in one launch of resident CTAs that wait
+// per instance, as the power loops do: the persistent engine without its grid
+// barrier and its last CTA's finalize.
+//
+// What bounds a phase of the persistent engine besides its rows is the chain
+// that ends it: the item counter's atomic, the last CTA's sums over all items
+// (4 us for eight sums of 70 items, 9 us of 1,360), one thread's state update
+// and write-back, the barrier (2.6 us) and the reload of the state.  Here an
+// item's partials go out slot by slot, its CTA counts itself on the instance's
+// counter, and when the counter is full every CTA of the instance sums the
+// partials itself, a warp per slot in the finalize's order, and advances its
+// own copy of the state.  The partials are double buffered by phase parity: a
+// CTA writes those of phase t + 2 after the counter of phase t + 1, when every
+// CTA has read phase t's.
+//
+// Whole units: one CTA an SM, of up to four groups of 256 threads with an item
+// each at a time, and up to kEngOwn items in all.  With four CTAs an SM instead
+// the four copies of the sums and of the state update met on the SM's FP64
+// units (an FP64 warp instruction takes 64 clocks or more of one): 6-8 us for
+// the sums and 11 us for the candidate phase's update at 1,360 items, where one
+// copy takes 2 and 2.5.  Split units (few FP64 items): a cluster of q CTAs an
+// item, whose values meet through distributed shared memory in block_reduce's
+// order, so that more SMs' FP64 units work on it.
+//
+// A CTA remembers which of its items moved a candidate out of the feasible set:
+// the others' share of delta^T A delta is zero and needs no rows.  Sums and
+// transitions are the engine's, so the results are its bits.  Every wait is
+// bounded by wait_ns (a whole launch by total_ns); a CTA that gives up sets the
+// error and leaves, and the others follow when they see it.
+
+// Slot k of an instance's `nitems` item partials (contiguous), summed by one
+// warp in the finalize's order (warp_finalize): lane l forms the sums of items
+// l + 32 i, + 256, ..., adds those of i = 0..7 and closes with the shuffle
+// tree.  Rounds whose values are all zero add nothing.
+__device__ __forceinline__ double slot_sum(const double *pp, int nitems, int lane, bool is_min) {
+  double th[kThreads / 32];
+#pragma unroll
+  for (int i = 0; i < kThreads / 32; ++i) th[i] = is_min ? DBL_MAX : 0.0;
+  for (int base = 0; base < nitems; base += kThreads) {
+    double x[kThreads / 32];
+    long long any = 0;
+#pragma unroll
+    for (int i = 0; i < kThreads / 32; ++i) {
+      const int t = base + lane + 32 * i;
+      x[i] = is_min ? DBL_MAX : 0.0;
+      if (t < nitems) x[i] = pp[t];
+      any |= __double_as_longlong(x[i]);
+    }
+    if (!__any_sync(0xffffffffu, any != 0)) continue;
+    const int ni = min(kThreads / 32, (nitems - base + 31) / 32);
+#pragma unroll
+    for (int i = 0; i < kThreads / 32; ++i)
+      if (i < ni) th[i] = is_min ? fmin(th[i], x[i]) : base == 0 ? x[i] : th[i] + x[i];
+  }
+  double a = th[0];
+  const int ni = min(kThreads / 32, (nitems + 31) / 32);
+#pragma unroll
+  for (int i = 1; i < kThreads / 32; ++i)
+    if (i < ni) a = is_min ? fmin(a, th[i]) : a + th[i];
+  if (!is_min && !__any_sync(0xffffffffu, a != 0.0)) return 0.0;
+  return is_min ? warp_min(a) : warp_sum(a);
+}
+
+// The same by all warps of the CTA for an instance of more than 256 items,
+// first the sums of items l + 32 i, + 256, ... (chain i of a slot, lane l) into
+// v, then as above.
+__device__ __forceinline__ void slot_chains(const double *part, int nitems, int nrows, bool wmin,
+                                            double (*v)[kThreads]) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  for (int c = warp; c < 8 * nrows; c += nw) {
+    const int row = c >> 3, i = c & 7;
+    const bool is_min = wmin && row == nrows - 1;
+    const double *pp = part + (size_t)(is_min ? kMinSlot : row) * nitems;
+    const double id = is_min ? DBL_MAX : 0.0;
+    double acc = id;
+    for (int base = lane + 32 * i; base - lane < nitems; base += 8 * kThreads) {
+      double x[8];
+      long long any = 0;
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {
+        const int t = base + r * kThreads;
+        x[r] = t < nitems ? pp[t] : id;
+        any |= __double_as_longlong(x[r]);
+      }
+      if (!__any_sync(0xffffffffu, any != 0)) continue;
+#pragma unroll
+      for (int r = 0; r < 8; ++r)
+        if (base - lane + r * kThreads < nitems) acc = is_min ? fmin(acc, x[r]) : acc + x[r];
+    }
+    v[row][32 * i + lane] = acc;
+  }
+}
+__device__ __forceinline__ double slot_close(const double *v, int lane, bool is_min) {
+  double a = v[lane];
+#pragma unroll
+  for (int i = 1; i < kThreads / 32; ++i) a = is_min ? fmin(a, v[lane + 32 * i]) : a + v[lane + 32 * i];
+  return is_min ? warp_min(a) : warp_sum(a);
+}
+
+// block_reduce by one group of 256 threads (named barrier 1 + g).
+__device__ double group_reduce(double *part, RedBuf &red, int ns, bool with_min, int g) {
+  const int lane = threadIdx.x & 31, gt = threadIdx.x & (kThreads - 1), warp = gt >> 5;
+#pragma unroll
+  for (int k = 0; k < kPart; ++k) {
+    if (k == kMinSlot ? !with_min : k >= ns) continue;
+    red.v[k == kMinSlot ? ns : k][gt] = part[k];
+  }
+  group_bar(g);
+  const int nrows = ns + (with_min ? 1 : 0);
+  if (warp < nrows) {
+    const bool is_min = with_min && warp == ns;
+    const double *src = red.v[warp];
+    double x[kThreads / 32];
+    long long any = 0;
+#pragma unroll
+    for (int i = 0; i < kThreads / 32; ++i) {
+      x[i] = src[lane + 32 * i];
+      any |= __double_as_longlong(x[i]);
+    }
+    double acc = 0.0;
+    if (__any_sync(0xffffffffu, any != 0)) {  // an all-zero slot needs no additions
+      acc = x[0];
+#pragma unroll
+      for (int i = 1; i < kThreads / 32; ++i) acc = is_min ? fmin(acc, x[i]) : acc + x[i];
+      acc = is_min ? warp_min(acc) : warp_sum(acc);
+    }
+    if (lane == 0) red.out[warp] = acc;
+  }
+  group_bar(g);
+  double r = 0.0;
+  if (gt < ns) r = red.out[gt];
+  else if (with_min && gt == kMinSlot) r = red.out[ns];
+  return r;
+}
+
+template <int kThr, bool kSplit>
+__global__ void __launch_bounds__(kThr) engine_sync_kernel(EngineSyncArgs args) {
+  constexpr int kOwn = kSplit ? 1 : kEngOwn;
+  extern __shared__ __align__(16) unsigned char g_engine[];
+  RedBuf *red = reinterpret_cast<RedBuf *>(g_engine);  // one a group
+  __shared__ InstDesc sD[kOwn];
+  __shared__ InstState sS[kOwn];
+  __shared__ SyncItem sItem[kOwn];
+  __shared__ int sSlot[kOwn], sMoved[kOwn];  // item o: its state copy; its rows matter in PH_CG_DAD
+  __shared__ double sums[kPart];
+  __shared__ int sFail;
+  const int q = kSplit ? args.q : 1;
+  const int rank = q > 1 ? (int)cluster_rank() : 0;
+  const int R = kThreads / q;  // rows of this CTA's part of a unit
+  const int threads = blockDim.x, ngroups = kSplit ? 1 : threads / kThreads;
+  const int g = kSplit ? 0 : (int)threadIdx.x / kThreads;
+  const int gt = kSplit ? (int)threadIdx.x : (int)threadIdx.x & (kThreads - 1);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int u0 = (int)blockIdx.x / q, ustep = (int)gridDim.x / q;
+  const int nown = kSplit ? 1 : min(kOwn, (args.units - u0 + ustep - 1) / ustep);
+  const long long t_start = gtimer();
+  for (int o = 0; o < nown; ++o) {
+    const SyncItem it = args.items[u0 + o * ustep];
+    if (threadIdx.x == 0) {
+      sItem[o] = it;
+      sMoved[o] = 1;
+      int s = o;  // items of one instance share the first one's copy of the state
+      for (int p = o - 1; p >= 0; --p)
+        if (sItem[p].inst == it.inst) s = p;
+      sSlot[o] = s;
+    }
+    const int *srcd = reinterpret_cast<const int *>(args.desc + it.inst);
+    int *dstd = reinterpret_cast<int *>(&sD[o]);
+    for (int w = threadIdx.x; w < (int)(sizeof(InstDesc) / 4); w += threads) dstd[w] = ldro(srcd + w);
+    const int *srcs = reinterpret_cast<const int *>(args.states + it.inst);
+    int *dsts = reinterpret_cast<int *>(&sS[o]);
+    for (int w = threadIdx.x; w < (int)(sizeof(InstState) / 4); w += threads) dsts[w] = srcs[w];
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    g_staged = 0;
+    sFail = 0;
+    for (int o = 0; o < nown; ++o)  // the CTA of an instance's first item alone records the trace
+      if (sItem[o].local != 0 || rank != 0) sD[o].trace = nullptr;
+  }
+  __syncthreads();
+  for (int t = 0; t < args.max_phases; ++t) {
+    const int par = t & 1;
+    bool ran = false;
+    for (int o = 0; o < nown; ++o) ran |= sS[sSlot[o]].phase != PH_DONE;
+    if (!ran) break;
+    for (int o = g; o < nown; o += ngroups) {
+      const InstDesc &D = sD[o];
+      const InstState &S = sS[sSlot[o]];
+      const int phase = S.phase;
+      if (phase == PH_DONE) continue;
+      const int ns = nslots(phase);
+      const bool wmin = phase == PH_PL_SPMV;
+      double *pp = D.part + (size_t)par * kPart * D.nitems + sItem[o].local;
+      if (phase == PH_CG_DAD && !sMoved[o]) {
+        if (gt == 0) pp[0] = 0.0;
+      } else {
+        double part[kPart];
+#pragma unroll
+        for (int k = 0; k < kPart; ++k) part[k] = (k == kMinSlot) ? DBL_MAX : 0.0;
+        const int slot = sItem[o].local * kThreads + rank * R + gt;
+        if (gt < R && slot < D.nv) row_op(D, S, row_vertex(D.A, slot), slot, part);
+        if (!kSplit) {
+          const double r = group_reduce(part, red[g], ns, wmin, g);
+          if (gt < ns) pp[(size_t)gt * D.nitems] = r;
+          else if (wmin && gt == kMinSlot) pp[(size_t)kMinSlot * D.nitems] = r;
+          // the candidate phase's second sum counts the rows P(y) moved (a
+          // split unit's CTAs would have to agree, so they keep the flag)
+          if (phase == PH_CG_YF && gt == 1) sMoved[o] = r != 0.0;
+        } else {
+          if (gt < R) {
+#pragma unroll
+            for (int k = 0; k < kPart; ++k) {
+              if (k == kMinSlot ? !wmin : k >= ns) continue;
+              red[0].v[k == kMinSlot ? ns : k][gt] = part[k];
+            }
+          }
+          cluster_sync_acq_rel();
+          // row k of the sums by rank k mod q, in block_reduce's order
+          for (int k = rank + q * warp; k < ns + (wmin ? 1 : 0); k += q * (kThr / 32)) {
+            const bool is_min = wmin && k == ns;
+            double x[kThreads / 32], acc;
+#pragma unroll
+            for (int i = 0; i < kThreads / 32; ++i)
+              x[i] = ld_dsmem(dsmem_addr(&red[0].v[k][(lane + 32 * i) & (R - 1)],
+                                         (unsigned int)((32 * i) / R)));
+            acc = x[0];
+#pragma unroll
+            for (int i = 1; i < kThreads / 32; ++i) acc = is_min ? fmin(acc, x[i]) : acc + x[i];
+            acc = is_min ? warp_min(acc) : warp_sum(acc);
+            if (lane == 0) pp[(size_t)(is_min ? kMinSlot : k) * D.nitems] = acc;
+          }
+        }
+      }
+      if (kSplit) __syncthreads();
+      else group_bar(g);
+      if (gt == 0) red_add_release(D.cnt, 1u);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int o = 0; o < nown; ++o)
+        if (sSlot[o] == o && sS[o].phase != PH_DONE &&
+            !wait_count(sD[o].cnt, (unsigned int)((t + 1) * sD[o].nitems * q), args.ctl, args.wait_ns))
+          sFail = 1;
+      if (gtimer() - t_start > args.total_ns) {
+        atomicCAS(&args.ctl->err, 0, -4);  // MPRGP_TIMEOUT
+        sFail = 1;
+      }
+    }
+    __syncthreads();
+    if (sFail) {
+      // A peer whose wait for this phase ended well goes on to the next one's
+      // cluster barrier and reads this CTA's values after it: meet it there,
+      // read nothing, and stay until it arrives once more.  It does, since
+      // the next phase's counter never fills without this CTA.
+      if (q > 1) cluster_sync_acq_rel();
+      break;
+    }
+    for (int o = 0; o < nown; ++o) {
+      if (sSlot[o] != o || sS[o].phase == PH_DONE) continue;
+      const InstDesc &D = sD[o];
+      const int phase = sS[o].phase, ns = nslots(phase);
+      const bool wmin = phase == PH_PL_SPMV;
+      const int nrows = ns + (wmin ? 1 : 0);
+      const double *pp = D.part + (size_t)par * kPart * D.nitems;
+      const bool many = !kSplit && D.nitems > kThreads;
+      if (many) {
+        slot_chains(pp, D.nitems, nrows, wmin, red[0].v);
+        __syncthreads();
+      }
+      for (int k = warp; k < kPart; k += threads / 32) {
+        const bool is_min = k == kMinSlot;
+        double a = 0.0;
+        if (k < ns || (wmin && is_min))
+          a = many ? slot_close(red[0].v[is_min ? ns : k], lane, is_min)
+                   : slot_sum(pp + (size_t)k * D.nitems, D.nitems, lane, is_min);
+        if (lane == 0) sums[k] = a;
+      }
+      __syncthreads();
+      if (threadIdx.x == 0) advance(D, sS[o], sums);
+      __syncthreads();
+    }
+  }
+  for (int o = 0; o < nown; ++o)
+    if (rank == 0 && sItem[o].local == 0 && threadIdx.x == 0) args.states[sItem[o].inst] = sS[sSlot[o]];
+  if (q > 1) cluster_sync_acq_rel();  // no CTA leaves while another may read its values
 }
 
 // ---------------------------------------------------- cluster solver -----
@@ -3782,8 +4066,8 @@ __global__ void __launch_bounds__(256, MPRGP_SPMV_MIN_BLOCKS) spmv_kernel(SellMa
 // (the run's desc entries point into it), so a launch can fetch an item's
 // desc and state in one round of loads.  Between runs each state lives with
 // its problem (`home`).  Before a run the fresh instances' initial states are
-// already in the array (uploaded from the host) and their phase-item counters
-// are cleared, the others' states are copied in from home; after it every
+// already in the array (uploaded from the host), the others' states are copied
+// in from home, and every instance's counter is cleared; after it every
 // state is copied back home (the array then also goes to the host).  One CTA
 // per instance.
 static_assert(sizeof(InstState) % 8 == 0, "InstState is copied as 8-byte words");
@@ -3799,10 +4083,8 @@ __global__ void state_scatter_kernel(const InstDesc *__restrict__ desc, int n, I
   if (j >= n) return;
   if (clear_records)
     for (int i = threadIdx.x; i <= 4 * desc[j].nitems; i += blockDim.x) desc[j].part[i] = 0.0;
-  if (fresh[j]) {
-    if (threadIdx.x == 0) *desc[j].cnt = 0u;
-    return;
-  }
+  if (threadIdx.x == 0) *desc[j].cnt = 0u;
+  if (fresh[j]) return;
   const unsigned long long *src = reinterpret_cast<const unsigned long long *>(home[j]);
   unsigned long long *dst = reinterpret_cast<unsigned long long *>(states + j);
   for (int w = threadIdx.x; w < kStateWords; w += blockDim.x) dst[w] = src[w];
@@ -3834,6 +4116,57 @@ cudaError_t launch_engine(const EngineArgs &args, int grid, cudaStream_t stream)
   void *params[] = {(void *)&args};
   return cudaLaunchCooperativeKernel((const void *)engine_kernel, dim3(grid), dim3(kThreads),
                                      params, (size_t)args.stage_bytes, stream);
+}
+// The waiting engine with q CTAs a unit, or (q == 1) CTAs of `groups` groups.
+static void engine_sync_config(int q, int groups, int grid, cudaStream_t stream,
+                               cudaLaunchConfig_t &cfg, cudaLaunchAttribute (&at)[2]) {
+  cfg = {};
+  cfg.gridDim = dim3((unsigned int)grid);
+  cfg.blockDim = dim3(q > 1 ? kThreads / 2 : groups * kThreads);
+  cfg.dynamicSmemBytes = sizeof(RedBuf) * (q > 1 ? 1 : groups);
+  cfg.stream = stream;
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = (unsigned int)q;
+  at[1].val.clusterDim.y = 1;
+  at[1].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = q > 1 ? 2 : 1;
+}
+static const void *engine_sync_fn(int q) {
+  return q > 1 ? (const void *)engine_sync_kernel<kThreads / 2, true>
+               : (const void *)engine_sync_kernel<4 * kThreads, false>;
+}
+cudaError_t launch_engine_sync(const EngineSyncArgs &args, int groups, int grid,
+                               cudaStream_t stream) {
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute at[2];
+  engine_sync_config(args.q, groups, grid, stream, cfg, at);
+  void *params[] = {(void *)&args};
+  return cudaLaunchKernelExC(&cfg, engine_sync_fn(args.q), params);
+}
+// CTAs of that form that can be resident at once (q == 1: of four groups).
+cudaError_t engine_sync_capacity(int q, int nsm, int *ctas) {
+  int n = 0;
+  cudaError_t e = cudaFuncSetAttribute(engine_sync_fn(q), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)sizeof(RedBuf) * 4);
+  *ctas = 0;
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute at[2];
+  engine_sync_config(q, 4, q, nullptr, cfg, at);
+  if (q == 1) {
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, engine_sync_fn(1), 4 * kThreads,
+                                                      cfg.dynamicSmemBytes);
+    *ctas = n * nsm;
+    return e;
+  }
+  cfg.attrs = at + 1;
+  cfg.numAttrs = 1;
+  e = cudaOccupancyMaxActiveClusters(&n, engine_sync_fn(q), &cfg);
+  *ctas = n * q;
+  return e;
 }
 // Resident engine CTAs per SM with `stage_bytes` of dynamic shared memory.
 cudaError_t engine_max_blocks_per_sm(int *n, int stage_bytes) {

@@ -153,6 +153,7 @@ struct PowCtl {
 };
 constexpr int kPowerUnroll = 8;  // power launches per evaluation of the loop condition
 constexpr int kPowOwn = 4;       // items per CTA of the persistent power loop
+constexpr int kEngOwn = 16;      // ... and of the waiting engine
 constexpr int kCodeInvalid = -5;  // MPRGP_INVALID: the result code of an invalid instance
 
 // Small instances run on the cluster solver: one thread-block cluster per
@@ -181,6 +182,15 @@ struct SyncArgs {
   const SyncItem *items;
   int units, q;  // q: CTAs of a unit
   long long wait_ns;
+  Ctl *ctl;
+};
+
+struct EngineSyncArgs {
+  const InstDesc *desc;
+  InstState *states;
+  const SyncItem *items;  // limit unused
+  int units, q, max_phases, pad;
+  long long wait_ns, total_ns;
   Ctl *ctl;
 };
 
