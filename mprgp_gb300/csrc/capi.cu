@@ -21,6 +21,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/mprgp_gpu.h"
+#include "coop_gate.h"
 #include "engine.h"
 #include "nvtx_ranges.h"
 
@@ -33,9 +34,9 @@ cudaError_t launch_power_persistent(const SyncArgs &args, int fp32, int grid, cu
 cudaError_t power_persistent_max_blocks_per_sm(int fp32, int *n);
 cudaError_t launch_power_clusters(const SyncArgs &args, int fp32, int csize, cudaStream_t stream);
 cudaError_t power_clusters_max_active(int csize, int *n);
-cudaError_t launch_engine_sync(const EngineSyncArgs &args, int groups, int grid,
+cudaError_t launch_engine_sync(const EngineSyncArgs &args, int groups, int grid, int smem,
                                cudaStream_t stream);
-cudaError_t engine_sync_capacity(int q, int nsm, int *ctas);
+cudaError_t engine_sync_capacity(int q, int smem, int nsm, int *ctas);
 cudaError_t launch_cluster(const ClusterArgs &args, int csize, cudaStream_t stream);
 cudaError_t cluster_max_active(int csize, int *n);
 cudaError_t launch_power_direct(int grid, int variant, int launches, const EngineArgs *d_args,
@@ -50,16 +51,23 @@ void launch_planes_setup(int nv, const int *plane_ptr, const double *in, double 
 void launch_planes_axis(int m, const double *in, unsigned char *axis, cudaStream_t st);
 void launch_state_scatter(const InstDesc *desc, int n, InstState *states, InstState *const *home,
                           const int *fresh, int clear_records, cudaStream_t st);
-cudaError_t power_sync_capacity(int q, int fp32, int smem, int nsm, int *ctas);
-cudaError_t launch_power_sync(const SyncArgs &args, int fp32, int grid, int smem,
+cudaError_t power_sync_capacity(int q, int fp32, int comps, int smem, int nsm, int *ctas);
+cudaError_t launch_power_sync(const SyncArgs &args, int fp32, int comps, int grid, int smem,
                               cudaStream_t stream);
 void launch_state_gather(const InstDesc *desc, int n, InstState *states, InstState *const *home,
                          cudaStream_t st);
-void launch_spmv(const SellMatrix &A, int nv, bool fp32, const double *x, double *y,
+void launch_spmv(const SellMatrix &A, int nv, int nsm, bool fp32, const double *x, double *y,
                  cudaStream_t st);
 }  // namespace mprgp
 
 using namespace mprgp;
+
+namespace mprgp {
+CoopGate &coop_gate(int device) {
+  static CoopGate gates[64];
+  return gates[device & 63];
+}
+}  // namespace mprgp
 
 // Device and pinned-host resources of one engine lane, and the run in flight
 // on it.  Lane 0 runs on the context stream (the synchronous calls); the
@@ -163,9 +171,8 @@ struct mprgp_context {
   int cluster_ok[kClusterClasses] = {0, 0, 0, 0, 0};  // cluster sizes 1, 2, 4, 8, 16 usable
   int power_cluster_ok[kClusterClasses] = {0, 0, 0, 0, 0};  // ... by the power loop's kernel
   int ctas_per_sm = 0;   // persistent CTAs per SM (0 = all resident)
-  int engine_cap[2] = {0, 0};  // resident CTAs of the waiting engine (whole units, split units)
   size_t l2_bytes = 0;   // the device's L2 size
-  std::map<std::tuple<int, int, int>, int> sync_cap;  // resident CTAs of the power sync loop's forms
+  std::map<std::tuple<int, int, int>, int> sync_cap;  // resident CTAs of the waiting loops' forms
   cudaMemPool_t pool = nullptr;      // every device array of the context's problems
   mprgp_problem *scratch = nullptr;
   int bps_power = 0;
@@ -749,14 +756,14 @@ int lane_reserve_units(mprgp_context *c, Lane &L, int units) {
 // CTA), or (q == 0) the persistent loop, several items a CTA; grid == 0 when
 // neither applies.
 struct SyncPlan {
-  int q = 0, smem = 0, grid = 0, groups = 1;
+  int q = 0, comps = 1, smem = 0, grid = 0, groups = 1;
 };
-int sync_capacity(mprgp_context *c, int q, int fp32, int smem) {
-  const auto key = std::make_tuple(q, fp32, smem);
+int sync_capacity(mprgp_context *c, int q, int fp32, int comps, int smem) {
+  const auto key = std::make_tuple(q, 4 * fp32 + comps, smem);
   auto it = c->sync_cap.find(key);
   if (it == c->sync_cap.end()) {
     int n = 0;
-    if (power_sync_capacity(q, fp32, smem, c->nsm, &n) != cudaSuccess) {
+    if (power_sync_capacity(q, fp32, comps, smem, c->nsm, &n) != cudaSuccess) {
       cudaGetLastError();
       n = 0;
     }
@@ -766,22 +773,37 @@ int sync_capacity(mprgp_context *c, int q, int fp32, int smem) {
 }
 SyncPlan sync_plan(mprgp_context *c, int units, int max_slots, int fp32) {
   SyncPlan P;
-  // The fewest CTAs an item whose slices fit shared memory, or twice as many
-  // (three instead of two eighths of an SM's rows a CTA can pack an SM better).
-  // 1,760 vertices mixed: 4.85 us a phase with q = 1, 5.5 with 2, 4 or 8;
-  // 17,856 in FP64: 13.7 with q = 2, 14.2 with 4, 18.3 with 8.
   const int slice = max_slots * kSlice * (9 * (fp32 ? 4 : 8) + 4);
+  auto bytes = [&](int q) {  // a CTA's slices, in few distinct sizes
+    return ((long long)slice * (kThreads / kSlice / q) + 4095) / 4096 * 4096;
+  };
+  auto fits = [&](int q, int comps) {
+    if (bytes(q) > kSyncStageBytes || units * q > sync_capacity(c, q, fp32, comps, (int)bytes(q)))
+      return false;
+    P.q = q;
+    P.comps = comps;
+    P.smem = (int)bytes(q);
+    P.grid = units * q;
+    return true;
+  };
+  // FP64 rows by three threads, one a component, while each scheduler of an SM
+  // gets one or two such warps: a row's 135 FP64 FMAs (15 blocks) take 6 us as
+  // one warp's chain, a component's 45 take 2.
+  // 425 vertices: 10.7 -> 7.7 us a phase, 6,720: 12.3 -> 9.3.  (Three quarters
+  // of the SMs: clusters do not pack them further, and two CTAs on an SM cost
+  // what the split gains: 9,464 vertices 13.2 us, 12.6 with whole rows.)
+  if (!fp32)
+    for (int q = 8; q >= 4; q /= 2)
+      if (4 * units * q <= 3 * c->nsm && fits(q, 3)) return P;
+  // Else the fewest CTAs an item whose slices fit shared memory, or twice as
+  // many (smaller CTAs can pack an SM better).  1,760 vertices mixed: 4.85 us
+  // a phase with q = 1, 5.5 with 2, 4 or 8; 17,856 in FP64: 13.7 with q = 2,
+  // 14.2 with 4, 18.3 with 8.
   int tried = 0;
   for (int q = 1; q <= kThreads / kSlice && tried < 2; q *= 2) {
-    const long long bytes = (long long)slice * (kThreads / kSlice / q);
-    const long long smem = (bytes + 4095) / 4096 * 4096;  // few distinct sizes
-    if (smem > kSyncStageBytes) continue;
+    if (bytes(q) > kSyncStageBytes) continue;
     ++tried;
-    if (units * q > sync_capacity(c, q, fp32, (int)smem)) continue;
-    P.q = q;
-    P.smem = (int)smem;
-    P.grid = units * q;
-    break;
+    if (fits(q, 1)) break;
   }
   return P;
 }
@@ -799,13 +821,40 @@ SyncPlan persistent_plan(mprgp_context *c, int units) {
   return P;
 }
 
+int engine_capacity(mprgp_context *c, int q, int smem) {
+  const auto key = std::make_tuple(q, -1, smem);
+  auto it = c->sync_cap.find(key);
+  if (it == c->sync_cap.end()) {
+    int n = 0;
+    if (engine_sync_capacity(q, smem, c->nsm, &n) != cudaSuccess) {
+      cudaGetLastError();
+      n = 0;
+    }
+    it = c->sync_cap.emplace(key, n).first;
+  }
+  return it->second;
+}
 // The waiting engine's layout; grid == 0 when it does not apply.
-SyncPlan engine_plan(mprgp_context *c, int units, bool fp64, bool beside) {
+SyncPlan engine_plan(mprgp_context *c, int units, int max_slots, bool fp64, bool beside) {
   SyncPlan P;
-  // FP64 items while two CTAs of each have an SM of their own: an item's eight
-  // row warps take 135 FP64 FMAs each, two warps a scheduler in one CTA
-  // (6,720 vertices with box bounds 22.6 -> 21.0 ms, 17,856 16.6 -> 16.1).
-  if (fp64 && 2 * units <= std::min(c->nsm, c->engine_cap[1])) {
+  // FP64 items: eight or four CTAs of three threads a row, with their matrix
+  // slices in shared memory, while three quarters of the SMs hold them (the
+  // rule of sync_plan); else two CTAs while each has an SM of its own: an
+  // item's eight row warps take 135 FP64 FMAs each, two warps a scheduler in
+  // one CTA (17,856 vertices 16.6 -> 16.1 ms with two).
+  if (fp64)
+    for (int q = 8; q >= 4; q /= 2) {
+      const long long bytes = (long long)max_slots * kSlice * (9 * 8 + 4) * (kThreads / kSlice / q);
+      const long long smem = (bytes + 4095) / 4096 * 4096;
+      if (4 * units * q > 3 * c->nsm || smem > kEngStageBytes ||
+          units * q > engine_capacity(c, q, (int)smem))
+        continue;
+      P.q = q;
+      P.smem = (int)smem;
+      P.grid = q * units;
+      return P;
+    }
+  if (fp64 && 2 * units <= std::min(c->nsm, engine_capacity(c, 2, 0))) {
     P.q = 2;
     P.grid = 2 * units;
     return P;
@@ -813,7 +862,7 @@ SyncPlan engine_plan(mprgp_context *c, int units, bool fp64, bool beside) {
   // One CTA an SM with equally many items, in as few rounds as four groups
   // give; beside cluster solves, smaller CTAs of one group, which find room as
   // those finish (a batch of 48 takes 25.6 ms so, 28.8 with one CTA an SM).
-  const int ctas = std::min(c->nsm, c->engine_cap[0]) * (beside ? 4 : 1);
+  const int ctas = std::min(c->nsm, engine_capacity(c, 1, 0)) * (beside ? 4 : 1);
   const int per = ctas > 0 ? (units + ctas - 1) / ctas : kEngOwn + 1;
   if (per <= kEngOwn) {
     const int rounds = beside ? per : (per + 3) / 4;
@@ -1042,7 +1091,10 @@ int engine_begin(mprgp_context *c, int k, int n, mprgp_problem *const *probs,
     plan = sync_plan(c, all.units, all.slots, all.fp32 ? 1 : 0);
     small_in_plan = plan.grid > 0;
   }
-  if (alone && large.one() && plan.grid == 0) plan = persistent_plan(c, large.units);
+  // ... and on a server's power lane in the mixed form (a burst of 48 requests
+  // 39.3 -> 33.2 ms; in FP64, 91.3 -> 92.3, the graph loop stays)
+  if ((alone || (k == 3 && large.fp32 > 0)) && large.one() && plan.grid == 0)
+    plan = persistent_plan(c, large.units);
   R.power_sync = plan.grid > 0;
   const Count &sync = small_in_plan ? all : large;
   // The instances' other phases: the waiting engine for the large ones of a
@@ -1055,14 +1107,14 @@ int engine_begin(mprgp_context *c, int k, int n, mprgp_problem *const *probs,
   SyncPlan eplan;
   if (eng_on && n_large == 0 && quantum == 0 && cluster_quantum == 0 && eng.fp32 == 0 &&
       (all.n == 0 || small_in_plan))
-    eplan = engine_plan(c, eng.units, true, false);
+    eplan = engine_plan(c, eng.units, eng.slots, true, false);
   if (eplan.q < 2) eplan = SyncPlan();
   R.engine_small = eplan.grid > 0;
   if (eng_on && n_large > 0) {
     eng = Count();
     for (int i = 0; i < n; ++i)
       if (R.pos[i] < n_large) eng.add(probs[i], desc[R.pos[i]]);
-    eplan = engine_plan(c, eng.units, eng.fp32 == 0, n > n_large);
+    eplan = engine_plan(c, eng.units, eng.slots, eng.fp32 == 0, n > n_large);
   }
   R.engine_sync = eplan.grid > 0;
   int nunits = 0, class_unit[kClusterClasses], engine_unit = 0;
@@ -1201,8 +1253,11 @@ int engine_begin(mprgp_context *c, int k, int n, mprgp_problem *const *probs,
     sa.items = L.d_unit;
     sa.units = sync.units;
     sa.q = std::max(1, plan.q);
-    if (plan.q > 0) CK(launch_power_sync(sa, sync.fp32 ? 1 : 0, plan.grid, plan.smem, s));
-    else CK(launch_power_persistent(sa, sync.fp32 ? 1 : 0, plan.grid, s));
+    const int fp32 = sync.fp32 ? 1 : 0;
+    CK(gated_launch(s, [&] {
+      return plan.q > 0 ? launch_power_sync(sa, fp32, plan.comps, plan.grid, plan.smem, s)
+                        : launch_power_persistent(sa, fp32, plan.grid, s);
+    }));
     CK(cudaEventRecord(L.e_pow, s));
   }
   if (n - n_large > 0 && small_in_plan) CK(cudaEventRecord(L.fork_ev, s));
@@ -1241,7 +1296,7 @@ int engine_begin(mprgp_context *c, int k, int n, mprgp_problem *const *probs,
     ea.wait_ns = args.wait_ns;
     ea.total_ns = args.total_ns;
     ea.ctl = L.ctl;
-    CK(launch_engine_sync(ea, eplan.groups, eplan.grid, s));
+    CK(gated_launch(s, [&] { return launch_engine_sync(ea, eplan.groups, eplan.grid, eplan.smem, s); }));
   }
   for (int q = 0; q < kClusterClasses; ++q)
     if (R.class_n[q] && !R.engine_small) CK(cudaStreamWaitEvent(s, L.join_ev[q], 0));
@@ -1250,7 +1305,7 @@ int engine_begin(mprgp_context *c, int k, int n, mprgp_problem *const *probs,
   } else if (R.egraph && R.egraph_stream)
     CK(launch_power_direct(egrid, 2, R.egraph_stream, L.d_args, L.d_pc2, s));
   else if (R.egraph) CK(cudaGraphLaunch(eexec, s));
-  else if (n_large > 0 && quantum >= 0) CK(launch_engine(args, grid, s));
+  else if (n_large > 0 && quantum >= 0) CK(gated_launch(s, [&] { return launch_engine(args, grid, s); }));
   CK(cudaEventRecord(L.e1, s));
   if (R.power) CK(cudaMemcpyAsync(&io.pc_out[0], L.d_pc, sizeof(PowCtl), cudaMemcpyDeviceToHost, s));
   if (R.egraph) CK(cudaMemcpyAsync(&io.pc_out[1], L.d_pc2, sizeof(PowCtl), cudaMemcpyDeviceToHost, s));
@@ -1494,11 +1549,6 @@ int mprgp_context_create(int device, mprgp_context **out) {
   CK(cudaMemPoolCreate(&c->pool, &props));
   unsigned long long keep = ~0ULL;  // never trim: freed blocks serve the next problem
   CK(cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &keep));
-  CK(engine_sync_capacity(1, c->nsm, &c->engine_cap[0]));
-  if (engine_sync_capacity(2, c->nsm, &c->engine_cap[1]) != cudaSuccess) {
-    cudaGetLastError();
-    c->engine_cap[1] = 0;
-  }
   CK(power_max_blocks_per_sm(0, &c->bps_power_v[0]));
   CK(power_max_blocks_per_sm(1, &c->bps_power_v[1]));
   CK(power_max_blocks_per_sm(2, &c->bps_power_v[2]));
@@ -1930,7 +1980,7 @@ int mprgp_problem_spmv(mprgp_problem *p, const double *x_dev, double *y_dev, int
   A.bad = p->bad;
 #endif
   p->ctx->launches++;
-  launch_spmv(A, p->nv, f32, x_dev, y_dev, p->ctx->stream);
+  launch_spmv(A, p->nv, p->ctx->nsm, f32, x_dev, y_dev, p->ctx->stream);
   CK(cudaGetLastError());
   return MPRGP_OK;
 }

@@ -1234,6 +1234,27 @@ __device__ __forceinline__ double ratio_v(const InstDesc &, const VSep &C, const
 
 __device__ __forceinline__ double *B(const InstDesc &D, int i) { return D.buf[i]; }
 
+// Products formed before the row work, by three threads a row (the waiting
+// engine's split units): product `which` of row ri, component c, at
+// g_pre[which * 3 + c][ri].
+constexpr int kPreRows = kThreads / 4;  // rows of a split unit's CTA, at most
+__shared__ double g_pre[6][kPreRows];
+__device__ __forceinline__ int pre_row() {  // three warps carry 32 rows' components
+  return (int)(threadIdx.x >> 5) / 3 * 32 + (int)(threadIdx.x & 31);
+}
+__device__ __forceinline__ void pre_product(int which, double out[3]) {
+  const int ri = pre_row();
+#pragma unroll
+  for (int c = 0; c < 3; ++c) out[c] = g_pre[3 * which + c][ri];
+}
+// A row's product with an FP64 source: formed before (kPre) or here.
+template <bool kPre, typename Src>
+__device__ __forceinline__ void row_product(const InstDesc &D, int slot, int which, const Src &src,
+                                            double out[3]) {
+  if constexpr (kPre) pre_product(which, out);
+  else spmv_row<double>(D.A, D.A.v64, slot, src, out);
+}
+
 // Shared epilogue once g is final for a row and the face is re-decided:
 // DECIDE_FACE(x); PHI(g); z = precond; p = z; then the loop top's BETA and
 // the sums |phi+beta|^2, beta.beta, PHITPHI, z.g, COUNT_CONSTRAINTS.
@@ -1439,6 +1460,7 @@ __device__ __forceinline__ void row_project(const InstDesc &D, int xin, int xout
   }
 }
 
+template <bool kPre>
 __device__ __noinline__ void row_init(const InstDesc &D, const InstState &S, int v, int slot,
                                       double *part) {
   if (S.phase == PH_PROJ0 || S.phase == PH_FINAL) {
@@ -1460,13 +1482,14 @@ __device__ __noinline__ void row_init(const InstDesc &D, const InstState &S, int
     st3(D.ev, v, t);
   }
   double x[3], ax[3];
-  spmv_row<double>(D.A, D.A.v64, slot, SrcV{B(D, B_X0 + S.xc)}, ax);
+  row_product<kPre>(D, slot, 0, SrcV{B(D, B_X0 + S.xc)}, ax);
   ld3(B(D, B_X0 + S.xc), v, x);
   const double g[3] = {ax[0] - ldro(D.b + 3 * (size_t)v), ax[1] - ldro(D.b + 3 * (size_t)v + 1),
                        ax[2] - ldro(D.b + 3 * (size_t)v + 2)};
   epilogue(D, S, v, x, g, part);
 }
 
+template <bool kPre>
 __device__ __noinline__ void row_cg_spmv(const InstDesc &D, const InstState &S, int v, int slot,
                                          double *part) {
   const bool f32 = D.prec == PREC_MIXED;
@@ -1477,15 +1500,18 @@ __device__ __noinline__ void row_cg_spmv(const InstDesc &D, const InstState &S, 
     ld3(pp, v, p);
     if (S.phase == PH_CG_ENTRY && !S.g_cons) {
       double ax[3];
-      spmv_row<double>(D.A, D.A.v64, slot, SrcV{B(D, B_X0 + S.xc)}, ax);
+      row_product<kPre>(D, slot, 1, SrcV{B(D, B_X0 + S.xc)}, ax);
       double e[3];
 #pragma unroll
       for (int d = 0; d < 3; ++d) e[d] = (ax[d] - ldro(D.b + 3 * (size_t)v + d)) - g[d];
       st3(B(D, B_E), v, e);
       part[2] += dot3(p, e);
     }
-    spmv_any(D, f32 && S.phase != PH_PL_SPMV, slot, SrcV{pp},
-             SrcF{f32 ? D.buf32[F_P0 + S.pc] : nullptr}, ap);
+    if constexpr (kPre)
+      pre_product(0, ap);
+    else
+      spmv_any(D, f32 && S.phase != PH_PL_SPMV, slot, SrcV{pp},
+               SrcF{f32 ? D.buf32[F_P0 + S.pc] : nullptr}, ap);
   } else {
     const double *zz = B(D, B_Z0 + S.zc), *po = B(D, B_P0 + S.pc);
     double z[3];
@@ -1496,9 +1522,12 @@ __device__ __noinline__ void row_cg_spmv(const InstDesc &D, const InstState &S, 
     st3(B(D, B_P0 + (S.pc ^ 1)), v, p);
     const bool f32p = f32 && S.phase != PH_PL_SPMV;
     if (f32p) st3f(D.buf32[F_P0 + (S.pc ^ 1)], v, p);
-    spmv_any(D, f32p, slot, SrcPNew{zz, po, S.beta_cg},
-             SrcPNewF{f32p ? D.buf32[F_Z0 + S.zc] : nullptr,
-                      f32p ? D.buf32[F_P0 + S.pc] : nullptr, (float)S.beta_cg}, ap);
+    if constexpr (kPre)
+      pre_product(0, ap);
+    else
+      spmv_any(D, f32p, slot, SrcPNew{zz, po, S.beta_cg},
+               SrcPNewF{f32p ? D.buf32[F_Z0 + S.zc] : nullptr,
+                        f32p ? D.buf32[F_P0 + S.pc] : nullptr, (float)S.beta_cg}, ap);
     if (S.e_nz && S.phase == PH_CG_SPMV) {
       double e[3];
       ld3(B(D, B_E), v, e);
@@ -1642,6 +1671,7 @@ __device__ __noinline__ void row_cg_yf(const InstDesc &D, const InstState &S, in
 }
 
 // delta^T A delta over the rows where P(y) moved y (rare).
+template <bool kPre>
 __device__ __noinline__ void row_cg_dad(const InstDesc &D, const InstState &S, int v, int slot,
                                         double *part) {
   (void)S;
@@ -1649,7 +1679,7 @@ __device__ __noinline__ void row_cg_dad(const InstDesc &D, const InstState &S, i
   ld3(B(D, B_W), v, dl);
   if (dl[0] == 0.0 && dl[1] == 0.0 && dl[2] == 0.0) return;
   double ad[3];
-  spmv_row<double>(D.A, D.A.v64, slot, SrcV{B(D, B_W)}, ad);
+  row_product<kPre>(D, slot, 0, SrcV{B(D, B_W)}, ad);
   part[0] += dot3(dl, ad);
 }
 
@@ -1754,6 +1784,7 @@ __device__ __noinline__ void pl_exp_a_general(const InstDesc &D, const InstState
   pl_exp_a(D, S, C, v);
 }
 
+template <bool kPre>
 __device__ __noinline__ void row_exp(const InstDesc &D, const InstState &S, int v, int slot, double *part) {
   if (S.phase == PH_EXP_A) {  // y = P(x)
     row_project(D, B_X0 + S.xc, B_X0 + (S.xc ^ 1), v);
@@ -1763,7 +1794,7 @@ __device__ __noinline__ void row_exp(const InstDesc &D, const InstState &S, int 
   if (S.phase == PH_EXP_B) {  // g = A y - b; DECIDE_FACE(y); PHI; x = P(y - abar phi)
     const double *yb = B(D, B_X0 + (S.xc ^ 1));
     double y[3], ay[3];
-    spmv_row<double>(D.A, D.A.v64, slot, SrcV{yb}, ay);
+    row_product<kPre>(D, slot, 0, SrcV{yb}, ay);
     const double g[3] = {ay[0] - ldro(D.b + 3 * (size_t)v),
                          ay[1] - ldro(D.b + 3 * (size_t)v + 1),
                          ay[2] - ldro(D.b + 3 * (size_t)v + 2)};
@@ -1808,6 +1839,7 @@ __device__ __noinline__ void prop_b_general(const InstDesc &D, const InstState &
   prop_b(D, S, C, v, part);
 }
 
+template <bool kPre>
 __device__ __noinline__ void row_prop(const InstDesc &D, const InstState &S, int v, int slot,
                                       double *part) {
   const double *db = B(D, B_BT0 + S.bc);
@@ -1816,13 +1848,18 @@ __device__ __noinline__ void row_prop(const InstDesc &D, const InstState &S, int
     ld3(db, v, dd);
     if (S.phase == PH_PROP_A) {  // g = A x - B and AD = A D in one pass
       double ax[3];
-      spmv2_row(D.A, slot, SrcV{B(D, B_X0 + S.xc)}, SrcV{db}, ax, ad);
+      if constexpr (kPre) {
+        pre_product(0, ax);
+        pre_product(1, ad);
+      } else {
+        spmv2_row(D.A, slot, SrcV{B(D, B_X0 + S.xc)}, SrcV{db}, ax, ad);
+      }
 #pragma unroll
       for (int d = 0; d < 3; ++d) g[d] = ax[d] - ldro(D.b + 3 * (size_t)v + d);
       st3(B(D, B_G0 + S.gc), v, g);
     } else {
       ld3(B(D, B_G0 + S.gc), v, g);
-      spmv_row<double>(D.A, D.A.v64, slot, SrcV{db}, ad);
+      row_product<kPre>(D, slot, 0, SrcV{db}, ad);
     }
     st3(B(D, B_W), v, ad);
     part[0] += dot3(g, dd);
@@ -1878,6 +1915,7 @@ __device__ __noinline__ void row_pl_cg(const InstDesc &D, const InstState &S, in
   else pl_cg_general(D, S, v, part);
 }
 
+template <bool kPre = false>
 __device__ void row_op(const InstDesc &D, const InstState &S, int v, int slot, double *part) {
   switch (S.phase) {
     case PH_POW_RAND:
@@ -1887,19 +1925,19 @@ __device__ void row_op(const InstDesc &D, const InstState &S, int v, int slot, d
     case PH_FINAL:
     case PH_INIT:
     case PH_EXP_C:
-    case PH_PL_EXP_B: row_init(D, S, v, slot, part); break;
+    case PH_PL_EXP_B: row_init<kPre>(D, S, v, slot, part); break;
     case PH_CG_ENTRY:
     case PH_CG_SPMV:
-    case PH_PL_SPMV: row_cg_spmv(D, S, v, slot, part); break;
+    case PH_PL_SPMV: row_cg_spmv<kPre>(D, S, v, slot, part); break;
     case PH_CG_YF: row_cg_yf(D, S, v, slot, part); break;
-    case PH_CG_DAD: row_cg_dad(D, S, v, slot, part); break;
+    case PH_CG_DAD: row_cg_dad<kPre>(D, S, v, slot, part); break;
     case PH_RU: row_ru(D, S, v, slot, part); break;
     case PH_EXP_A:
     case PH_EXP_B:
-    case PH_PL_EXP_A: row_exp(D, S, v, slot, part); break;
+    case PH_PL_EXP_A: row_exp<kPre>(D, S, v, slot, part); break;
     case PH_PROP_A:
     case PH_PROP_B:
-    case PH_PL_PROP_A: row_prop(D, S, v, slot, part); break;
+    case PH_PL_PROP_A: row_prop<kPre>(D, S, v, slot, part); break;
     case PH_PL_CG: row_pl_cg(D, S, v, slot, part); break;
     default: break;
   }
@@ -3163,6 +3201,43 @@ __device__ __forceinline__ void sync_row_staged(const double *sv, const int *sc,
                                                 int j1, const double *src, double out[3]) {
   sync_row<kCh>(sv, sc, lane, j0, j1, SrcV{src}, out);
 }
+// One component of a row's product from the staged FP64 copy: the same
+// accumulator as in the whole row, by a thread of its own.
+template <int kCh>
+__device__ __forceinline__ double sync_comp(const double *sv, const int *sc, int lane, int comp,
+                                            int j0, int j1, const double *src,
+                                            const double *minus = nullptr, double beta = 0.0) {
+  // entries 3c, 3c + 1, 3c + 2 of the block: pairs at 64 k + 2 l, the last at 256 + l
+  const int o0 = comp == 0 ? 2 * lane : comp == 1 ? 64 + 2 * lane + 1 : 192 + 2 * lane;
+  const int o1 = comp == 0 ? 2 * lane + 1 : comp == 1 ? 128 + 2 * lane : 192 + 2 * lane + 1;
+  const int o2 = comp == 0 ? 64 + 2 * lane : comp == 1 ? 128 + 2 * lane + 1 : 256 + lane;
+  double a = 0.0;
+  for (int jb = j0; jb < j1; jb += kCh) {
+    double xv[kCh][3];
+#pragma unroll
+    for (int u = 0; u < kCh; ++u) {
+      if (jb + u >= j1) continue;
+      const int c = sc[(jb + u) * kSlice + lane];
+      ld3(src, c, xv[u]);
+      if (minus) {  // src - beta minus
+        double pp[3];
+        ld3(minus, c, pp);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) xv[u][d] = xv[u][d] - beta * pp[d];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kCh; ++u) {
+      if (jb + u >= j1) break;
+      const double *b = sv + (size_t)(jb + u) * (9 * kSlice);
+      a = fma(b[o0], xv[u][0], a);
+      a = fma(b[o1], xv[u][1], a);
+      a = fma(b[o2], xv[u][2], a);
+    }
+  }
+  return a;
+}
+
 // The product of a loop's first phase when it was resumed or starts from ev,
 // from global memory; out of line, and by value, since it runs once.
 template <typename VT>
@@ -3180,12 +3255,12 @@ __device__ __noinline__ Row3<VT> sync_row_first(const InstDesc &D, int src, int 
 // then the columns as vertices.  One pass before the loop.
 template <typename VT>
 __device__ __forceinline__ void sync_stage(const SellMatrix &A, const VT *vals, int s0, int s1,
-                                           int threads) {
+                                           int threads, unsigned char *dst) {
   const int f = ldro(A.slice_off + s0), l = ldro(A.slice_off + s1);
   const int nv16 = (l - f) * 9 * kSlice * (int)sizeof(VT) / 16;
   const float4 *src = reinterpret_cast<const float4 *>(vals + (size_t)f * (9 * kSlice));
-  for (int i = threadIdx.x; i < nv16; i += threads) cp_async16(g_stage + 16 * (size_t)i, src + i);
-  int *sc = reinterpret_cast<int *>(g_stage + 16 * (size_t)nv16);
+  for (int i = threadIdx.x; i < nv16; i += threads) cp_async16(dst + 16 * (size_t)i, src + i);
+  int *sc = reinterpret_cast<int *>(dst + 16 * (size_t)nv16);
   for (int i = threadIdx.x; i < (l - f) * kSlice; i += threads)
     sc[i] = checked_col(A, ldro(A.cols + (size_t)f * kSlice + i));
   asm volatile("cp.async.wait_all;\n" ::: "memory");
@@ -3220,19 +3295,23 @@ __device__ __noinline__ void sync_reduce(const InstDesc &D, InstState &S, int pa
   }
 }
 
-template <typename VT, int kThr, int kMinBlocks, int kCh>
+template <typename VT, int kComps, int kThr, int kMinBlocks, int kCh>
 __global__ void __launch_bounds__(kThr, kMinBlocks) power_sync_kernel(SyncArgs args) {
   constexpr bool kSplit = kThr < kStepThreads;  // units may be split over a cluster
+  constexpr int kN = 3 / kComps;                // components a thread carries
   __shared__ InstDesc sD;
   __shared__ InstState sS;
   __shared__ double sPart[2][kThreads];
+  __shared__ double sVec[kComps == 3 ? 2 : 1][kComps][kComps == 3 ? kThreads / 4 : 1];  // d, w by row
   __shared__ int sFail[2], sLeave;       // this CTA's wait ran out (by phase parity); a peer's did
   const int q = kSplit ? args.q : 1;     // CTAs of a unit (a cluster)
   const int rank = q > 1 ? (int)cluster_rank() : 0;
   const int R = kThreads / q;            // rows of this CTA
-  const int threads = R + 32;
+  const int threads = R * kComps + 32;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const bool rw = (int)threadIdx.x >= R;  // the reduction warp
+  const bool rw = (int)threadIdx.x >= R * kComps;  // the reduction warp
+  const int comp = kComps == 3 ? warp % 3 : 0;     // the thread's component and
+  const int ri = (kComps == 3 ? warp / 3 : warp) * 32 + lane;  // row of the CTA
   const SyncItem unit = args.items[(int)blockIdx.x / q];
   if (threadIdx.x == 0) {
     g_staged = 0;
@@ -3250,25 +3329,26 @@ __global__ void __launch_bounds__(kThr, kMinBlocks) power_sync_kernel(SyncArgs a
   const InstDesc &D = sD;
   InstState &S = sS;
   // the thread's row, its slots in the staged copy, its vectors
-  const int slot = unit.local * kThreads + rank * R + (int)threadIdx.x;
+  const int slot = unit.local * kThreads + rank * R + ri;
   const bool row = !rw && slot < D.nv;
   const int v = row ? row_vertex(D.A, slot) : 0;
   int j0 = 0, j1 = 0, voff = 0;
-  VT own[3] = {0, 0, 0};                    // the phase's source at the row
-  VT tk[3] = {0, 0, 0}, tp[3] = {0, 0, 0};  // t_k and t_{k-1}
+  VT own[kN], tk[kN], tp[kN];  // the phase's source at the row; t_k and t_{k-1}
+#pragma unroll
+  for (int d = 0; d < kN; ++d) own[d] = tk[d] = tp[d] = 0;
   {
     const int s0 = min(unit.local * (kThreads / kSlice) + rank * (R / kSlice), D.A.nslices);
     const int s1 = min(s0 + R / kSlice, D.A.nslices);
     sync_stage(D.A, sizeof(VT) == 4 ? reinterpret_cast<const VT *>(D.A.v32)
-                                    : reinterpret_cast<const VT *>(D.A.v64), s0, s1, threads);
+                                    : reinterpret_cast<const VT *>(D.A.v64), s0, s1, threads, g_stage);
     const int f = ldro(D.A.slice_off + s0), l = ldro(D.A.slice_off + s1);
     voff = (l - f) * 9 * kSlice * (int)sizeof(VT);
     if (row) {
       j0 = ldro(D.A.slice_off + (slot >> 5)) - f;
       j1 = ldro(D.A.slice_off + (slot >> 5) + 1) - f;
       if (S.phase == PH_POW || S.phase == PH_POW_LAST) {  // resumed, or started from ev
-        for (int d = 0; d < 3; ++d) {
-          const size_t i = 3 * (size_t)v + d;
+        for (int d = 0; d < kN; ++d) {
+          const size_t i = 3 * (size_t)v + comp + d;
           own[d] = S.pow_src < 0 ? (VT)D.ev[i] : pow_vec(D, S.pow_src, VT())[i];
           if (S.pow_k >= 1) tk[d] = pow_vec(D, B_T0 + ((S.pow_k - 1) & 1), VT())[i];
         }
@@ -3282,7 +3362,9 @@ __global__ void __launch_bounds__(kThr, kMinBlocks) power_sync_kernel(SyncArgs a
   for (int t = 0;; ++t) {
     const int par = t & 1;
     const unsigned long long tag = ((t >> 1) & 1) ? 0ull : kSignBit;
-    VT wr[3] = {0, 0, 0};  // the raw product of raw_src
+    VT wr[kN];  // the raw product of raw_src
+#pragma unroll
+    for (int d = 0; d < kN; ++d) wr[d] = 0;
     int raw_src = kNoSrc;
     if (t > 0) {
       if (rw) {
@@ -3294,7 +3376,12 @@ __global__ void __launch_bounds__(kThr, kMinBlocks) power_sync_kernel(SyncArgs a
         raw_src = phase_in == PH_POW_RAND ? B_W1
                   : phase_in == PH_POW    ? ((k_in & 1) ? B_W1 : B_W)
                                           : kNoSrc;
-        if (row && raw_src != kNoSrc) sync_row_staged<kCh>(sv, sc, lane, j0, j1, pow_vec(D, raw_src, VT()), wr);
+        if (row && raw_src != kNoSrc) {
+          if constexpr (kComps == 3)
+            wr[0] = sync_comp<kCh>(sv, sc, lane, comp, j0, j1, pow_vec(D, raw_src, VT()));
+          else
+            sync_row_staged<kCh>(sv, sc, lane, j0, j1, pow_vec(D, raw_src, VT()), wr);
+        }
       }
       block_bar(threads);
       if (q == 1 && sFail[par]) break;
@@ -3302,44 +3389,64 @@ __global__ void __launch_bounds__(kThr, kMinBlocks) power_sync_kernel(SyncArgs a
     const int phase = S.phase;
     if (!power_phase(phase) || t >= unit.limit) break;
     double p0 = 0.0, p1 = 0.0;
+    VT dd[kN];  // t_k - t_{k-1}
+#pragma unroll
+    for (int d = 0; d < kN; ++d) dd[d] = 0;
     if (row) {
       if (phase == PH_POW_RAND) {
-        double part[2] = {0.0, 0.0};
-        row_power_rand(D, v, part);
-        p0 = part[0];
+        if (comp == 0) {
+          double part[2] = {0.0, 0.0};
+          row_power_rand(D, v, part);
+          p0 = part[0];
+        }
 #pragma unroll
-        for (int d = 0; d < 3; ++d) own[d] = (VT)seeded_uniform(D.seed, 3ull * v + d);
+        for (int d = 0; d < kN; ++d) own[d] = (VT)seeded_uniform(D.seed, 3ull * v + comp + d);
       } else {  // row_power32_fin / row_power64_fin from registers
         if (phase == PH_POW && S.pow_src != raw_src) {  // no product yet
           const Row3<VT> r = sync_row_first<VT>(D, S.pow_src, slot);
-          wr[0] = r.w[0];
-          wr[1] = r.w[1];
-          wr[2] = r.w[2];
+#pragma unroll
+          for (int d = 0; d < kN; ++d) wr[d] = kComps == 1 ? r.w[d] : comp == 0 ? r.w[0] : comp == 1 ? r.w[1] : r.w[2];
         }
         const VT scale = (VT)S.pow_scale;
-        const VT u[3] = {own[0] * scale, own[1] * scale, own[2] * scale};
-        if (phase == PH_POW_LAST || S.pow_k >= 1) {
-          const VT d[3] = {u[0] - tk[0], u[1] - tk[1], u[2] - tk[2]};
-          p0 = sq3(d);
-        }
-        if (phase == PH_POW) {
-          VT *wv = pow_vec(D, (S.pow_k & 1) ? B_W1 : B_W, VT()) + 3 * (size_t)v;
+        const bool diff = phase == PH_POW_LAST || S.pow_k >= 1;
+        VT *wv = pow_vec(D, (S.pow_k & 1) ? B_W1 : B_W, VT()) + 3 * (size_t)v + comp;
 #pragma unroll
-          for (int d = 0; d < 3; ++d) {
+        for (int d = 0; d < kN; ++d) {
+          const VT u = own[d] * scale;
+          if (diff) dd[d] = u - tk[d];
+          if (phase == PH_POW) {
             tp[d] = tk[d];
-            tk[d] = u[d];
+            tk[d] = u;
             own[d] = wr[d] * scale;
             wv[d] = own[d];
           }
-          p1 = sq3(own);
+        }
+        if constexpr (kComps == 1) {
+          if (diff) p0 = sq3(dd);
+          if (phase == PH_POW) p1 = sq3(own);
+        }
+      }
+    }
+    if constexpr (kComps == 3) {  // the rows' norms need their three threads' components
+      if (phase != PH_POW_RAND) {
+        if (!rw) {
+          sVec[0][comp][ri] = dd[0];
+          sVec[1][comp][ri] = phase == PH_POW && row ? own[0] : 0.0;
+        }
+        __syncthreads();
+        if (!rw && comp == 0) {
+          const double d[3] = {sVec[0][0][ri], sVec[0][1][ri], sVec[0][2][ri]};
+          const double w[3] = {sVec[1][0][ri], sVec[1][1][ri], sVec[1][2][ri]};
+          p0 = dot3(d, d);
+          p1 = dot3(w, w);
         }
       }
     }
     if (phase == PH_POW) kl = S.pow_k;
     // the item's sums of phase t, in block_reduce's order
-    if (!rw) {
-      sPart[0][threadIdx.x] = p0;
-      sPart[1][threadIdx.x] = p1;
+    if (!rw && comp == 0) {
+      sPart[0][ri] = p0;
+      sPart[1][ri] = p1;
     }
     if (q > 1) {
       cluster_sync_acq_rel();
@@ -3381,8 +3488,8 @@ __global__ void __launch_bounds__(kThr, kMinBlocks) power_sync_kernel(SyncArgs a
     }
   }
   if (row && kl >= 0) {  // t_k and t_{k-1}, where PH_INIT looks for ev
-    for (int d = 0; d < 3; ++d) {
-      const size_t i = 3 * (size_t)v + d;
+    for (int d = 0; d < kN; ++d) {
+      const size_t i = 3 * (size_t)v + comp + d;
       pow_vec(D, B_T0 + (kl & 1), VT())[i] = tk[d];
       if (kl >= 1) pow_vec(D, B_T0 + ((kl - 1) & 1), VT())[i] = tp[d];
     }
@@ -3581,6 +3688,56 @@ __global__ void __launch_bounds__(kStepThreads, kMinBlocks)
 // bounded by wait_ns (a whole launch by total_ns); a CTA that gives up sets the
 // error and leaves, and the others follow when they see it.
 
+// The products a row of the FP64 form needs in phase S.phase, component `comp`,
+// into g_pre: the sources the row functions name.
+struct StagedRow {  // the row's slots j0..j1 in the staged copy of its slices
+  const double *sv;
+  const int *sc;
+  int j0, j1;
+};
+__device__ __noinline__ double staged_comp(const StagedRow &r, int comp, const double *z,
+                                           const double *minus, double beta) {
+  return sync_comp<16>(r.sv, r.sc, (int)(threadIdx.x & 31), comp, r.j0, r.j1, z, minus, beta);
+}
+__device__ __forceinline__ void form_products(const InstDesc &D, const InstState &S,
+                                              const StagedRow &row, int v, int comp, int ri) {
+  const double *x = B(D, B_X0 + S.xc), *p = B(D, B_P0 + S.pc), *d = B(D, B_BT0 + S.bc);
+  const double *z = nullptr, *minus = nullptr, *second = nullptr;
+  switch (S.phase) {
+    case PH_INIT:
+    case PH_EXP_C:
+    case PH_PL_EXP_B: z = x; break;
+    case PH_EXP_B: z = B(D, B_X0 + (S.xc ^ 1)); break;
+    case PH_CG_ENTRY:
+      z = p;
+      if (!S.g_cons) second = x;
+      break;
+    case PH_CG_SPMV:
+    case PH_PL_SPMV:
+      if (S.phase == PH_PL_SPMV && S.p_is_z) {
+        z = p;
+      } else {
+        z = B(D, B_Z0 + S.zc);
+        minus = p;
+      }
+      break;
+    case PH_PROP_A:
+      z = x;
+      second = d;
+      break;
+    case PH_PL_PROP_A: z = d; break;
+    case PH_CG_DAD: {
+      double dl[3];
+      ld3(B(D, B_W), v, dl);
+      if (dl[0] != 0.0 || dl[1] != 0.0 || dl[2] != 0.0) z = B(D, B_W);
+      break;
+    }
+    default: break;
+  }
+  if (z) g_pre[comp][ri] = staged_comp(row, comp, z, minus, S.beta_cg);
+  if (second) g_pre[3 + comp][ri] = staged_comp(row, comp, second, nullptr, 0.0);
+}
+
 // Slot k of an instance's `nitems` item partials (contiguous), summed by one
 // warp in the finalize's order (warp_finalize): lane l forms the sums of items
 // l + 32 i, + 256, ..., adds those of i = 0..7 and closes with the shuffle
@@ -3686,8 +3843,8 @@ __device__ double group_reduce(double *part, RedBuf &red, int ns, bool with_min,
   return r;
 }
 
-template <int kThr, bool kSplit>
-__global__ void __launch_bounds__(kThr) engine_sync_kernel(EngineSyncArgs args) {
+template <int kThr, bool kSplit, bool kPre>
+__global__ void __launch_bounds__(kThr, 1) engine_sync_kernel(EngineSyncArgs args) {
   constexpr int kOwn = kSplit ? 1 : kEngOwn;
   extern __shared__ __align__(16) unsigned char g_engine[];
   RedBuf *red = reinterpret_cast<RedBuf *>(g_engine);  // one a group
@@ -3732,6 +3889,29 @@ __global__ void __launch_bounds__(kThr) engine_sync_kernel(EngineSyncArgs args) 
       if (sItem[o].local != 0 || rank != 0) sD[o].trace = nullptr;
   }
   __syncthreads();
+  int v_split = 0;  // the row's vertex (a split unit's CTA keeps its rows)
+  if (kSplit) {
+    const int ri = kPre ? pre_row() : gt;
+    const int slot = sItem[0].local * kThreads + rank * R + ri;
+    if (ri < R && slot < sD[0].nv) v_split = row_vertex(sD[0].A, slot);
+  }
+  // three threads a row: its slices in shared memory for the whole launch
+  StagedRow staged = {nullptr, nullptr, 0, 0};
+  if constexpr (kPre) {
+    const SellMatrix &A = sD[0].A;
+    const int s0 = min(sItem[0].local * (kThreads / kSlice) + rank * (R / kSlice), A.nslices);
+    const int s1 = min(s0 + R / kSlice, A.nslices);
+    unsigned char *dst = g_engine + sizeof(RedBuf);
+    sync_stage(A, A.v64, s0, s1, threads, dst);
+    const int f = ldro(A.slice_off + s0), l = ldro(A.slice_off + s1), sl = s0 + (pre_row() >> 5);
+    staged.sv = reinterpret_cast<const double *>(dst);
+    staged.sc = reinterpret_cast<const int *>(dst + (size_t)(l - f) * 9 * kSlice * sizeof(double));
+    if (sl < s1) {
+      staged.j0 = ldro(A.slice_off + sl) - f;
+      staged.j1 = ldro(A.slice_off + sl + 1) - f;
+    }
+    __syncthreads();
+  }
   for (int t = 0; t < args.max_phases; ++t) {
     const int par = t & 1;
     bool ran = false;
@@ -3751,8 +3931,15 @@ __global__ void __launch_bounds__(kThr) engine_sync_kernel(EngineSyncArgs args) 
         double part[kPart];
 #pragma unroll
         for (int k = 0; k < kPart; ++k) part[k] = (k == kMinSlot) ? DBL_MAX : 0.0;
-        const int slot = sItem[o].local * kThreads + rank * R + gt;
-        if (gt < R && slot < D.nv) row_op(D, S, row_vertex(D.A, slot), slot, part);
+        const int ri = kPre ? pre_row() : gt;  // the thread's row of the part
+        const int slot = sItem[o].local * kThreads + rank * R + ri;
+        const bool in = ri < R && slot < D.nv;
+        if constexpr (kPre) {
+          if (in) form_products(D, S, staged, v_split, warp % 3, ri);
+          __syncthreads();
+        }
+        if (in && (!kPre || warp % 3 == 0))
+          row_op<kPre>(D, S, kSplit ? v_split : row_vertex(D.A, slot), slot, part);
         if (!kSplit) {
           const double r = group_reduce(part, red[g], ns, wmin, g);
           if (gt < ns) pp[(size_t)gt * D.nitems] = r;
@@ -3761,16 +3948,16 @@ __global__ void __launch_bounds__(kThr) engine_sync_kernel(EngineSyncArgs args) 
           // split unit's CTAs would have to agree, so they keep the flag)
           if (phase == PH_CG_YF && gt == 1) sMoved[o] = r != 0.0;
         } else {
-          if (gt < R) {
+          if (ri < R && (!kPre || warp % 3 == 0)) {
 #pragma unroll
             for (int k = 0; k < kPart; ++k) {
               if (k == kMinSlot ? !wmin : k >= ns) continue;
-              red[0].v[k == kMinSlot ? ns : k][gt] = part[k];
+              red[0].v[k == kMinSlot ? ns : k][ri] = part[k];
             }
           }
           cluster_sync_acq_rel();
           // row k of the sums by rank k mod q, in block_reduce's order
-          for (int k = rank + q * warp; k < ns + (wmin ? 1 : 0); k += q * (kThr / 32)) {
+          for (int k = rank + q * warp; k < ns + (wmin ? 1 : 0); k += q * (threads / 32)) {
             const bool is_min = wmin && k == ns;
             double x[kThreads / 32], acc;
 #pragma unroll
@@ -4062,6 +4249,47 @@ __global__ void __launch_bounds__(256, MPRGP_SPMV_MIN_BLOCKS) spmv_kernel(SellMa
   st3(y, v, o);
 }
 
+// The FP64 product of a matrix whose rows do not fill the SMs: three threads a
+// row, one a component, five of the row's slots in flight.  A row's 135 FP64
+// FMAs (15 blocks) are a chain of 6 us in one warp; a component's 45 take 2 and
+// meet two other warps' on other schedulers.  Every accumulator adds in slot
+// order, as above.  396 vertices: 12.4 -> 8.2 us a call (most of the rest is
+// the call), 20,286: 14.4 -> 10.0, 40,824: 22.6 -> 16.4; 71,808: 24.6 -> 26.7,
+// so the rule below ends at ten slices an SM (48,640 rows on 152 SMs).
+__global__ void __launch_bounds__(96) spmv_comp_kernel(SellMatrix A, int nv,
+                                                       const double *__restrict__ x,
+                                                       double *__restrict__ y) {
+  constexpr int K = 5;
+  const int s = blockIdx.x, comp = (int)(threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int slot = s * kSlice + lane;
+  if (slot >= nv) return;
+  const int v = row_vertex(A, slot);
+  const int j0 = ldro(A.slice_off + s), j1 = ldro(A.slice_off + s + 1);
+  double acc = 0.0;
+  for (int jb = j0; jb < j1; jb += K) {
+    int c[K];
+    double m[K][3], xv[K][3];
+    // (slots past the row's end repeat its last one; their terms are left out)
+#pragma unroll
+    for (int u = 0; u < K; ++u)
+      c[u] = checked_col(A, ldro(A.cols + (size_t)min(jb + u, j1 - 1) * kSlice + lane));
+#pragma unroll
+    for (int u = 0; u < K; ++u) {
+      const size_t j = (size_t)min(jb + u, j1 - 1);
+#pragma unroll
+      for (int e = 0; e < 3; ++e) m[u][e] = ldro(A.v64 + sell_index(j, 3 * comp + e, lane, double()));
+      ld3(x, c[u], xv[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < K; ++u) {
+      if (jb + u >= j1) break;
+#pragma unroll
+      for (int e = 0; e < 3; ++e) acc = fma(m[u][e], xv[u][e], acc);
+    }
+  }
+  y[3 * (size_t)v + comp] = acc;
+}
+
 // During an engine run the instance states live in one array in desc order
 // (the run's desc entries point into it), so a launch can fetch an item's
 // desc and state in one round of loads.  Between runs each state lives with
@@ -4118,12 +4346,13 @@ cudaError_t launch_engine(const EngineArgs &args, int grid, cudaStream_t stream)
                                      params, (size_t)args.stage_bytes, stream);
 }
 // The waiting engine with q CTAs a unit, or (q == 1) CTAs of `groups` groups.
-static void engine_sync_config(int q, int groups, int grid, cudaStream_t stream,
+static void engine_sync_config(int q, int groups, int grid, int smem, cudaStream_t stream,
                                cudaLaunchConfig_t &cfg, cudaLaunchAttribute (&at)[2]) {
   cfg = {};
   cfg.gridDim = dim3((unsigned int)grid);
-  cfg.blockDim = dim3(q > 1 ? kThreads / 2 : groups * kThreads);
-  cfg.dynamicSmemBytes = sizeof(RedBuf) * (q > 1 ? 1 : groups);
+  // four or eight CTAs a unit: three threads a row, and warps that only sum
+  cfg.blockDim = dim3(q > 2 ? kThreads : q > 1 ? kThreads / 2 : groups * kThreads);
+  cfg.dynamicSmemBytes = sizeof(RedBuf) * (q > 1 ? 1 : groups) + (size_t)smem;
   cfg.stream = stream;
   at[0].id = cudaLaunchAttributeCooperative;
   at[0].val.cooperative = 1;
@@ -4135,27 +4364,30 @@ static void engine_sync_config(int q, int groups, int grid, cudaStream_t stream,
   cfg.numAttrs = q > 1 ? 2 : 1;
 }
 static const void *engine_sync_fn(int q) {
-  return q > 1 ? (const void *)engine_sync_kernel<kThreads / 2, true>
-               : (const void *)engine_sync_kernel<4 * kThreads, false>;
+  return q > 2   ? (const void *)engine_sync_kernel<kThreads, true, true>
+         : q > 1 ? (const void *)engine_sync_kernel<kThreads / 2, true, false>
+                 : (const void *)engine_sync_kernel<4 * kThreads, false, false>;
 }
-cudaError_t launch_engine_sync(const EngineSyncArgs &args, int groups, int grid,
+cudaError_t launch_engine_sync(const EngineSyncArgs &args, int groups, int grid, int smem,
                                cudaStream_t stream) {
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute at[2];
-  engine_sync_config(args.q, groups, grid, stream, cfg, at);
+  engine_sync_config(args.q, groups, grid, smem, stream, cfg, at);
   void *params[] = {(void *)&args};
   return cudaLaunchKernelExC(&cfg, engine_sync_fn(args.q), params);
 }
-// CTAs of that form that can be resident at once (q == 1: of four groups).
-cudaError_t engine_sync_capacity(int q, int nsm, int *ctas) {
+// CTAs of that form that can be resident at once (q == 1: of four groups; smem:
+// staged bytes a CTA).
+cudaError_t engine_sync_capacity(int q, int smem, int nsm, int *ctas) {
   int n = 0;
   cudaError_t e = cudaFuncSetAttribute(engine_sync_fn(q), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)sizeof(RedBuf) * 4);
+                                       q > 2 ? kEngStageBytes + (int)sizeof(RedBuf)
+                                             : (int)sizeof(RedBuf) * 4);
   *ctas = 0;
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute at[2];
-  engine_sync_config(q, 4, q, nullptr, cfg, at);
+  engine_sync_config(q, 4, q, smem, nullptr, cfg, at);
   if (q == 1) {
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, engine_sync_fn(1), 4 * kThreads,
                                                       cfg.dynamicSmemBytes);
@@ -4375,20 +4607,20 @@ cudaError_t power_clusters_max_active(int csize, int *n) {
 cudaError_t power_persistent_max_blocks_per_sm(int fp32, int *n) {
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, power_persistent_fn(fp32), kStepThreads, 0);
 }
-// The power sync loop's kernel for q CTAs a unit.
-template <typename VT>
-static const void *power_sync_fn(int q) {
-  return q > 1 ? (const void *)power_sync_kernel<VT, kThreads / 2 + 32, 3, 8>
-               : (const void *)power_sync_kernel<VT, kStepThreads, 1, 8>;
+// The power sync loop's kernel for q CTAs a unit and `comps` threads a row.
+static const void *power_sync_fn(int q, int fp32, int comps) {
+  if (comps == 3) return (const void *)power_sync_kernel<double, 3, 3 * kThreads / 4 + 32, 1, 16>;
+  if (fp32)
+    return q > 1 ? (const void *)power_sync_kernel<float, 1, kThreads / 2 + 32, 3, 8>
+                 : (const void *)power_sync_kernel<float, 1, kStepThreads, 1, 8>;
+  return q > 1 ? (const void *)power_sync_kernel<double, 1, kThreads / 2 + 32, 3, 8>
+               : (const void *)power_sync_kernel<double, 1, kStepThreads, 1, 8>;
 }
-static const void *power_sync_fn(int q, int fp32) {
-  return fp32 ? power_sync_fn<float>(q) : power_sync_fn<double>(q);
-}
-static void power_sync_config(int q, int grid, int smem, cudaStream_t stream, cudaLaunchConfig_t &cfg,
-                              cudaLaunchAttribute (&at)[2]) {
+static void power_sync_config(int q, int comps, int grid, int smem, cudaStream_t stream,
+                              cudaLaunchConfig_t &cfg, cudaLaunchAttribute (&at)[2]) {
   cfg = {};
   cfg.gridDim = dim3((unsigned int)grid);
-  cfg.blockDim = dim3((unsigned int)(kThreads / q + 32));
+  cfg.blockDim = dim3((unsigned int)(kThreads / q * comps + 32));
   cfg.dynamicSmemBytes = (size_t)smem;
   cfg.stream = stream;
   at[0].id = cudaLaunchAttributeCooperative;
@@ -4401,9 +4633,9 @@ static void power_sync_config(int q, int grid, int smem, cudaStream_t stream, cu
   cfg.numAttrs = q > 1 ? 2 : 1;
 }
 // CTAs of that form that can be resident at once (smem: staged bytes a CTA).
-cudaError_t power_sync_capacity(int q, int fp32, int smem, int nsm, int *ctas) {
+cudaError_t power_sync_capacity(int q, int fp32, int comps, int smem, int nsm, int *ctas) {
   *ctas = 0;
-  const void *fn = power_sync_fn(q, fp32);
+  const void *fn = power_sync_fn(q, fp32, comps);
   // (one value for every query: the attribute is the kernel's, not the launch's)
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kSyncStageBytes);
   if (e != cudaSuccess) return e;
@@ -4415,20 +4647,20 @@ cudaError_t power_sync_capacity(int q, int fp32, int smem, int nsm, int *ctas) {
   }
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute at[2];
-  power_sync_config(q, q, smem, nullptr, cfg, at);
+  power_sync_config(q, comps, q, smem, nullptr, cfg, at);
   cfg.attrs = at + 1;
   cfg.numAttrs = 1;
   e = cudaOccupancyMaxActiveClusters(&n, fn, &cfg);
   *ctas = n * q;
   return e;
 }
-cudaError_t launch_power_sync(const SyncArgs &args, int fp32, int grid, int smem,
+cudaError_t launch_power_sync(const SyncArgs &args, int fp32, int comps, int grid, int smem,
                               cudaStream_t stream) {
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute at[2];
-  power_sync_config(args.q, grid, smem, stream, cfg, at);
+  power_sync_config(args.q, comps, grid, smem, stream, cfg, at);
   void *params[] = {(void *)&args};
-  return cudaLaunchKernelExC(&cfg, power_sync_fn(args.q, fp32), params);
+  return cudaLaunchKernelExC(&cfg, power_sync_fn(args.q, fp32, comps), params);
 }
 cudaError_t power_max_blocks_per_sm(int variant, int *n) {
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, power_kernel_fn(variant),
@@ -4453,9 +4685,11 @@ void launch_planes_setup(int nv, const int *plane_ptr, const double *in, double 
 void launch_planes_axis(int m, const double *in, unsigned char *axis, cudaStream_t st) {
   if (m > 0) planes_axis_kernel<<<(m + 255) / 256, 256, 0, st>>>(m, in, axis);
 }
-void launch_spmv(const SellMatrix &A, int nv, bool fp32, const double *x, double *y,
+void launch_spmv(const SellMatrix &A, int nv, int nsm, bool fp32, const double *x, double *y,
                  cudaStream_t st) {
+  const int slices = (nv + kSlice - 1) / kSlice;
   if (fp32) spmv_kernel<float><<<(nv + 255) / 256, 256, 0, st>>>(A, A.v32, nv, x, y);
+  else if (slices <= 10 * nsm) spmv_comp_kernel<<<slices, 96, 0, st>>>(A, nv, x, y);
   else spmv_kernel<double><<<(nv + 255) / 256, 256, 0, st>>>(A, A.v64, nv, x, y);
 }
 

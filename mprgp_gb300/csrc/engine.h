@@ -171,7 +171,8 @@ struct ClusterArgs {
   int max_phases;        // quantum / hard bound on phases
 };
 
-constexpr int kSyncStageBytes = 220 * 1024;  // shared memory of a power sync CTA's slices, at most
+constexpr int kSyncStageBytes = 216 * 1024;  // shared memory of a power sync CTA's slices, at most
+constexpr int kEngStageBytes = 200 * 1024;   // ... of a waiting engine's
 // One item of an instance in the power sync loop (`limit`: its phases there).
 struct SyncItem {
   int inst, local, limit, pad;

@@ -30,6 +30,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/mprgp_gpu.h"
+#include "coop_gate.h"
 
 namespace mprgp {
 void set_last_error(const char *what);
@@ -851,8 +852,10 @@ int mprgp_ica_solve(mprgp_context *ctx, int nv, int nnzb, const int *row_ptr, co
       ca.rows = (const IcaRow *)(d + o_rows);
       e = cudaLaunchKernelEx(&ccfg, ica_cluster_kernel, ca);
     } else if (e == cudaSuccess)
-      e = cudaLaunchCooperativeKernel((const void *)ica_kernel, dim3(grid), dim3(kIcaThreads),
-                                      params, 0, s);
+      e = mprgp::gated_launch(s, [&] {
+        return cudaLaunchCooperativeKernel((const void *)ica_kernel, dim3(grid), dim3(kIcaThreads),
+                                           params, 0, s);
+      });
     if (e == cudaSuccess) e = cudaEventRecord(e1, s);
   }
   IcaCtl ctl{};

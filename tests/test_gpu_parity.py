@@ -691,3 +691,28 @@ def test_spmv_column_forms(ctx, far):
     ctx.sync()
     assert rel(yd.cpu().numpy(), y_ref) < 1e-5
     pr.close()
+
+
+@pytest.mark.parametrize("dims", [(1, 1, 1), (3, 3, 1), (3, 3, 15), (20, 20, 45), (35, 35, 36),
+                                  (35, 35, 37)])
+def test_spmv_forms(ctx, dims):
+    """The FP64 product on both sides of the size where three threads a row
+    give way to one, and at partial slices: each row against the 64-bit sum,
+    within 2 n eps of the row's absolute sum (n = 45 products)."""
+    torch = pytest.importorskip("torch")
+    qp = corner(*dims, seed=6)
+    x = np.random.default_rng(1).standard_normal(qp.n)
+    pr = M.Problem(ctx, qp.nv)
+    pr.set_planes(qp.plane_ptr, qp.planes)  # a row order other than the vertices'
+    pr.set_matrix(qp.row_ptr, qp.cols, qp.vals, precisions=1)
+    xd, yd = torch.from_numpy(x).cuda(), torch.zeros(qp.n, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    pr.spmv(xd.data_ptr(), yd.data_ptr(), M.PREC_FP64)
+    ctx.sync()
+    rows = np.repeat(np.arange(qp.nv), np.diff(qp.row_ptr))
+    blocks, xb = qp.vals.reshape(-1, 3, 3), x.reshape(-1, 3)[qp.cols]
+    y, size = np.zeros((qp.nv, 3)), np.zeros((qp.nv, 3))
+    np.add.at(y, rows, np.einsum("kij,kj->ki", blocks, xb))
+    np.add.at(size, rows, np.einsum("kij,kj->ki", np.abs(blocks), np.abs(xb)))
+    assert (np.abs(yd.cpu().numpy() - y.reshape(-1)) <= 90 * 2.3e-16 * size.reshape(-1)).all()
+    pr.close()
