@@ -36,7 +36,7 @@ struct mprgp_fem {
   int *tets = nullptr;                   // 4 per tet
   int *row_ptr = nullptr, *cols = nullptr;
   int *vt_ptr = nullptr, *vt = nullptr;  // incident (tet << 2 | local corner) per vertex
-  int max_up = 0;                        // blocks right of the diagonal in a row, at most
+  int max_len = 0;                       // blocks in a row, at most
   double *geom = nullptr;                // kGeom per tet: V, grad N_0..3, padding
   double *X = nullptr;                   // rest shape
   double *mass = nullptr, *KX = nullptr;
@@ -110,135 +110,91 @@ __device__ __forceinline__ int find_block(const int *__restrict__ cols, int r0, 
   return lo;
 }
 
-// A's rows by warps of 32 rows, one row a lane.
+// A's rows by warps of 32 rows, one row a lane: K_ab = V (lam gNa gNb^T +
+// mu gNb gNa^T + mu (gNa . gNb) I) summed over the tets around a (in incidence
+// order), scaled by h^2, plus the lumped mass on the diagonal block; K X along
+// the way.
 //
-// K_ab = V (lam gNa gNb^T + mu gNb gNa^T + mu (gNa . gNb) I) summed over the
-// tets of an edge is lam P + mu P^T + mu tr(P) I with P = sum V gNa gNb^T, so
-// a tet adds nine products to a block instead of some sixty operations; GB300
-// issues one FP64 warp instruction in 64 clocks or more per scheduler, and
-// these bound the assembly (348,145 vertices, 2M tets: 0.77 ms, against 4.81
-// with a thread per row adding whole element blocks in global memory; the
-// matrix alone takes 0.06 ms to write).  Blocks right of the
-// diagonal are formed once and written with their transposes (K is symmetric;
-// the mirrored position comes from a search in the other row).  K X of the
-// rest shape X needs no blocks: sum_b gNb X_b^T = I in every tet, so
-// (K X)_a = (3 lam + 2 mu) sum V gNa.
-//
-// The lanes' blocks lie side by side in shared memory (entry k of lane l at
+// The lanes' rows lie side by side in shared memory (entry k of lane l at
 // 33 k + l: no bank conflicts while the lanes add to blocks of their own, nor
-// while the warp copies one row out), the diagonal first, so that each row's
-// upper part leaves as one contiguous piece.
+// while the warp copies one row out), so the sums never travel through global
+// memory and each row leaves as one contiguous piece.  What bounds it then is
+// the FP64 unit: five operations an entry, 144 entries a tet, and an FP64 warp
+// instruction takes 64 clocks or more of a scheduler (348,145 vertices, 2M
+// tets: 3.20 ms, against 4.81 with the rows in global memory; the operations
+// alone take about 2.9).  Fewer operations exist (P = sum V gNa gNb^T with the
+// two moduli applied at the end, upper blocks mirrored: 0.77 ms), but they
+// round differently, and on a small stiff body a last bit of A moves the
+// solution by as much as the solver's tolerance lets it.
 constexpr int kRowPad = 33;
-constexpr int kUpperSmemMax = 220 * 1024;  // rows of up to 84 blocks right of the diagonal
-__host__ __device__ constexpr int upper_smem(int max_up) {
-  return kRowPad * (max_up + 1) * (9 * 8 + 4 + 4);
+constexpr int kRowSmemMax = 220 * 1024;  // rows of up to 89 blocks
+__host__ __device__ constexpr int row_smem(int max_len) {
+  return kRowPad * max_len * (9 * 8 + 4);
 }
 __global__ void __launch_bounds__(32)
-    assemble_upper_kernel(int nv, int max_up, const int4 *__restrict__ tets,
-                          const double *__restrict__ geom, const int *__restrict__ row_ptr,
-                          const int *__restrict__ cols, const int *__restrict__ vt_ptr,
-                          const int *__restrict__ vt, double lam, double mu, double rho, double h2,
-                          double *vals, double *mass, double *KX) {
+    assemble_smem_kernel(int nv, int max_len, const int4 *__restrict__ tets,
+                         const double *__restrict__ geom, const int *__restrict__ row_ptr,
+                         const int *__restrict__ cols, const int *__restrict__ vt_ptr,
+                         const int *__restrict__ vt, const double *__restrict__ X, double lam,
+                         double mu, double rho, double h2, double *vals, double *mass, double *KX) {
   extern __shared__ __align__(16) unsigned char smem[];
-  double *P = reinterpret_cast<double *>(smem);                      // 9 per block
-  int *scol = reinterpret_cast<int *>(P + kRowPad * 9 * (max_up + 1));  // the block's column
-  int *spos = scol + kRowPad * (max_up + 1);                         // its mirror's position
+  double *P = reinterpret_cast<double *>(smem);                // 9 per block
+  int *scol = reinterpret_cast<int *>(P + kRowPad * 9 * max_len);  // the block's column
   const int lane = threadIdx.x;
   const int a = blockIdx.x * 32 + lane;
-  int d = 0, nup = -1;  // the diagonal block, blocks right of it (-1: no row)
+  int r0 = 0, len = 0;
   if (a < nv) {
-    const int r1 = row_ptr[a + 1];
-    d = find_block(cols, row_ptr[a], r1, a);
-    nup = r1 - d - 1;
-    for (int s = 1; s <= nup; ++s) {
-      const int b = cols[d + s];
-      scol[s * kRowPad + lane] = b;
-      spos[s * kRowPad + lane] = find_block(cols, row_ptr[b], row_ptr[b + 1], a);
-    }
-    for (int k = 9; k < 9 * (nup + 1); ++k) P[k * kRowPad + lane] = 0.0;
-    double m = 0.0, w[3] = {0.0, 0.0, 0.0}, q[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    r0 = row_ptr[a];
+    len = row_ptr[a + 1] - r0;
+    for (int s = 0; s < len; ++s) scol[s * kRowPad + lane] = cols[r0 + s];
+    for (int k = 0; k < 9 * len; ++k) P[k * kRowPad + lane] = 0.0;
+    double m = 0.0, kx[3] = {0.0, 0.0, 0.0};
     for (int idx = vt_ptr[a]; idx < vt_ptr[a + 1]; ++idx) {
       const int t = vt[idx] >> 2, la = vt[idx] & 3;
       const int4 tv = tets[t];
       const double *g = geom + kGeom * (size_t)t;
       const double V = g[0];
-      const double g0 = g[1 + 3 * la], g1 = g[2 + 3 * la], g2 = g[3 + 3 * la];
-      const double w0 = V * g0, w1 = V * g1, w2 = V * g2;
       m += rho * V / 4.0;
-      w[0] += w0;
-      w[1] += w1;
-      w[2] += w2;
-      q[0] = fma(w0, g0, q[0]);
-      q[1] = fma(w0, g1, q[1]);
-      q[2] = fma(w0, g2, q[2]);
-      q[3] = fma(w1, g1, q[3]);
-      q[4] = fma(w1, g2, q[4]);
-      q[5] = fma(w2, g2, q[5]);
+      const double gA[3] = {g[1 + 3 * la], g[2 + 3 * la], g[3 + 3 * la]};
 #pragma unroll
       for (int lb = 0; lb < 4; ++lb) {
-        const int b = lb == 0 ? tv.x : lb == 1 ? tv.y : lb == 2 ? tv.z : tv.w;
-        if (b <= a) continue;
-        int lo = 1, hi = nup;  // its slot
+        const int bv = lb == 0 ? tv.x : lb == 1 ? tv.y : lb == 2 ? tv.z : tv.w;
+        const double gB[3] = {g[1 + 3 * lb], g[2 + 3 * lb], g[3 + 3 * lb]};
+        const double xb[3] = {X[3 * (size_t)bv], X[3 * (size_t)bv + 1], X[3 * (size_t)bv + 2]};
+        int lo = 0, hi = len - 1;  // the block's place in the row
         while (lo < hi) {
           const int mid = (lo + hi) >> 1;
-          if (scol[mid * kRowPad + lane] < b) lo = mid + 1;
+          if (scol[mid * kRowPad + lane] < bv) lo = mid + 1;
           else hi = mid;
         }
-        double *p = P + 9 * lo * kRowPad + lane;
+        const double dd = gA[0] * gB[0] + gA[1] * gB[1] + gA[2] * gB[2];
+        double *blk = P + 9 * lo * kRowPad + lane;
 #pragma unroll
-        for (int j = 0; j < 3; ++j) {
-          const double gb = g[1 + 3 * lb + j];
-          p[j * kRowPad] = fma(w0, gb, p[j * kRowPad]);
-          p[(3 + j) * kRowPad] = fma(w1, gb, p[(3 + j) * kRowPad]);
-          p[(6 + j) * kRowPad] = fma(w2, gb, p[(6 + j) * kRowPad]);
-        }
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+          for (int j = 0; j < 3; ++j) {
+            const double sh = lam * gA[i] * gB[j] + mu * gA[j] * gB[i];
+            const double k = V * (i == j ? sh + mu * dd : sh);
+            blk[(3 * i + j) * kRowPad] += h2 * k;
+            kx[i] += k * xb[j];
+          }
       }
     }
-    const double lh = h2 * lam, mh = h2 * mu, c = 3.0 * lam + 2.0 * mu;
-    for (int s = 1; s <= nup; ++s) {
-      double *p = P + 9 * s * kRowPad + lane;
-      double e[9];
-#pragma unroll
-      for (int k = 0; k < 9; ++k) e[k] = p[k * kRowPad];
-      const double tr = mh * (e[0] + e[4] + e[8]);
-#pragma unroll
-      for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-          const double k = fma(mh, e[3 * j + i], lh * e[3 * i + j]);
-          p[(3 * i + j) * kRowPad] = i == j ? k + tr : k;
-        }
-    }
-    {  // the diagonal block: P is symmetric
-      const double tr = mh * (q[0] + q[3] + q[5]), s = lh + mh;
-      double *p = P + lane;
-      p[0] = fma(s, q[0], tr) + m;
-      p[4 * kRowPad] = fma(s, q[3], tr) + m;
-      p[8 * kRowPad] = fma(s, q[5], tr) + m;
-      p[kRowPad] = p[3 * kRowPad] = s * q[1];
-      p[2 * kRowPad] = p[6 * kRowPad] = s * q[2];
-      p[5 * kRowPad] = p[7 * kRowPad] = s * q[4];
-    }
+    int dg = 0;
+    while (scol[dg * kRowPad + lane] != a) ++dg;
+    for (int d = 0; d < 3; ++d) P[(9 * dg + 4 * d) * kRowPad + lane] += m;
     mass[a] = m;
-    for (int i = 0; i < 3; ++i) KX[3 * (size_t)a + i] = c * w[i];
+    for (int d = 0; d < 3; ++d) KX[3 * (size_t)a + d] = kx[d];
   }
   __syncwarp();
-  // Copy out row by row: the upper part, then the mirrored blocks, three at a
-  // time (27 lanes).
-  const int sub = lane / 9, e = lane - 9 * sub, et = 3 * (e % 3) + e / 3;
-  for (int r = 0; r < 32; ++r) {
-    const int dr = __shfl_sync(0xffffffffu, d, r), nr = __shfl_sync(0xffffffffu, nup, r);
-    if (nr < 0) break;
-    for (int k = lane; k < 9 * (nr + 1); k += 32) vals[9 * (size_t)dr + k] = P[k * kRowPad + r];
-    for (int s = 1 + sub; s <= nr; s += 3)
-      if (sub < 3) vals[9 * (size_t)spos[s * kRowPad + r] + e] = P[(9 * s + et) * kRowPad + r];
+  for (int r = 0; r < 32; ++r) {  // copy out row by row
+    const int rr = __shfl_sync(0xffffffffu, r0, r), n = 9 * __shfl_sync(0xffffffffu, len, r);
+    for (int k = lane; k < n; k += 32) vals[9 * (size_t)rr + k] = P[k * kRowPad + r];
   }
 }
 
-// The same for a mesh with a row too wide for shared memory: one thread per
-// vertex a adds the element blocks (in incidence order, scaled by h^2) to its
-// row in global memory, plus the lumped mass on the diagonal block; K X along
-// the way.
+// The same with the rows in global memory, one thread per vertex, for a mesh
+// with a row too wide for shared memory.
 __global__ void assemble_rows_kernel(int nv, const int *__restrict__ tets,
                                      const double *__restrict__ geom,
                                      const int *__restrict__ row_ptr, const int *__restrict__ cols,
@@ -348,7 +304,7 @@ int mprgp_fem_create(mprgp_context *ctx, int nv, int ntet, const int *tets, cons
   std::vector<int> row_ptr(nv + 1, 0), cols;
   cols.reserve(16LL * nv);
   std::vector<int> nb;
-  int max_up = 0;
+  int max_len = 0;
   for (int a = 0; a < nv; ++a) {
     nb.clear();
     nb.push_back(a);
@@ -360,7 +316,7 @@ int mprgp_fem_create(mprgp_context *ctx, int nv, int ntet, const int *tets, cons
     nb.erase(std::unique(nb.begin(), nb.end()), nb.end());
     cols.insert(cols.end(), nb.begin(), nb.end());
     row_ptr[a + 1] = (int)cols.size();
-    max_up = std::max(max_up, (int)(nb.end() - std::upper_bound(nb.begin(), nb.end(), a)));
+    max_len = std::max(max_len, (int)nb.size());
   }
   auto *f = new mprgp_fem();
   f->ctx = ctx;
@@ -368,7 +324,7 @@ int mprgp_fem_create(mprgp_context *ctx, int nv, int ntet, const int *tets, cons
   f->nv = nv;
   f->ntet = ntet;
   f->nnzb = row_ptr[nv];
-  f->max_up = max_up;
+  f->max_len = max_len;
   f->lam = poisson * young / ((1.0 + poisson) * (1.0 - 2.0 * poisson));
   f->mu = young / (2.0 * (1.0 + poisson));
   f->rho = rho;
@@ -425,14 +381,13 @@ int mprgp_fem_assemble(mprgp_fem *f, double h, const double gravity[3], const do
   cudaStream_t s = f->stream;
   const double g[3] = {gravity ? gravity[0] : 0.0, gravity ? gravity[1] : 0.0,
                        gravity ? gravity[2] : 0.0};
-  const int smem = upper_smem(f->max_up);
-  if (f->max_up < 1024 && smem <= kUpperSmemMax) {
-    if (smem > 48 * 1024)
-      FK(cudaFuncSetAttribute(assemble_upper_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              kUpperSmemMax));
-    assemble_upper_kernel<<<(f->nv + 31) / 32, 32, smem, s>>>(
-        f->nv, f->max_up, reinterpret_cast<const int4 *>(f->tets), f->geom, f->row_ptr, f->cols,
-        f->vt_ptr, f->vt, f->lam, f->mu, f->rho, h * h, f->vals, f->mass, f->KX);
+  const int smem = f->max_len < 1024 ? row_smem(f->max_len) : kRowSmemMax + 1;
+  if (smem <= kRowSmemMax) {
+    FK(cudaFuncSetAttribute(assemble_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                            kRowSmemMax));
+    assemble_smem_kernel<<<(f->nv + 31) / 32, 32, smem, s>>>(
+        f->nv, f->max_len, reinterpret_cast<const int4 *>(f->tets), f->geom, f->row_ptr, f->cols,
+        f->vt_ptr, f->vt, f->X, f->lam, f->mu, f->rho, h * h, f->vals, f->mass, f->KX);
   } else {
     assemble_rows_kernel<<<(f->nv + 127) / 128, 128, 0, s>>>(
         f->nv, f->tets, f->geom, f->row_ptr, f->cols, f->vt_ptr, f->vt, f->X, f->lam, f->mu,

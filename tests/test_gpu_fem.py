@@ -93,13 +93,23 @@ def _assembled(tets, X, E, nu, rho, h):
     return A
 
 
+def _hub(points, rng):
+    """Points on a spiral and one vertex (the first) joined to all of them."""
+    ang = np.arange(points - 1) * 0.37
+    ring = np.stack([np.cos(ang), np.sin(ang), 0.1 * np.arange(points - 1)], axis=1)
+    ring += 0.05 * rng.standard_normal(ring.shape)
+    i = np.arange(1, points - 2)
+    return (np.vstack([[0.1, 0.2, -1.0], ring]),
+            np.stack([np.zeros_like(i), i, i + 1, i + 2], axis=1))
+
+
 @pytest.mark.parametrize("points,hub", [
     (4, "first"),     # a single tet: one partial warp
     (33, "last"),     # one row past a warp
-    (84, "first"),    # the widest row that fits shared memory (83 blocks right of the hub's)
-    (86, "first"),    # one that does not: the form in global memory
+    (89, "first"),    # the widest row that fits shared memory
+    (90, "first"),    # one that does not: the form in global memory
     (150, "first"),
-    (150, "last"),    # the hub's row is as wide, its upper part empty
+    (150, "last"),
 ])
 def test_assembly_of_a_hub(ctx, points, hub):
     """A vertex joined to every other one, on both sides of the width that
@@ -107,12 +117,7 @@ def test_assembly_of_a_hub(ctx, points, hub):
     200 eps times the largest entry, and ten times that for the gradients'
     own rounding on random tets."""
     rng = np.random.default_rng(points)
-    ang = np.arange(points - 1) * 0.37
-    ring = np.stack([np.cos(ang), np.sin(ang), 0.1 * np.arange(points - 1)], axis=1)
-    ring += 0.05 * rng.standard_normal(ring.shape)
-    P = np.vstack([[0.1, 0.2, -1.0], ring])
-    i = np.arange(1, points - 2)
-    tets = np.stack([np.zeros_like(i), i, i + 1, i + 2], axis=1)
+    P, tets = _hub(points, rng)
     if hub == "last":
         P = np.vstack([P[1:], P[:1]])
         tets = (tets - 1) % points
@@ -134,3 +139,24 @@ def test_assembly_of_a_hub(ctx, points, hub):
     scale = np.abs(K).sum(axis=1).max() * np.abs(X).max() + np.abs(want).max()
     assert np.abs(b - want).max() <= 2000 * 2.2e-16 * scale
     fem.close()
+
+
+@pytest.mark.parametrize("dims", [(1, 1, 1), (3, 4, 7), (9, 9, 9)])
+def test_assembly_forms_agree(ctx, dims):
+    """A body beside a hub too wide for shared memory is assembled in global
+    memory; alone, in shared memory: the same operations in the same order, so
+    the same bits."""
+    rng = np.random.default_rng(5)
+    tets, X, x0, v0 = M.beam_mesh(*dims, young=1e5, poisson=0.4, v0_sigma=0.1, seed=3)
+    tets = np.asarray(tets).reshape(-1, 4)
+    X = X + 0.003 * rng.standard_normal(X.size)
+    P, hub = _hub(120, rng)
+    both = []
+    for t, x in ((tets, X), (np.vstack([tets, hub + X.size // 3]), np.hstack([X, P.ravel() + 9]))):
+        fem = M.FemMesh(ctx, t.astype(np.int32), x, 1e5, 0.4, 1000.0)
+        fem.assemble(0.01, (0.0, -9.8, 0.0), x)
+        both.append(fem.get())
+    nv = X.size // 3
+    nb = both[0][0][nv]
+    for one, two, n in zip(both[0], both[1], (nv + 1, nb, nb, X.size, nv)):
+        assert np.array_equal(np.asarray(one).reshape(n, -1), np.asarray(two)[:n].reshape(n, -1))
