@@ -189,6 +189,28 @@ def test_bounds_parity(ctx, kind_name, kind):
     assert np.array_equal(fg, fo)
 
 
+@pytest.mark.parametrize("dims", [(2, 2, 3), (6, 6, 14), (9, 9, 30)])
+@pytest.mark.parametrize("width", [0.0, 1e-9, 1e-4, 1e300])
+def test_box_widths(ctx, dims, width):
+    """Boxes from a point to none at all around every third unknown: steps far
+    over a bound, short of it, and bounds whose gap overflows.  Bound: that of
+    the other bound kinds against the oracle."""
+    qp = M.beam(*dims, seed=9)
+    A, b, _, _ = H.qp_from_beam(qp)
+    L, U = np.full(qp.n, -1e300), np.full(qp.n, 1e300)
+    L[1::3] = 0.0
+    L[0::3] = qp.x0[0::3] - width
+    U[0::3] = qp.x0[0::3] + width
+    x0 = np.clip(qp.x0, L, U)
+    tol = 1e-10 * np.linalg.norm(b)
+    xo, fo, so, _ = H.oracle_solve("box", A, b, x0, L=L, U=U, tol=tol, max_it=20000, seed=SEED)
+    opt = M.default_options(tol=tol, max_it=20000, kind=M.KIND_BOX, seed=SEED)
+    xg, fg, sg = ctx.solve_bsr(qp, opt, x0, L=L, U=U)
+    assert sg.code == so["code"] == 0
+    assert rel(xg, xo) <= 1e-8
+    assert np.array_equal(fg, fo)
+
+
 def test_batch_equals_single(ctx):
     qps = [M.beam(a, b, c, extra_planes_max=e, extra_planes_min=e, plane_mode=2, seed=s)
            for (a, b, c, e, s) in [(4, 4, 6, 0, 5), (3, 5, 7, 2, 6), (6, 4, 9, 1, 7)]]
