@@ -797,7 +797,7 @@ SyncPlan sync_plan(mprgp_context *c, int units, int max_slots, int fp32) {
       if (4 * units * q <= 3 * c->nsm && fits(q, 3)) return P;
   // Else the fewest CTAs an item whose slices fit shared memory, or twice as
   // many (smaller CTAs can pack an SM better).  1,760 vertices mixed: 4.85 us
-  // a phase with q = 1, 5.5 with 2, 4 or 8; 17,856 in FP64: 13.7 with q = 2,
+  // a phase with q = 1, 5.5 with 2, 4 or 8; 17,856 in FP64: 11.5 with q = 2,
   // 14.2 with 4, 18.3 with 8.
   int tried = 0;
   for (int q = 1; q <= kThreads / kSlice && tried < 2; q *= 2) {

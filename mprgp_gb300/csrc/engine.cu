@@ -4675,11 +4675,18 @@ cudaError_t power_persistent_max_blocks_per_sm(int fp32, int *n) {
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, power_persistent_fn(fp32), kStepThreads, 0);
 }
 // The power sync loop's kernel for q CTAs a unit and `comps` threads a row.
-static const void *power_sync_fn(int q, int fp32, int comps) {
+// A CTA that takes more than half of an SM's shared memory is alone there, so
+// its rows may have all the registers: with the 128 that three CTAs an SM leave
+// a thread, FP64 rows spill (17,856 vertices, two CTAs an item: 13.9 us a phase;
+// 11.5 alone with five slots in flight, 11.6 with 8 or 16, 11.9 with four, 12.2
+// with three).
+static const void *power_sync_fn(int q, int fp32, int comps, int smem) {
   if (comps == 3) return (const void *)power_sync_kernel<double, 3, 3 * kThreads / 4 + 32, 1, 16>;
   if (fp32)
     return q > 1 ? (const void *)power_sync_kernel<float, 1, kThreads / 2 + 32, 3, 8>
                  : (const void *)power_sync_kernel<float, 1, kStepThreads, 1, 8>;
+  if (q > 1 && smem > kSyncStageBytes / 2)
+    return (const void *)power_sync_kernel<double, 1, kThreads / 2 + 32, 1, 5>;
   return q > 1 ? (const void *)power_sync_kernel<double, 1, kThreads / 2 + 32, 3, 8>
                : (const void *)power_sync_kernel<double, 1, kStepThreads, 1, 8>;
 }
@@ -4702,7 +4709,7 @@ static void power_sync_config(int q, int comps, int grid, int smem, cudaStream_t
 // CTAs of that form that can be resident at once (smem: staged bytes a CTA).
 cudaError_t power_sync_capacity(int q, int fp32, int comps, int smem, int nsm, int *ctas) {
   *ctas = 0;
-  const void *fn = power_sync_fn(q, fp32, comps);
+  const void *fn = power_sync_fn(q, fp32, comps, smem);
   // (one value for every query: the attribute is the kernel's, not the launch's)
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kSyncStageBytes);
   if (e != cudaSuccess) return e;
@@ -4727,7 +4734,7 @@ cudaError_t launch_power_sync(const SyncArgs &args, int fp32, int comps, int gri
   cudaLaunchAttribute at[2];
   power_sync_config(args.q, comps, grid, smem, stream, cfg, at);
   void *params[] = {(void *)&args};
-  return cudaLaunchKernelExC(&cfg, power_sync_fn(args.q, fp32, comps), params);
+  return cudaLaunchKernelExC(&cfg, power_sync_fn(args.q, fp32, comps, smem), params);
 }
 cudaError_t power_max_blocks_per_sm(int variant, int *n) {
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, power_kernel_fn(variant),
