@@ -260,9 +260,12 @@ __device__ __forceinline__ double seeded_uniform(unsigned long long seed, unsign
 // is one coalesced line; x is gathered per neighbour vertex.  VT is the value
 // type of A and of the accumulator (FP32 accumulation for the FP32 copy).
 struct SrcV {
-  static constexpr int kChunk = 4;
+  static constexpr int kChunk = 3;
   const double *p;
   __device__ __forceinline__ void operator()(int c, double o[3]) const { ld3(p, c, o); }
+};
+struct SrcV4 : SrcV {
+  static constexpr int kChunk = 4;
 };
 struct SrcPNew {
   static constexpr int kChunk = 3;  // z - beta p   (CGStep's p = z - beta*p)
@@ -394,8 +397,10 @@ __device__ __forceinline__ int col_of(const SellMatrix &A, size_t j, int lane, i
 // follows from the registers a slot takes: three for the FP32 power pass
 // (48.2 us a phase on 348,145 vertices, 50.6 with four, 56.5 with five: spills;
 // and a tetrahedral grid's 15 blocks a row leave no rest), two for the CG pass,
-// which gathers two vectors (a timestep's solve 86.2 ms, 90.5 with four), four
-// for the rest (the standalone FP64 product: two 95, three and four 89 us).
+// which gathers two vectors (a timestep's solve 86.2 ms, 90.5 with four), three
+// for the FP64 passes of the solver (the same solve 83.8 ms, 84.7 with four; an
+// FP64 solve of 24,696 vertices 17.6, 17.9 with four), and four for the
+// standalone FP64 product (two 95, three and four 89 us).
 template <bool k16, typename VT, typename Src>
 __device__ __forceinline__ void spmv_row_body(const SellMatrix &A, const VT *__restrict__ vals,
                                               int lane, int vrow, int j0, int j1,
@@ -1538,12 +1543,15 @@ template <bool kPre>
 __device__ __noinline__ void row_cg_spmv(const InstDesc &D, const InstState &S, int v, int slot,
                                          double *part) {
   const bool f32 = D.prec == PREC_MIXED;
+  // The direction and the gradient at the row are read after the product, whose
+  // slots in flight need the registers.
   double p[3], ap[3], g[3];
-  ld3(B(D, B_G0 + S.gc), v, g);
+  const double *pr = B(D, B_P0 + S.pc);  // the direction
+  if constexpr (kPre) ld3(B(D, B_G0 + S.gc), v, g);
   if (S.phase == PH_CG_ENTRY || (S.phase == PH_PL_SPMV && S.p_is_z)) {
-    const double *pp = B(D, B_P0 + S.pc);
-    ld3(pp, v, p);
+    ld3(pr, v, p);
     if (S.phase == PH_CG_ENTRY && !S.g_cons) {
+      ld3(B(D, B_G0 + S.gc), v, g);
       double ax[3];
       row_product<kPre>(D, slot, 1, SrcV{B(D, B_X0 + S.xc)}, ax);
       double e[3];
@@ -1555,7 +1563,7 @@ __device__ __noinline__ void row_cg_spmv(const InstDesc &D, const InstState &S, 
     if constexpr (kPre)
       pre_product(0, ap);
     else
-      spmv_any(D, f32 && S.phase != PH_PL_SPMV, slot, SrcV{pp},
+      spmv_any(D, f32 && S.phase != PH_PL_SPMV, slot, SrcV{pr},
                SrcF{f32 ? D.buf32[F_P0 + S.pc] : nullptr}, ap);
   } else {
     const double *zz = B(D, B_Z0 + S.zc), *po = B(D, B_P0 + S.pc);
@@ -1564,6 +1572,7 @@ __device__ __noinline__ void row_cg_spmv(const InstDesc &D, const InstState &S, 
     ld3(po, v, p);
 #pragma unroll
     for (int d = 0; d < 3; ++d) p[d] = z[d] - S.beta_cg * p[d];
+    pr = B(D, B_P0 + (S.pc ^ 1));
     st3(B(D, B_P0 + (S.pc ^ 1)), v, p);
     const bool f32p = f32 && S.phase != PH_PL_SPMV;
     if (f32p) st3f(D.buf32[F_P0 + (S.pc ^ 1)], v, p);
@@ -1575,11 +1584,16 @@ __device__ __noinline__ void row_cg_spmv(const InstDesc &D, const InstState &S, 
                         f32p ? D.buf32[F_P0 + S.pc] : nullptr, (float)S.beta_cg}, ap);
     if (S.e_nz && S.phase == PH_CG_SPMV) {
       double e[3];
+      ld3(pr, v, p);
       ld3(B(D, B_E), v, e);
       part[2] += dot3(p, e);
     }
   }
   st3(B(D, B_AP), v, ap);
+  if constexpr (!kPre) {
+    ld3(pr, v, p);
+    ld3(B(D, B_G0 + S.gc), v, g);
+  }
   part[0] += dot3(p, ap);
   part[1] += dot3(p, g);
   if (S.phase == PH_PL_SPMV) {
@@ -1665,25 +1679,25 @@ __device__ __noinline__ void cg_yf_box(const InstDesc &D, const InstState &S, in
 __device__ __noinline__ void row_cg_yf(const InstDesc &D, const InstState &S, int v, int slot,
                                        double *part) {
   (void)slot;
+  if (D.kind < KIND_DECOUPLED) {
+    cg_yf_box(D, S, v, part);
+    return;
+  }
+  double ap[3], y[3], gy[3], x[3], p[3], g[3];  // (before the constraints: one round trip)
+  ld3(B(D, B_X0 + S.xc), v, x);
+  ld3(B(D, B_P0 + S.pc), v, p);
+  ld3(B(D, B_AP), v, ap);
+  ld3(B(D, B_G0 + S.gc), v, g);
   VSep C;
   if (!load_cons(D, v, C)) {
-    if (D.kind < KIND_DECOUPLED) cg_yf_box(D, S, v, part);
-    else cg_yf_general(D, S, v, part);
+    cg_yf_general(D, S, v, part);
     return;
   }
   const int f = load_face(D, C);
-  double ap[3], y[3], gy[3];
-  ld3(B(D, B_AP), v, ap);
-  {
-    double x[3], p[3], g[3];
-    ld3(B(D, B_X0 + S.xc), v, x);
-    ld3(B(D, B_P0 + S.pc), v, p);
-    ld3(B(D, B_G0 + S.gc), v, g);
 #pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      y[d] = x[d] - S.alpha * p[d];
-      gy[d] = g[d] - S.alpha * ap[d];
-    }
+  for (int d = 0; d < 3; ++d) {
+    y[d] = x[d] - S.alpha * p[d];
+    gy[d] = g[d] - S.alpha * ap[d];
   }
   st3(B(D, B_X0 + (S.xc ^ 1)), v, y);
   st3(B(D, B_G0 + (S.gc ^ 1)), v, gy);
@@ -3314,7 +3328,10 @@ struct Row3 {
 template <typename VT>
 __device__ __noinline__ Row3<VT> sync_row_first(const InstDesc &D, int src, int slot) {
   Row3<VT> r;
-  pow_raw(D, src, slot, r.w);
+  if constexpr (sizeof(VT) == 8)
+    spmv_row<double>(D.A, D.A.v64, slot, SrcV4{src < 0 ? D.ev : B(D, src)}, r.w);
+  else
+    pow_raw(D, src, slot, r.w);
   return r;
 }
 
@@ -4312,7 +4329,7 @@ __global__ void __launch_bounds__(256, MPRGP_SPMV_MIN_BLOCKS) spmv_kernel(SellMa
   const int v = row_vertex(A, slot);
   double o[3];
   if constexpr (sizeof(VT) == 4) spmv_row<VT>(A, vals, slot, SrcVtoF{x}, o);
-  else spmv_row<VT>(A, vals, slot, SrcV{x}, o);
+  else spmv_row<VT>(A, vals, slot, SrcV4{x}, o);
   st3(y, v, o);
 }
 
