@@ -30,7 +30,8 @@ cudaError_t launch_engine(const EngineArgs &args, int grid, cudaStream_t stream)
 cudaError_t build_power_graph(int grid, int variant, const EngineArgs *d_args, PowCtl *d_pc,
                               cudaGraph_t *graph, cudaGraphExec_t *exec);
 cudaError_t power_max_blocks_per_sm(int variant, int *n);
-cudaError_t launch_power_persistent(const SyncArgs &args, int fp32, int grid, cudaStream_t stream);
+cudaError_t launch_power_persistent(const SyncArgs &args, int fp32, int per_sm, int grid,
+                                    cudaStream_t stream);
 cudaError_t power_persistent_max_blocks_per_sm(int fp32, int *n);
 cudaError_t launch_power_clusters(const SyncArgs &args, int fp32, int csize, cudaStream_t stream);
 cudaError_t power_clusters_max_active(int csize, int *n);
@@ -1254,9 +1255,12 @@ int engine_begin(mprgp_context *c, int k, int n, mprgp_problem *const *probs,
     sa.units = sync.units;
     sa.q = std::max(1, plan.q);
     const int fp32 = sync.fp32 ? 1 : 0;
+    // (beside other kernels the persistent loop leaves them registers)
+    const bool alone = k == 0 && (n == n_large || small_in_plan);
+    const int per_sm = alone ? (plan.grid + c->nsm - 1) / c->nsm : c->bps_power_pp;
     CK(gated_launch(s, [&] {
       return plan.q > 0 ? launch_power_sync(sa, fp32, plan.comps, plan.grid, plan.smem, s)
-                        : launch_power_persistent(sa, fp32, plan.grid, s);
+                        : launch_power_persistent(sa, fp32, per_sm, plan.grid, s);
     }));
     CK(cudaEventRecord(L.e_pow, s));
   }

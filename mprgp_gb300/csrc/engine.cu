@@ -4638,13 +4638,24 @@ cudaError_t cluster_max_active(int csize, int *n) {
   cfg.numAttrs = 1;
   return cudaOccupancyMaxActiveClusters(n, cluster_kernel, &cfg);
 }
-static const void *power_persistent_fn(int fp32) {
+// The CTAs an SM holds at once set the registers of a row: a run of one or two
+// items an SM has the room, and its rows then wait for fewer loads at a time
+// (24,696 vertices, FP64: 14.9 -> 14.0 us a phase with room for two; 50,625
+// mixed: 8.6 -> 7.8).  Three an SM help FP32 rows (92,256 vertices: 11.0 ->
+// 10.1 us); FP64 rows, which the FP64 unit bounds there, take 39.6 so and 38.6
+// with room for four.
+static const void *power_persistent_fn(int fp32, int per_sm = 4) {
+  if (per_sm <= 2)
+    return fp32 ? (const void *)power_persistent_kernel<float, 2>
+                : (const void *)power_persistent_kernel<double, 2>;
+  if (per_sm == 3 && fp32) return (const void *)power_persistent_kernel<float, 3>;
   return fp32 ? (const void *)power_persistent_kernel<float, 4>
               : (const void *)power_persistent_kernel<double, 4>;
 }
-cudaError_t launch_power_persistent(const SyncArgs &args, int fp32, int grid, cudaStream_t stream) {
+cudaError_t launch_power_persistent(const SyncArgs &args, int fp32, int per_sm, int grid,
+                                    cudaStream_t stream) {
   void *params[] = {(void *)&args};
-  return cudaLaunchCooperativeKernel(power_persistent_fn(fp32), dim3(grid), dim3(kStepThreads),
+  return cudaLaunchCooperativeKernel(power_persistent_fn(fp32, per_sm), dim3(grid), dim3(kStepThreads),
                                      params, 0, stream);
 }
 // The same kernel with the items of each instance in one cluster of `csize`
