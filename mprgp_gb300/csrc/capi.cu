@@ -1059,9 +1059,11 @@ int engine_begin(mprgp_context *c, int k, int n, mprgp_problem *const *probs,
   // The power method in the forms whose CTAs wait for each other (unless the
   // tuning asks for the launch loops): a synchronous run's instances, small
   // ones too, by the power sync loop when all their CTAs are resident at once;
-  // else its large ones by the persistent loop; small ones, on every lane, by
-  // the persistent loop's kernel with one cluster an instance.
-  const bool waiting = power_launches > 0 && c->power_kernel && c->power_graph && c->power_step;
+  // else its large ones by the persistent loop and its small ones by the same
+  // kernel with one cluster an instance.  A server's asynchronous lanes keep
+  // the launch loops and the cluster solver: kernels that wait for their peers
+  // stay out of runs that share the SMs with other streams.
+  const bool waiting = k == 0 && power_launches > 0 && c->power_kernel && c->power_graph && c->power_step;
   const bool alone = k == 0 && !other_lanes_active(c, k);
   struct Count {
     int units = 0, slots = 0, fp32 = 0, n = 0;
@@ -1092,10 +1094,7 @@ int engine_begin(mprgp_context *c, int k, int n, mprgp_problem *const *probs,
     plan = sync_plan(c, all.units, all.slots, all.fp32 ? 1 : 0);
     small_in_plan = plan.grid > 0;
   }
-  // ... and on a server's power lane in the mixed form (a burst of 48 requests
-  // 39.3 -> 33.2 ms; in FP64, 91.3 -> 92.3, the graph loop stays)
-  if ((alone || (k == 3 && large.fp32 > 0)) && large.one() && plan.grid == 0)
-    plan = persistent_plan(c, large.units);
+  if (alone && large.one() && plan.grid == 0) plan = persistent_plan(c, large.units);
   R.power_sync = plan.grid > 0;
   const Count &sync = small_in_plan ? all : large;
   // The instances' other phases: the waiting engine for the large ones of a
@@ -1256,8 +1255,8 @@ int engine_begin(mprgp_context *c, int k, int n, mprgp_problem *const *probs,
     sa.q = std::max(1, plan.q);
     const int fp32 = sync.fp32 ? 1 : 0;
     // (beside other kernels the persistent loop leaves them registers)
-    const bool alone = k == 0 && (n == n_large || small_in_plan);
-    const int per_sm = alone ? (plan.grid + c->nsm - 1) / c->nsm : c->bps_power_pp;
+    const bool no_clusters = n == n_large || small_in_plan;
+    const int per_sm = no_clusters ? (plan.grid + c->nsm - 1) / c->nsm : c->bps_power_pp;
     CK(gated_launch(s, [&] {
       return plan.q > 0 ? launch_power_sync(sa, fp32, plan.comps, plan.grid, plan.smem, s)
                         : launch_power_persistent(sa, fp32, per_sm, plan.grid, s);

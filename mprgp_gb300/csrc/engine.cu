@@ -3601,7 +3601,7 @@ __global__ void __launch_bounds__(kThr, kMinBlocks) power_sync_kernel(SyncArgs a
 // as graph launches; its matrix pass alone, L2-resident, takes 10.4).
 // Instances do not wait for each other.  With the items of an instance in one
 // cluster the same kernel needs no cooperative launch (the cluster's CTAs are
-// resident together): the small instances of a batch or a server lane, which
+// resident together): the small instances of a batch, which
 // took 9.7 us a phase in the cluster solver, take about 7.  The results are
 // the launch form's bits.
 // Waits until an instance's items have all counted phase t - 1, `target` in
@@ -4661,7 +4661,7 @@ cudaError_t launch_power_persistent(const SyncArgs &args, int fp32, int per_sm, 
 // The same kernel with the items of each instance in one cluster of `csize`
 // CTAs (args.items holds csize units an instance, absent ones with limit 0).
 // A cluster's CTAs are resident together, so no cooperative launch is needed
-// and any number of instances can be queued beside other lanes' kernels.
+// and any number of instances can be queued.
 static void power_clusters_config(int csize, int grid, cudaStream_t stream, cudaLaunchConfig_t &cfg,
                                   cudaLaunchAttribute (&at)[1]) {
   cfg = {};
