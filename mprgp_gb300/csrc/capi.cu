@@ -1244,6 +1244,7 @@ int engine_begin(mprgp_context *c, int k, int n, mprgp_problem *const *probs,
   std::memset(&sa, 0, sizeof(sa));
   sa.desc = L.d_desc;
   sa.states = L.d_st;
+  sa.ninst = n;
   sa.wait_ns = args.wait_ns;
   sa.ctl = L.ctl;
   // The cluster-size classes run on side streams, concurrently with each
@@ -1296,6 +1297,7 @@ int engine_begin(mprgp_context *c, int k, int n, mprgp_problem *const *probs,
     ea.units = eng.units;
     ea.q = eplan.q;
     ea.max_phases = args.max_phases;
+    ea.ninst = n;
     ea.wait_ns = args.wait_ns;
     ea.total_ns = args.total_ns;
     ea.ctl = L.ctl;
@@ -1435,7 +1437,9 @@ int engine_end(mprgp_context *c, int k, mprgp_stats *stats, int *done) {
     if (done) done[i] = finished || err || (!finished && unbounded);
     if ((finished || err || unbounded) && x.code < worst) worst = x.code;
   }
-  if (ctl1.err) return fail(ctl1.err, "device wait limit reached");
+  if (ctl1.err)
+    return fail(ctl1.err, ctl1.err == kCodeLaunch ? "a kernel was launched with another shape than its own"
+                                                  : "device wait limit reached");
   return worst < MPRGP_NOT_CONVERGED ? worst : MPRGP_OK;
 }
 

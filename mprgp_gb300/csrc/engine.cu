@@ -19,6 +19,7 @@
 #include <cuda_runtime.h>
 
 #include "engine.h"
+#include "split_launch.h"
 
 namespace mprgp {
 
@@ -50,10 +51,11 @@ constexpr double kEps = 1e-9;  // ScalarUtil<double>::scalar_eps (MathBasic.cpp:
 // ------------------------------------------------------------ primitives --
 // Bounds-checked debug build (-DMPRGP_CHECKS): indices the kernels read from
 // device arrays -- block columns, SELL row order, plane offsets -- are checked
-// before use.  A bad one sets a bit in the instance's invalid-input word
-// (2: block column, 4: plane offsets, 8: SELL row) and is replaced by a safe
-// index, so nothing is read out of bounds; the solve then reports
-// MPRGP_INVALID.  The release build compiles the checks out.
+// before use, and the waiting kernels' staged slices against their shared
+// memory.  A bad one sets a bit in the instance's invalid-input word
+// (2: block column, 4: plane offsets, 8: SELL row, 16: staged slices) and is
+// replaced by a safe index, so nothing is read out of bounds; the solve then
+// reports MPRGP_INVALID.  The release build compiles the checks out.
 #ifdef MPRGP_CHECKS
 #define MPRGP_CHECK(cond, word, bit, fix) \
   do {                                    \
@@ -3335,12 +3337,23 @@ __device__ __noinline__ Row3<VT> sync_row_first(const InstDesc &D, int src, int 
   return r;
 }
 
-// Slices of one unit part in shared memory: the values as in global memory,
-// then the columns as vertices.  One pass before the loop.
+// Slices s0..s1 of one unit part in shared memory: the values as in global
+// memory, then the columns as vertices.  One pass before the loop.  Returns the
+// first slot and the number of slots staged; `used` bytes of the dynamic shared
+// memory lie before `dst`.
+__device__ __forceinline__ unsigned int dynamic_smem() {
+  unsigned int r;
+  asm volatile("mov.u32 %0, %%dynamic_smem_size;" : "=r"(r));
+  return r;
+}
 template <typename VT>
-__device__ __forceinline__ void sync_stage(const SellMatrix &A, const VT *vals, int s0, int s1,
-                                           int threads, unsigned char *dst) {
-  const int f = ldro(A.slice_off + s0), l = ldro(A.slice_off + s1);
+__device__ __forceinline__ int2 sync_stage(const SellMatrix &A, const VT *vals, int s0, int s1,
+                                           int threads, unsigned char *dst, int used) {
+  const int f = ldro(A.slice_off + s0);
+  int l = ldro(A.slice_off + s1);
+  MPRGP_CHECK(l >= f && (long long)used + (long long)(l - f) * kSlice * (9 * (int)sizeof(VT) + 4) <=
+                            (long long)dynamic_smem(),
+              A.bad, 16, l = f);
   const int nv16 = (l - f) * 9 * kSlice * (int)sizeof(VT) / 16;
   const float4 *src = reinterpret_cast<const float4 *>(vals + (size_t)f * (9 * kSlice));
   for (int i = threadIdx.x; i < nv16; i += threads) cp_async16(dst + 16 * (size_t)i, src + i);
@@ -3348,6 +3361,17 @@ __device__ __forceinline__ void sync_stage(const SellMatrix &A, const VT *vals, 
   for (int i = threadIdx.x; i < (l - f) * kSlice; i += threads)
     sc[i] = checked_col(A, ldro(A.cols + (size_t)f * kSlice + i));
   asm volatile("cp.async.wait_all;\n" ::: "memory");
+  return make_int2(f, l - f);
+}
+
+// A launch whose shape or unit list is not what the kernel was written for: the
+// CTA reports it and leaves, before its first access to a peer's shared memory
+// or to an instance.
+__device__ __forceinline__ void refuse(Ctl *ctl) {
+  if (threadIdx.x == 0) atomicCAS(&ctl->err, 0, kCodeLaunch);
+}
+__device__ __forceinline__ bool unit_ok(const SyncItem &u, int ninst) {
+  return u.inst >= 0 && u.inst < ninst && u.local >= 0;
 }
 
 __device__ __forceinline__ double sq3(const float d[3]) {
@@ -3388,7 +3412,7 @@ __global__ void __launch_bounds__(kThr, kMinBlocks) power_sync_kernel(SyncArgs a
   __shared__ double sPart[2][kThreads];
   __shared__ double sVec[kComps == 3 ? 2 : 1][kComps][kComps == 3 ? kThreads / 4 : 1];  // d, w by row
   __shared__ int sFail[2], sLeave;       // this CTA's wait ran out (by phase parity); a peer's did
-  const int q = kSplit ? args.q : 1;     // CTAs of a unit (a cluster)
+  const int q = kSplit ? (int)cluster_size() : 1;  // CTAs of a unit (a cluster)
   const int rank = q > 1 ? (int)cluster_rank() : 0;
   const int R = kThreads / q;            // rows of this CTA
   const int threads = R * kComps + 32;
@@ -3396,7 +3420,16 @@ __global__ void __launch_bounds__(kThr, kMinBlocks) power_sync_kernel(SyncArgs a
   const bool rw = (int)threadIdx.x >= R * kComps;  // the reduction warp
   const int comp = kComps == 3 ? warp % 3 : 0;     // the thread's component and
   const int ri = (kComps == 3 ? warp / 3 : warp) * 32 + lane;  // row of the CTA
+  if (!split_shape_ok(args.q, args.units, threads, (int)cluster_size(), (int)gridDim.x,
+                      (int)blockDim.x)) {
+    refuse(args.ctl);
+    return;
+  }
   const SyncItem unit = args.items[(int)blockIdx.x / q];
+  if (!unit_ok(unit, args.ninst)) {  // (the same unit in every CTA of a cluster)
+    refuse(args.ctl);
+    return;
+  }
   if (threadIdx.x == 0) {
     g_staged = 0;
     sFail[0] = sFail[1] = sLeave = 0;
@@ -3412,6 +3445,10 @@ __global__ void __launch_bounds__(kThr, kMinBlocks) power_sync_kernel(SyncArgs a
   __syncthreads();
   const InstDesc &D = sD;
   InstState &S = sS;
+  if (unit.local >= D.nitems) {
+    refuse(args.ctl);
+    return;
+  }
   // the thread's row, its slots in the staged copy, its vectors
   const int slot = unit.local * kThreads + rank * R + ri;
   const bool row = !rw && slot < D.nv;
@@ -3423,13 +3460,14 @@ __global__ void __launch_bounds__(kThr, kMinBlocks) power_sync_kernel(SyncArgs a
   {
     const int s0 = min(unit.local * (kThreads / kSlice) + rank * (R / kSlice), D.A.nslices);
     const int s1 = min(s0 + R / kSlice, D.A.nslices);
-    sync_stage(D.A, sizeof(VT) == 4 ? reinterpret_cast<const VT *>(D.A.v32)
-                                    : reinterpret_cast<const VT *>(D.A.v64), s0, s1, threads, g_stage);
-    const int f = ldro(D.A.slice_off + s0), l = ldro(D.A.slice_off + s1);
-    voff = (l - f) * 9 * kSlice * (int)sizeof(VT);
+    const int2 staged = sync_stage(
+        D.A, sizeof(VT) == 4 ? reinterpret_cast<const VT *>(D.A.v32)
+                             : reinterpret_cast<const VT *>(D.A.v64),
+        s0, s1, threads, g_stage, 0);
+    voff = staged.y * 9 * kSlice * (int)sizeof(VT);
     if (row) {
-      j0 = ldro(D.A.slice_off + (slot >> 5)) - f;
-      j1 = ldro(D.A.slice_off + (slot >> 5) + 1) - f;
+      j0 = min(ldro(D.A.slice_off + (slot >> 5)) - staged.x, staged.y);
+      j1 = min(ldro(D.A.slice_off + (slot >> 5) + 1) - staged.x, staged.y);
       if (S.phase == PH_POW || S.phase == PH_POW_LAST) {  // resumed, or started from ev
         for (int d = 0; d < kN; ++d) {
           const size_t i = 3 * (size_t)v + comp + d;
@@ -3657,6 +3695,10 @@ __global__ void __launch_bounds__(kStepThreads, kMinBlocks)
                                     (int)gridDim.x);
   for (int o = 0; o < nown; ++o) {
     const SyncItem it = args.items[blockIdx.x + o * gridDim.x];
+    if (!unit_ok(it, args.ninst)) {  // (its peers find the error while they wait)
+      refuse(args.ctl);
+      return;
+    }
     if (threadIdx.x == 0) sItem[o] = it;
     const int *srcd = reinterpret_cast<const int *>(args.desc + it.inst);
     int *dstd = reinterpret_cast<int *>(&sD[o]);
@@ -3669,6 +3711,11 @@ __global__ void __launch_bounds__(kStepThreads, kMinBlocks)
   }
   if (threadIdx.x == 0) sFail = 0;
   __syncthreads();
+  for (int o = 0; o < nown; ++o)  // a unit past the instance's items is an absent one, without phases
+    if (sItem[o].local >= sD[o].nitems && sItem[o].limit > 0) {
+      refuse(args.ctl);
+      return;
+    }
   unsigned int pend = 0u;  // bit o: item o's rows ran in the previous phase
   for (int t = 0;; ++t) {
     const int par = t & 1;
@@ -3938,9 +3985,13 @@ __global__ void __launch_bounds__(kThr, 1) engine_sync_kernel(EngineSyncArgs arg
   __shared__ int sSlot[kOwn], sMoved[kOwn];  // item o: its state copy; its rows matter in PH_CG_DAD
   __shared__ double sums[kPart];
   __shared__ int sFail;
-  const int q = kSplit ? args.q : 1;
+  const int q = kSplit ? (int)cluster_size() : 1;
   const int rank = q > 1 ? (int)cluster_rank() : 0;
   const int R = kThreads / q;  // rows of this CTA's part of a unit
+  if (kSplit && !split_shape_ok(args.q, args.units, kThr, q, (int)gridDim.x, (int)blockDim.x)) {
+    refuse(args.ctl);
+    return;
+  }
   const int threads = blockDim.x, ngroups = kSplit ? 1 : threads / kThreads;
   const int g = kSplit ? 0 : (int)threadIdx.x / kThreads;
   const int gt = kSplit ? (int)threadIdx.x : (int)threadIdx.x & (kThreads - 1);
@@ -3950,6 +4001,10 @@ __global__ void __launch_bounds__(kThr, 1) engine_sync_kernel(EngineSyncArgs arg
   const long long t_start = gtimer();
   for (int o = 0; o < nown; ++o) {
     const SyncItem it = args.items[u0 + o * ustep];
+    if (!unit_ok(it, args.ninst)) {  // (a split unit's CTAs agree; others' peers find the error)
+      refuse(args.ctl);
+      return;
+    }
     if (threadIdx.x == 0) {
       sItem[o] = it;
       sMoved[o] = 1;
@@ -3973,6 +4028,11 @@ __global__ void __launch_bounds__(kThr, 1) engine_sync_kernel(EngineSyncArgs arg
       if (sItem[o].local != 0 || rank != 0) sD[o].trace = nullptr;
   }
   __syncthreads();
+  for (int o = 0; o < nown; ++o)
+    if (sItem[o].local >= sD[o].nitems) {
+      refuse(args.ctl);
+      return;
+    }
   int v_split = 0;  // the row's vertex (a split unit's CTA keeps its rows)
   if (kSplit) {
     const int ri = kPre ? pre_row() : gt;
@@ -3986,13 +4046,13 @@ __global__ void __launch_bounds__(kThr, 1) engine_sync_kernel(EngineSyncArgs arg
     const int s0 = min(sItem[0].local * (kThreads / kSlice) + rank * (R / kSlice), A.nslices);
     const int s1 = min(s0 + R / kSlice, A.nslices);
     unsigned char *dst = g_engine + sizeof(RedBuf);
-    sync_stage(A, A.v64, s0, s1, threads, dst);
-    const int f = ldro(A.slice_off + s0), l = ldro(A.slice_off + s1), sl = s0 + (pre_row() >> 5);
+    const int2 slots = sync_stage(A, A.v64, s0, s1, threads, dst, (int)sizeof(RedBuf));
+    const int sl = s0 + (pre_row() >> 5);
     staged.sv = reinterpret_cast<const double *>(dst);
-    staged.sc = reinterpret_cast<const int *>(dst + (size_t)(l - f) * 9 * kSlice * sizeof(double));
+    staged.sc = reinterpret_cast<const int *>(dst + (size_t)slots.y * 9 * kSlice * sizeof(double));
     if (sl < s1) {
-      staged.j0 = ldro(A.slice_off + sl) - f;
-      staged.j1 = ldro(A.slice_off + sl + 1) - f;
+      staged.j0 = min(ldro(A.slice_off + sl) - slots.x, slots.y);
+      staged.j1 = min(ldro(A.slice_off + sl + 1) - slots.x, slots.y);
     }
     __syncthreads();
   }
@@ -4431,21 +4491,10 @@ cudaError_t launch_engine(const EngineArgs &args, int grid, cudaStream_t stream)
 }
 // The waiting engine with q CTAs a unit, or (q == 1) CTAs of `groups` groups.
 static void engine_sync_config(int q, int groups, int grid, int smem, cudaStream_t stream,
-                               cudaLaunchConfig_t &cfg, cudaLaunchAttribute (&at)[2]) {
-  cfg = {};
-  cfg.gridDim = dim3((unsigned int)grid);
+                               SplitLaunch &L) {
   // four or eight CTAs a unit: three threads a row, and warps that only sum
-  cfg.blockDim = dim3(q > 2 ? kThreads : q > 1 ? kThreads / 2 : groups * kThreads);
-  cfg.dynamicSmemBytes = sizeof(RedBuf) * (q > 1 ? 1 : groups) + (size_t)smem;
-  cfg.stream = stream;
-  at[0].id = cudaLaunchAttributeCooperative;
-  at[0].val.cooperative = 1;
-  at[1].id = cudaLaunchAttributeClusterDimension;
-  at[1].val.clusterDim.x = (unsigned int)q;
-  at[1].val.clusterDim.y = 1;
-  at[1].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = q > 1 ? 2 : 1;
+  split_launch(L, q, grid, q > 2 ? kThreads : q > 1 ? kThreads / 2 : groups * kThreads,
+               sizeof(RedBuf) * (q > 1 ? 1 : groups) + (size_t)smem, stream);
 }
 static const void *engine_sync_fn(int q) {
   return q > 2   ? (const void *)engine_sync_kernel<kThreads, true, true>
@@ -4454,11 +4503,10 @@ static const void *engine_sync_fn(int q) {
 }
 cudaError_t launch_engine_sync(const EngineSyncArgs &args, int groups, int grid, int smem,
                                cudaStream_t stream) {
-  cudaLaunchConfig_t cfg;
-  cudaLaunchAttribute at[2];
-  engine_sync_config(args.q, groups, grid, smem, stream, cfg, at);
+  SplitLaunch L;
+  engine_sync_config(args.q, groups, grid, smem, stream, L);
   void *params[] = {(void *)&args};
-  return cudaLaunchKernelExC(&cfg, engine_sync_fn(args.q), params);
+  return cudaLaunchKernelExC(&L.cfg, engine_sync_fn(args.q), params);
 }
 // CTAs of that form that can be resident at once (q == 1: of four groups; smem:
 // staged bytes a CTA).
@@ -4469,18 +4517,15 @@ cudaError_t engine_sync_capacity(int q, int smem, int nsm, int *ctas) {
                                              : (int)sizeof(RedBuf) * 4);
   *ctas = 0;
   if (e != cudaSuccess) return e;
-  cudaLaunchConfig_t cfg;
-  cudaLaunchAttribute at[2];
-  engine_sync_config(q, 4, q, smem, nullptr, cfg, at);
+  SplitLaunch L;
+  engine_sync_config(q, 4, q, smem, nullptr, L);
   if (q == 1) {
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, engine_sync_fn(1), 4 * kThreads,
-                                                      cfg.dynamicSmemBytes);
+                                                      L.cfg.dynamicSmemBytes);
     *ctas = n * nsm;
     return e;
   }
-  cfg.attrs = at + 1;
-  cfg.numAttrs = 1;
-  e = cudaOccupancyMaxActiveClusters(&n, engine_sync_fn(q), &cfg);
+  e = cudaOccupancyMaxActiveClusters(&n, engine_sync_fn(q), &L.cfg);
   *ctas = n * q;
   return e;
 }
@@ -4719,20 +4764,8 @@ static const void *power_sync_fn(int q, int fp32, int comps, int smem) {
                : (const void *)power_sync_kernel<double, 1, kStepThreads, 1, 8>;
 }
 static void power_sync_config(int q, int comps, int grid, int smem, cudaStream_t stream,
-                              cudaLaunchConfig_t &cfg, cudaLaunchAttribute (&at)[2]) {
-  cfg = {};
-  cfg.gridDim = dim3((unsigned int)grid);
-  cfg.blockDim = dim3((unsigned int)(kThreads / q * comps + 32));
-  cfg.dynamicSmemBytes = (size_t)smem;
-  cfg.stream = stream;
-  at[0].id = cudaLaunchAttributeCooperative;
-  at[0].val.cooperative = 1;
-  at[1].id = cudaLaunchAttributeClusterDimension;
-  at[1].val.clusterDim.x = (unsigned int)q;
-  at[1].val.clusterDim.y = 1;
-  at[1].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = q > 1 ? 2 : 1;
+                              SplitLaunch &L) {
+  split_launch(L, q, grid, kThreads / q * comps + 32, (size_t)smem, stream);
 }
 // CTAs of that form that can be resident at once (smem: staged bytes a CTA).
 cudaError_t power_sync_capacity(int q, int fp32, int comps, int smem, int nsm, int *ctas) {
@@ -4747,22 +4780,18 @@ cudaError_t power_sync_capacity(int q, int fp32, int comps, int smem, int nsm, i
     *ctas = n * nsm;
     return e;
   }
-  cudaLaunchConfig_t cfg;
-  cudaLaunchAttribute at[2];
-  power_sync_config(q, comps, q, smem, nullptr, cfg, at);
-  cfg.attrs = at + 1;
-  cfg.numAttrs = 1;
-  e = cudaOccupancyMaxActiveClusters(&n, fn, &cfg);
+  SplitLaunch L;
+  power_sync_config(q, comps, q, smem, nullptr, L);
+  e = cudaOccupancyMaxActiveClusters(&n, fn, &L.cfg);
   *ctas = n * q;
   return e;
 }
 cudaError_t launch_power_sync(const SyncArgs &args, int fp32, int comps, int grid, int smem,
                               cudaStream_t stream) {
-  cudaLaunchConfig_t cfg;
-  cudaLaunchAttribute at[2];
-  power_sync_config(args.q, comps, grid, smem, stream, cfg, at);
+  SplitLaunch L;
+  power_sync_config(args.q, comps, grid, smem, stream, L);
   void *params[] = {(void *)&args};
-  return cudaLaunchKernelExC(&cfg, power_sync_fn(args.q, fp32, comps, smem), params);
+  return cudaLaunchKernelExC(&L.cfg, power_sync_fn(args.q, fp32, comps, smem), params);
 }
 cudaError_t power_max_blocks_per_sm(int variant, int *n) {
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, power_kernel_fn(variant),

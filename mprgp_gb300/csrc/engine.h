@@ -155,6 +155,7 @@ constexpr int kPowerUnroll = 8;  // power launches per evaluation of the loop co
 constexpr int kPowOwn = 4;       // items per CTA of the persistent power loop
 constexpr int kEngOwn = 16;      // ... and of the waiting engine
 constexpr int kCodeInvalid = -5;  // MPRGP_INVALID: the result code of an invalid instance
+constexpr int kCodeLaunch = -6;   // MPRGP_CUDA_ERROR: a kernel saw another launch shape than its own
 
 // Small instances run on the cluster solver: one thread-block cluster per
 // instance, CTA r covering items r, r + cluster, ... (at most kClusterItems
@@ -182,6 +183,7 @@ struct SyncArgs {
   InstState *states;
   const SyncItem *items;
   int units, q;  // q: CTAs of a unit
+  int ninst, pad;
   long long wait_ns;
   Ctl *ctl;
 };
@@ -190,7 +192,7 @@ struct EngineSyncArgs {
   const InstDesc *desc;
   InstState *states;
   const SyncItem *items;  // limit unused
-  int units, q, max_phases, pad;
+  int units, q, max_phases, ninst;
   long long wait_ns, total_ns;
   Ctl *ctl;
 };

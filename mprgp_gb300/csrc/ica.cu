@@ -444,6 +444,12 @@ __global__ void __launch_bounds__(kCThreads) ica_cluster_kernel(IcaClusterArgs C
   __shared__ double s_tot;
   const IcaArgs &a = C.a;
   const int rank = (int)blockIdx.x, ncta = (int)gridDim.x;  // one cluster
+  unsigned int csize;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(csize));
+  if ((int)csize != ncta) {  // not the launch's shape: no peer to write to
+    if (threadIdx.x == 0) atomicCAS(&a.ctl->err, 0, 2);
+    return;
+  }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int sub = lane / 3, comp = lane - 3 * sub, lead = 3 * sub;  // block row of the warp
   const bool on = lane < 3 * kCRows;
@@ -867,6 +873,7 @@ int mprgp_ica_solve(mprgp_context *ctx, int nv, int nnzb, const int *row_ptr, co
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
   if (e != cudaSuccess) rc = fail(MPRGP_CUDA_ERROR, "ica_solve: CUDA call failed");
+  else if (ctl.err == 2) rc = fail(MPRGP_CUDA_ERROR, "ica_solve: launched with another cluster size");
   else if (ctl.err) rc = fail(MPRGP_TIMEOUT, "ica_solve: device wait limit reached");
   cudaFreeAsync(d, s);
   cudaStreamSynchronize(s);
