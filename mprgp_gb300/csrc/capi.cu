@@ -24,6 +24,7 @@
 #include "coop_gate.h"
 #include "engine.h"
 #include "nvtx_ranges.h"
+#include "run_plan.h"
 
 namespace mprgp {
 cudaError_t launch_engine(const EngineArgs &args, int grid, cudaStream_t stream);
@@ -645,6 +646,7 @@ int lane_init(mprgp_context *c, int k) {
 
 void lane_free(mprgp_context *c, Lane &L) {
   if (!L.ready) return;
+  lane_taken(coop_gate(c->device), L.e_end);
   if (L.stream) cudaStreamSynchronize(L.stream);
   for (int q = 0; q < kClusterClasses; ++q)
     if (L.side[q]) cudaStreamSynchronize(L.side[q]);
@@ -752,127 +754,33 @@ int lane_reserve_units(mprgp_context *c, Lane &L, int units) {
   return MPRGP_OK;
 }
 
-// How a synchronous run's power method is laid onto the GPU by the power sync
-// loop: q CTAs an item with their matrix slices in shared memory (smem bytes a
-// CTA), or (q == 0) the persistent loop, several items a CTA; grid == 0 when
-// neither applies.
-struct SyncPlan {
-  int q = 0, comps = 1, smem = 0, grid = 0, groups = 1;
+// CTAs of the waiting kernels' forms that the device holds at once, asked for
+// once a form (run_plan.h).
+struct Capacity {
+  mprgp_context *c;
+  template <typename F>
+  int cached(const std::tuple<int, int, int> &key, F query) const {
+    auto it = c->sync_cap.find(key);
+    if (it == c->sync_cap.end()) {
+      int n = 0;
+      if (query(&n) != cudaSuccess) {
+        cudaGetLastError();
+        n = 0;
+      }
+      it = c->sync_cap.emplace(key, n).first;
+    }
+    return it->second;
+  }
+  int power(int q, int fp32, int comps, int smem) const {
+    return cached(std::make_tuple(q, 4 * fp32 + comps, smem), [&](int *n) {
+      return power_sync_capacity(q, fp32, comps, smem, c->nsm, n);
+    });
+  }
+  int engine(int q, int smem) const {
+    return cached(std::make_tuple(q, -1, smem),
+                  [&](int *n) { return engine_sync_capacity(q, smem, c->nsm, n); });
+  }
 };
-int sync_capacity(mprgp_context *c, int q, int fp32, int comps, int smem) {
-  const auto key = std::make_tuple(q, 4 * fp32 + comps, smem);
-  auto it = c->sync_cap.find(key);
-  if (it == c->sync_cap.end()) {
-    int n = 0;
-    if (power_sync_capacity(q, fp32, comps, smem, c->nsm, &n) != cudaSuccess) {
-      cudaGetLastError();
-      n = 0;
-    }
-    it = c->sync_cap.emplace(key, n).first;
-  }
-  return it->second;
-}
-SyncPlan sync_plan(mprgp_context *c, int units, int max_slots, int fp32) {
-  SyncPlan P;
-  const int slice = max_slots * kSlice * (9 * (fp32 ? 4 : 8) + 4);
-  auto bytes = [&](int q) {  // a CTA's slices, in few distinct sizes
-    return ((long long)slice * (kThreads / kSlice / q) + 4095) / 4096 * 4096;
-  };
-  auto fits = [&](int q, int comps) {
-    if (bytes(q) > kSyncStageBytes || units * q > sync_capacity(c, q, fp32, comps, (int)bytes(q)))
-      return false;
-    P.q = q;
-    P.comps = comps;
-    P.smem = (int)bytes(q);
-    P.grid = units * q;
-    return true;
-  };
-  // FP64 rows by three threads, one a component, while each scheduler of an SM
-  // gets one or two such warps: a row's 135 FP64 FMAs (15 blocks) take 6 us as
-  // one warp's chain, a component's 45 take 2.
-  // 425 vertices: 10.7 -> 7.7 us a phase, 6,720: 12.3 -> 9.3.  (Three quarters
-  // of the SMs: clusters do not pack them further, and two CTAs on an SM cost
-  // what the split gains: 9,464 vertices 13.2 us, 12.6 with whole rows.)
-  if (!fp32)
-    for (int q = 8; q >= 4; q /= 2)
-      if (4 * units * q <= 3 * c->nsm && fits(q, 3)) return P;
-  // Else the fewest CTAs an item whose slices fit shared memory, or twice as
-  // many (smaller CTAs can pack an SM better).  1,760 vertices mixed: 4.85 us
-  // a phase with q = 1, 5.5 with 2, 4 or 8; 17,856 in FP64: 11.5 with q = 2,
-  // 14.2 with 4, 18.3 with 8.
-  int tried = 0;
-  for (int q = 1; q <= kThreads / kSlice && tried < 2; q *= 2) {
-    if (bytes(q) > kSyncStageBytes) continue;
-    ++tried;
-    if (fits(q, 1)) break;
-  }
-  return P;
-}
-SyncPlan persistent_plan(mprgp_context *c, int units) {
-  SyncPlan P;
-  const int cap = c->nsm * c->bps_power_pp;
-  // Up to two items a CTA, unless the tuning asks for the persistent loop:
-  // a phase takes 15.8 us against 23.2 as graph launches at 549 items, 29.9
-  // against 31.1 at 833 (two a CTA), but 52.4 against 51.0 at 1,360 (three a
-  // CTA, streaming from DRAM, which more CTAs hide better).
-  if (cap > 0 && units <= cap * (c->power_persistent ? kPowOwn : 2)) {
-    const int per = (units + cap - 1) / cap;  // equally many items a CTA
-    P.grid = (units + per - 1) / per;
-  }
-  return P;
-}
-
-int engine_capacity(mprgp_context *c, int q, int smem) {
-  const auto key = std::make_tuple(q, -1, smem);
-  auto it = c->sync_cap.find(key);
-  if (it == c->sync_cap.end()) {
-    int n = 0;
-    if (engine_sync_capacity(q, smem, c->nsm, &n) != cudaSuccess) {
-      cudaGetLastError();
-      n = 0;
-    }
-    it = c->sync_cap.emplace(key, n).first;
-  }
-  return it->second;
-}
-// The waiting engine's layout; grid == 0 when it does not apply.
-SyncPlan engine_plan(mprgp_context *c, int units, int max_slots, bool fp64, bool beside) {
-  SyncPlan P;
-  // FP64 items: eight or four CTAs of three threads a row, with their matrix
-  // slices in shared memory, while three quarters of the SMs hold them (the
-  // rule of sync_plan); else two CTAs while each has an SM of its own: an
-  // item's eight row warps take 135 FP64 FMAs each, two warps a scheduler in
-  // one CTA (17,856 vertices 16.6 -> 16.1 ms with two).
-  if (fp64)
-    for (int q = 8; q >= 4; q /= 2) {
-      const long long bytes = (long long)max_slots * kSlice * (9 * 8 + 4) * (kThreads / kSlice / q);
-      const long long smem = (bytes + 4095) / 4096 * 4096;
-      if (4 * units * q > 3 * c->nsm || smem > kEngStageBytes ||
-          units * q > engine_capacity(c, q, (int)smem))
-        continue;
-      P.q = q;
-      P.smem = (int)smem;
-      P.grid = q * units;
-      return P;
-    }
-  if (fp64 && 2 * units <= std::min(c->nsm, engine_capacity(c, 2, 0))) {
-    P.q = 2;
-    P.grid = 2 * units;
-    return P;
-  }
-  // One CTA an SM with equally many items, in as few rounds as four groups
-  // give; beside cluster solves, smaller CTAs of one group, which find room as
-  // those finish (a batch of 48 takes 25.6 ms so, 28.8 with one CTA an SM).
-  const int ctas = std::min(c->nsm, engine_capacity(c, 1, 0)) * (beside ? 4 : 1);
-  const int per = ctas > 0 ? (units + ctas - 1) / ctas : kEngOwn + 1;
-  if (per <= kEngOwn) {
-    const int rounds = beside ? per : (per + 3) / 4;
-    P.q = 1;
-    P.groups = (per + rounds - 1) / rounds;
-    P.grid = (units + per - 1) / per;
-  }
-  return P;
-}
 
 bool other_lanes_active(const mprgp_context *c, int k) {
   for (int j = 0; j < kLanes; ++j)
@@ -1056,99 +964,63 @@ int engine_begin(mprgp_context *c, int k, int n, mprgp_problem *const *probs,
   unsigned int in_power = 0;  // large instances in a power phase
   for (int i = 0; i < n; ++i)
     if (R.pos[i] < n_large && engine_in_power(probs[i])) ++in_power;
-  // The power method in the forms whose CTAs wait for each other (unless the
-  // tuning asks for the launch loops): a synchronous run's instances, small
-  // ones too, by the power sync loop when all their CTAs are resident at once;
-  // else its large ones by the persistent loop and its small ones by the same
-  // kernel with one cluster an instance.  A server's asynchronous lanes keep
-  // the launch loops and the cluster solver: kernels that wait for their peers
-  // stay out of runs that share the SMs with other streams.
-  const bool waiting = k == 0 && power_launches > 0 && c->power_kernel && c->power_graph && c->power_step;
-  const bool alone = k == 0 && !other_lanes_active(c, k);
-  struct Count {
-    int units = 0, slots = 0, fp32 = 0, n = 0;
-    void add(const mprgp_problem *p, const InstDesc &D) {
-      units += nitems_of(p->nv);
-      slots = std::max(slots, p->max_len);
-      fp32 += D.prec == PREC_MIXED ? 1 : 0;
-      ++n;
-    }
-    bool one() const { return n > 0 && (fp32 == 0 || fp32 == n); }  // of one precision
-  } all, large, cl[kClusterClasses];
-  bool cl_fits[kClusterClasses] = {true, true, true, true, true};
-  for (int i = 0; i < n && waiting; ++i) {
-    if (!engine_in_power(probs[i])) continue;
-    const InstDesc &D = desc[R.pos[i]];
-    if (R.pos[i] < n_large) {
-      all.add(probs[i], D);
-      large.add(probs[i], D);
-    } else if (cluster_quantum == 0) {
-      all.add(probs[i], D);
-      cl[cls[i]].add(probs[i], D);
-      cl_fits[cls[i]] &= D.nitems <= (1 << cls[i]);
-    }
-  }
-  SyncPlan plan;
-  bool small_in_plan = false;
-  if (alone && all.one()) {
-    plan = sync_plan(c, all.units, all.slots, all.fp32 ? 1 : 0);
-    small_in_plan = plan.grid > 0;
-  }
-  if (alone && large.one() && plan.grid == 0) plan = persistent_plan(c, large.units);
-  R.power_sync = plan.grid > 0;
-  const Count &sync = small_in_plan ? all : large;
-  // The instances' other phases: the waiting engine for the large ones of a
-  // synchronous run, and for small ones too when they are FP64 and few enough
-  // for split units (425 vertices: 14.2 -> 13.8 ms).
-  Count eng;
-  for (int i = 0; i < n; ++i) eng.add(probs[i], desc[R.pos[i]]);
-  const bool eng_on = alone && quantum >= 0 && !c->engine_graph && !c->stage && c->power_kernel &&
-                      c->ctas_per_sm == 0;
-  SyncPlan eplan;
-  if (eng_on && n_large == 0 && quantum == 0 && cluster_quantum == 0 && eng.fp32 == 0 &&
-      (all.n == 0 || small_in_plan))
-    eplan = engine_plan(c, eng.units, eng.slots, true, false);
-  if (eplan.q < 2) eplan = SyncPlan();
-  R.engine_small = eplan.grid > 0;
-  if (eng_on && n_large > 0) {
-    eng = Count();
-    for (int i = 0; i < n; ++i)
-      if (R.pos[i] < n_large) eng.add(probs[i], desc[R.pos[i]]);
-    eplan = engine_plan(c, eng.units, eng.slots, eng.fp32 == 0, n > n_large);
-  }
-  R.engine_sync = eplan.grid > 0;
+  // A synchronous run's kernels may wait for their peers while no lane of any
+  // context has a run in flight; the gate is held until they are issued, so that
+  // none begins meanwhile.  A lane's run begins behind those issued before it.
+  CoopGate &gate = coop_gate(c->device);
+  LaneStart lane_start(gate, k != 0);
+  std::unique_lock<std::mutex> hold(gate.m);
+  if (k != 0) CK(gate.behind_last(L.stream));
+  PlanSettings ps;
+  ps.nsm = c->nsm;
+  ps.alone = k == 0 && !other_lanes_active(c, k) && gate.lanes_idle();
+  ps.quantum = quantum;
+  ps.power_launches = power_launches;
+  ps.cluster_quantum = cluster_quantum;
+  ps.power_waits = c->power_kernel && c->power_graph && c->power_step;
+  ps.engine_waits = !c->engine_graph && !c->stage && c->power_kernel && c->ctas_per_sm == 0;
+  ps.persistent4 = c->power_persistent != 0;
+  ps.persistent_per_sm = c->bps_power_pp;
+  for (int q = 0; q < kClusterClasses; ++q) ps.power_cluster_ok[q] = c->power_cluster_ok[q] != 0;
+  std::vector<PlanInst> insts(n);
+  for (int i = 0; i < n; ++i)
+    insts[i] = {R.pos[i] < n_large, cls[i], nitems_of(probs[i]->nv), probs[i]->max_len,
+                desc[R.pos[i]].prec == PREC_MIXED, engine_in_power(probs[i]) != 0};
+  const RunPlan plan = plan_run(insts, ps, Capacity{c});
+  if (!ps.alone) hold.unlock();
+  R.power_sync = plan.power_sync;
+  R.engine_sync = plan.engine_sync;
+  R.engine_small = plan.engine_small;
   int nunits = 0, class_unit[kClusterClasses], engine_unit = 0;
   {
-    int want = R.power_sync ? sync.units : 0;
+    int want = R.power_sync ? plan.power_count.units : 0;
     for (int q = 0; q < kClusterClasses; ++q) {
-      R.class_units[q] = (!small_in_plan && cl[q].one() && cl_fits[q] && c->power_cluster_ok[q])
-                             ? cl[q].n << q
-                             : 0;
+      R.class_units[q] = plan.class_units[q];
       want += R.class_units[q];
     }
-    want += eplan.grid > 0 ? eng.units : 0;
+    want += plan.engine.grid > 0 ? plan.engine_count.units : 0;
     rc = lane_reserve_units(c, L, want);
     if (rc) return rc;
     if (R.power_sync)
       for (int i = 0; i < n; ++i) {
-        if (!engine_in_power(probs[i]) || !(R.pos[i] < n_large || small_in_plan)) continue;
-        const int limit = R.pos[i] < n_large ? power_launches : INT_MAX;
-        for (int t = 0; t < nitems_of(probs[i]->nv); ++t) L.h_unit[nunits++] = {R.pos[i], t, limit, 0};
+        if (!insts[i].in_power || !(insts[i].large || plan.small_in_plan)) continue;
+        const int limit = insts[i].large ? power_launches : INT_MAX;
+        for (int t = 0; t < insts[i].items; ++t) L.h_unit[nunits++] = {R.pos[i], t, limit, 0};
       }
     for (int q = 0; q < kClusterClasses; ++q) {
       class_unit[q] = nunits;
       if (!R.class_units[q]) continue;
       for (int i = 0; i < n; ++i) {
-        if (cls[i] != q || !engine_in_power(probs[i])) continue;
-        const int ni = nitems_of(probs[i]->nv);
-        for (int t = 0; t < (1 << q); ++t) L.h_unit[nunits++] = {R.pos[i], t, t < ni ? INT_MAX : 0, 0};
+        if (cls[i] != q || !insts[i].in_power) continue;
+        for (int t = 0; t < (1 << q); ++t)
+          L.h_unit[nunits++] = {R.pos[i], t, t < insts[i].items ? INT_MAX : 0, 0};
       }
     }
     engine_unit = nunits;
     if (R.engine_sync)
       for (int i = 0; i < n; ++i)
-        if (R.pos[i] < n_large || R.engine_small)
-          for (int t = 0; t < nitems_of(probs[i]->nv); ++t) L.h_unit[nunits++] = {R.pos[i], t, 0, 0};
+        if (insts[i].large || R.engine_small)
+          for (int t = 0; t < insts[i].items; ++t) L.h_unit[nunits++] = {R.pos[i], t, 0, 0};
   }
   cudaStream_t s = L.stream;
   if (s != c->stream) {  // the problems' uploads and setup kernels come first
@@ -1222,7 +1094,7 @@ int engine_begin(mprgp_context *c, int k, int n, mprgp_problem *const *probs,
   // latter while another lane has a run in flight, since a cooperative launch
   // needs every one of its CTAs resident at once.
   R.egraph = n_large > 0 && quantum >= 0 &&
-             (c->engine_graph || k != 0 || other_lanes_active(c, k));
+             (c->engine_graph || k != 0 || !ps.alone);
   cudaGraphExec_t eexec = nullptr;
   const int egrid = power_grid(c, prefix[n_large], 2);
   // Stream form of that loop (with the power loop's stream form, for
@@ -1249,22 +1121,23 @@ int engine_begin(mprgp_context *c, int k, int n, mprgp_problem *const *probs,
   sa.ctl = L.ctl;
   // The cluster-size classes run on side streams, concurrently with each
   // other and with the power loop; the engine starts once they are done.
-  if (n - n_large > 0 && !small_in_plan) CK(cudaEventRecord(L.fork_ev, s));
+  if (n - n_large > 0 && !plan.small_in_plan) CK(cudaEventRecord(L.fork_ev, s));
   if (R.power_sync) {
     sa.items = L.d_unit;
-    sa.units = sync.units;
-    sa.q = std::max(1, plan.q);
-    const int fp32 = sync.fp32 ? 1 : 0;
+    sa.units = plan.power_count.units;
+    sa.q = std::max(1, plan.power.q);
+    const int fp32 = plan.power_count.fp32 ? 1 : 0;
     // (beside other kernels the persistent loop leaves them registers)
-    const bool no_clusters = n == n_large || small_in_plan;
-    const int per_sm = no_clusters ? (plan.grid + c->nsm - 1) / c->nsm : c->bps_power_pp;
-    CK(gated_launch(s, [&] {
-      return plan.q > 0 ? launch_power_sync(sa, fp32, plan.comps, plan.grid, plan.smem, s)
-                        : launch_power_persistent(sa, fp32, per_sm, plan.grid, s);
+    const bool no_clusters = n == n_large || plan.small_in_plan;
+    const SyncPlan &pp = plan.power;
+    const int per_sm = no_clusters ? (pp.grid + c->nsm - 1) / c->nsm : c->bps_power_pp;
+    CK(gate.launch(s, [&] {
+      return pp.q > 0 ? launch_power_sync(sa, fp32, pp.comps, pp.grid, pp.smem, s)
+                      : launch_power_persistent(sa, fp32, per_sm, pp.grid, s);
     }));
     CK(cudaEventRecord(L.e_pow, s));
   }
-  if (n - n_large > 0 && small_in_plan) CK(cudaEventRecord(L.fork_ev, s));
+  if (n - n_large > 0 && plan.small_in_plan) CK(cudaEventRecord(L.fork_ev, s));
   for (int q = 0; q < kClusterClasses; ++q) {
     if (!R.class_n[q]) continue;
     if (R.engine_small) continue;
@@ -1279,7 +1152,7 @@ int engine_begin(mprgp_context *c, int k, int n, mprgp_problem *const *probs,
       sa.items = L.d_unit + class_unit[q];
       sa.units = R.class_units[q];
       sa.q = 1;
-      CK(launch_power_clusters(sa, cl[q].fp32 ? 1 : 0, 1 << q, L.side[q]));
+      CK(launch_power_clusters(sa, plan.class_fp32[q] ? 1 : 0, 1 << q, L.side[q]));
     }
     CK(launch_cluster(cargs, 1 << q, L.side[q]));
     CK(cudaEventRecord(L.join_ev[q], L.side[q]));
@@ -1294,23 +1167,31 @@ int engine_begin(mprgp_context *c, int k, int n, mprgp_problem *const *probs,
     ea.desc = L.d_desc;
     ea.states = L.d_st;
     ea.items = L.d_unit + engine_unit;
-    ea.units = eng.units;
-    ea.q = eplan.q;
+    ea.units = plan.engine_count.units;
+    ea.q = plan.engine.q;
     ea.max_phases = args.max_phases;
     ea.ninst = n;
     ea.wait_ns = args.wait_ns;
     ea.total_ns = args.total_ns;
     ea.ctl = L.ctl;
-    CK(gated_launch(s, [&] { return launch_engine_sync(ea, eplan.groups, eplan.grid, eplan.smem, s); }));
+    const SyncPlan &ep = plan.engine;
+    CK(gate.launch(s, [&] { return launch_engine_sync(ea, ep.groups, ep.grid, ep.smem, s); }));
   }
   for (int q = 0; q < kClusterClasses; ++q)
     if (R.class_n[q] && !R.engine_small) CK(cudaStreamWaitEvent(s, L.join_ev[q], 0));
+  for (int q = 0; q < kClusterClasses; ++q)
+    if (R.class_units[q]) {  // their power loops are over by here
+      CK(gate.mark(s));
+      break;
+    }
   if (R.engine_sync) {
     // launched above, beside the cluster classes
   } else if (R.egraph && R.egraph_stream)
     CK(launch_power_direct(egrid, 2, R.egraph_stream, L.d_args, L.d_pc2, s));
   else if (R.egraph) CK(cudaGraphLaunch(eexec, s));
-  else if (n_large > 0 && quantum >= 0) CK(gated_launch(s, [&] { return launch_engine(args, grid, s); }));
+  else if (n_large > 0 && quantum >= 0)
+    CK(gate.launch(s, [&] { return launch_engine(args, grid, s); }));
+  if (hold.owns_lock()) hold.unlock();
   CK(cudaEventRecord(L.e1, s));
   if (R.power) CK(cudaMemcpyAsync(&io.pc_out[0], L.d_pc, sizeof(PowCtl), cudaMemcpyDeviceToHost, s));
   if (R.egraph) CK(cudaMemcpyAsync(&io.pc_out[1], L.d_pc2, sizeof(PowCtl), cudaMemcpyDeviceToHost, s));
@@ -1325,6 +1206,7 @@ int engine_begin(mprgp_context *c, int k, int n, mprgp_problem *const *probs,
   R.cluster_quantum = cluster_quantum;
   R.power_launches = power_launches;
   R.active = true;
+  lane_start.issued(L.e_end);
   static const char *kRunNames[kLanes] = {"mprgp run", "mprgp lane small", "mprgp lane large",
                                           "mprgp lane power", "mprgp lane power",
                                           "mprgp lane power", "mprgp lane power"};
@@ -1363,6 +1245,7 @@ int engine_end(mprgp_context *c, int k, mprgp_stats *stats, int *done) {
   Lane &L = c->lane[k];
   LaneRun &R = L.run;
   R.active = false;
+  if (k != 0) lane_taken(coop_gate(c->device), L.e_end);
   nvtx_end(L.nvtx);
   L.nvtx = 0;
   const int n = R.n, n_large = R.n_large;
