@@ -139,15 +139,16 @@ int mprgp_context_counters(mprgp_context *ctx, long long *launches, double *solv
  * launch whose CTAs are all resident and wait per instance: with the matrix
  * slices in shared memory when they fit the SMs', else reading the matrix in
  * every phase with up to two items a CTA (bit 5 = 1: four), and small
- * instances with one cluster each (on server lanes too).  Other runs take the
- * power-step loop: no launch finalizes its own phase -- every CTA of the next
- * launch reduces the item partials and advances its copy of the state with one
- * extra warp while its rows already form their products, and a settle kernel
- * ends each graph body; bit 6 = 1 runs the phase kernel instead, whose last
- * CTA finalizes each launch (bit 2 applies to both loops; with bits 1, 2 or 6
- * small instances keep their power method in the cluster solver).  ctas_per_sm
- * caps the persistent grid (0 = every resident CTA).  Every setting gives
- * bitwise the same results. */
+ * instances with one cluster each.  Items beyond that, a server's lanes, and a
+ * synchronous run while a lane has one in flight take the power-step loop (small
+ * instances the cluster solver).  In that loop no launch finalizes its own
+ * phase -- every CTA of the next launch reduces the item partials and advances
+ * its copy of the state with one extra warp while its rows already form their
+ * products, and a settle kernel ends each graph body; bit 6 = 1 runs the phase
+ * kernel instead, whose last CTA finalizes each launch (bit 2 applies to both
+ * loops; with bits 1, 2 or 6 small instances keep their power method in the
+ * cluster solver).  ctas_per_sm caps the persistent grid (0 = every resident
+ * CTA).  Every setting gives bitwise the same results. */
 int mprgp_context_set_tuning(mprgp_context *ctx, int stage, int ctas_per_sm);
 /* Small instances -- up to `cluster` items of 256 vertices -- are solved by
  * one thread-block cluster each, one CTA per item (state in shared memory,

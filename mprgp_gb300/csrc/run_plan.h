@@ -167,12 +167,13 @@ template <typename Cap>
 RunPlan plan_run(const std::vector<PlanInst> &insts, const PlanSettings &s, const Cap &cap) {
   RunPlan R;
   const int n = (int)insts.size();
-  int n_large = 0;
+  int n_large = 0, in_power = 0;  // large instances; instances in a power phase
   PlanCount all, large, cl[kClusterClasses];
   bool cl_fits[kClusterClasses] = {true, true, true, true, true};
   const bool waiting = s.alone && s.power_launches > 0 && s.power_waits;
   for (const PlanInst &p : insts) {
     n_large += p.large ? 1 : 0;
+    in_power += p.in_power ? 1 : 0;
     if (!waiting || !p.in_power) continue;
     if (p.large) {
       all.add(p);
@@ -198,15 +199,16 @@ RunPlan plan_run(const std::vector<PlanInst> &insts, const PlanSettings &s, cons
   }
   // The instances' other phases: the waiting engine for the large ones of a
   // synchronous run, and for small ones too when they are FP64 and few enough
-  // for split units (425 vertices: a solve of 13.7 -> 9.0 ms, 4.7 of them by
-  // the power loop's form).
+  // for split units (425 vertices: a solve of 13.7 -> 9.0 ms, most of it by the
+  // power loop's form).  Not when their power method has yet to run and the
+  // tuning keeps it in the cluster solver.
   const bool eng_on = s.alone && s.quantum >= 0 && s.engine_waits;
   if (!eng_on) return R;
   PlanCount eng;
   for (const PlanInst &p : insts)
     if (n_large == 0 || p.large) eng.add(p);
   if (n_large == 0 && s.quantum == 0 && s.cluster_quantum == 0 && eng.fp32 == 0 &&
-      (all.n == 0 || R.small_in_plan)) {
+      (in_power == 0 || R.small_in_plan)) {
     R.engine = engine_plan(cap, s.nsm, eng.units, eng.slots, true, false);
     if (R.engine.q < 2) R.engine = SyncPlan();
     R.engine_small = R.engine.grid > 0;

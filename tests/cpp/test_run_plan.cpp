@@ -74,6 +74,14 @@ int main() {
   EXPECT(R.power_sync && !R.small_in_plan && R.power_count.n == 1);
   EXPECT(R.class_units[1] == 2 && R.class_units[3] == 8 && R.class_n[1] == 1 && R.class_fp32[1]);
   EXPECT(R.engine_sync && R.engine_count.n == 1);
+  // a tuning with the launch loops keeps a small FP64 instance's power method in
+  // the cluster solver; past it, the waiting engine takes it as before
+  PlanSettings loops = settings(true);
+  loops.power_waits = false;
+  EXPECT(!waits(plan_run({inst(2, false)}, loops, Cap())));
+  EXPECT(!waits(plan_run({inst(2, false), inst(3, false, false)}, loops, Cap())));
+  R = plan_run({inst(2, false, false)}, loops, Cap());
+  EXPECT(R.engine_small && !R.power_sync);
   // unit counts and grids agree
   for (const auto &r : runs) {
     R = plan_run(r, settings(true), Cap());

@@ -65,3 +65,17 @@ def test_small_solves_beside_lanes(precision):
     assert n == 4 and all(np.array_equal(a, b) for a, b in zip(ref, out))
     other.close()
     own.close()
+
+
+@pytest.mark.parametrize("precision", [M.PREC_FP64, M.PREC_MIXED])
+def test_launch_loop_tuning_keeps_the_cluster_solver(precision):
+    qps = [body((4, 4, 16), 1), body((5, 4, 14), 2)]
+    ctx = M.Context(0)
+    ref, n = solve(ctx, qps, precision)
+    assert n == 4
+    for bits in (2, 4, 64):
+        ctx.set_tuning(bits, 0)
+        out, n = solve(ctx, qps, precision)
+        assert n == 3  # one cluster class, the states in and out
+        assert all(np.array_equal(a, b) for a, b in zip(ref, out))
+    ctx.close()
