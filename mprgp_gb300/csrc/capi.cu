@@ -89,10 +89,11 @@ struct LaneRun {
   std::vector<mprgp_problem *> probs;
   std::vector<mprgp_options> opts;
   std::vector<int> pos;
+  std::vector<int> err_word;  // of the lane's control blocks, by instance (-1: none)
 };
 
 struct HostIO {  // pinned: the run's control blocks in and out
-  Ctl ctl_in, ctl_out;
+  Ctl ctl_in[kErrWords], ctl_out[kErrWords];
   PowCtl pc_in[2], pc_out[2];  // power loop, engine loop
   EngineArgs args;
 };
@@ -633,12 +634,12 @@ int lane_init(mprgp_context *c, int k) {
   CK(cudaEventCreate(&L.e_pow));
   CK(cudaMallocHost((void **)&L.io, sizeof(HostIO)));
   std::memset(L.io, 0, sizeof(HostIO));
-  int rc = dalloc(c, &L.ctl, 1);
+  int rc = dalloc(c, &L.ctl, kErrWords);
   if (!rc) rc = dalloc(c, &L.d_args, 1);
   if (!rc) rc = dalloc(c, &L.d_pc, 1);
   if (!rc) rc = dalloc(c, &L.d_pc2, 1);
   if (rc) return rc;
-  CK(cudaMemsetAsync(L.ctl, 0, sizeof(Ctl), c->stream));
+  CK(cudaMemsetAsync(L.ctl, 0, sizeof(Ctl) * kErrWords, c->stream));
   CK(cudaStreamSynchronize(c->stream));
   L.ready = true;
   return MPRGP_OK;
@@ -991,6 +992,8 @@ int engine_begin(mprgp_context *c, int k, int n, mprgp_problem *const *probs,
   R.power_sync = plan.power_sync;
   R.engine_sync = plan.engine_sync;
   R.engine_small = plan.engine_small;
+  R.err_word.resize(n);
+  for (int i = 0; i < n; ++i) R.err_word[i] = error_word(plan, insts[i]);
   int nunits = 0, class_unit[kClusterClasses], engine_unit = 0;
   {
     int want = R.power_sync ? plan.power_count.units : 0;
@@ -1042,10 +1045,10 @@ int engine_begin(mprgp_context *c, int k, int n, mprgp_problem *const *probs,
   launch_state_scatter(L.d_desc, n, L.d_st, L.d_home, L.d_fresh, nunits > 0 ? 1 : 0, s);
   CK(cudaGetLastError());
   HostIO &io = *L.io;
-  std::memset(&io.ctl_in, 0, sizeof(Ctl));
-  io.ctl_in.active = n_large;
-  io.ctl_in.snap[0] = io.ctl_in.snap[1] = n_large;
-  CK(cudaMemcpyAsync(L.ctl, &io.ctl_in, sizeof(Ctl), cudaMemcpyHostToDevice, s));
+  std::memset(io.ctl_in, 0, sizeof(io.ctl_in));
+  io.ctl_in[0].active = n_large;
+  io.ctl_in[0].snap[0] = io.ctl_in[0].snap[1] = n_large;
+  CK(cudaMemcpyAsync(L.ctl, io.ctl_in, sizeof(io.ctl_in), cudaMemcpyHostToDevice, s));
   EngineArgs &args = io.args;
   std::memset(&args, 0, sizeof(args));
   args.desc = L.d_desc;
@@ -1152,6 +1155,7 @@ int engine_begin(mprgp_context *c, int k, int n, mprgp_problem *const *probs,
       sa.items = L.d_unit + class_unit[q];
       sa.units = R.class_units[q];
       sa.q = 1;
+      sa.ctl = L.ctl + 1 + q;
       CK(launch_power_clusters(sa, plan.class_fp32[q] ? 1 : 0, 1 << q, L.side[q]));
     }
     CK(launch_cluster(cargs, 1 << q, L.side[q]));
@@ -1195,7 +1199,7 @@ int engine_begin(mprgp_context *c, int k, int n, mprgp_problem *const *probs,
   CK(cudaEventRecord(L.e1, s));
   if (R.power) CK(cudaMemcpyAsync(&io.pc_out[0], L.d_pc, sizeof(PowCtl), cudaMemcpyDeviceToHost, s));
   if (R.egraph) CK(cudaMemcpyAsync(&io.pc_out[1], L.d_pc2, sizeof(PowCtl), cudaMemcpyDeviceToHost, s));
-  CK(cudaMemcpyAsync(&io.ctl_out, L.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s));
+  CK(cudaMemcpyAsync(io.ctl_out, L.ctl, sizeof(io.ctl_out), cudaMemcpyDeviceToHost, s));
   launch_state_gather(L.d_desc, n, L.d_st, L.d_home, s);
   CK(cudaGetLastError());
   CK(cudaMemcpyAsync(L.h_st_out, L.d_st, sizeof(InstState) * n, cudaMemcpyDeviceToHost, s));
@@ -1277,21 +1281,19 @@ int engine_end(mprgp_context *c, int k, mprgp_stats *stats, int *done) {
     c->launches += ((n_large > 0 && R.quantum >= 0) || R.engine_small) ? 1 : 0;
   c->launches += 2;  // state scatter and gather
   c->solver_ms += ms;
-  const Ctl &ctl1 = io.ctl_out;
   int worst = MPRGP_OK;
-  bool small_power = false;  // small instances' power loops share the error word
-  for (int q = 0; q < kClusterClasses; ++q) small_power |= R.class_units[q] > 0;
   for (int i = 0; i < n; ++i) {
     mprgp_problem *p = R.probs[i];
     InstState x = L.h_st_out[R.pos[i]];
     p->phase_host = x.phase;
     const bool finished = x.phase == PH_DONE;
     const bool large = R.pos[i] < n_large;
-    // an engine error concerns the engine's instances; an instance left
-    // unfinished by a run that had no phase limit hit the hard phase bound
-    const bool err = (large || R.power_sync || R.engine_small || small_power) && ctl1.err;
+    // an error concerns the instances of the launch that reported it; an
+    // instance left unfinished by a run that had no phase limit hit the hard
+    // phase bound
+    const int word = R.err_word[i], err = word < 0 ? 0 : io.ctl_out[word].err;
     const bool unbounded = (large ? R.quantum : R.cluster_quantum) == 0;
-    if (err) x.code = ctl1.err;
+    if (err) x.code = err;
     else if (!finished && unbounded) x.code = MPRGP_TIMEOUT;
     p->xc = x.xc;
     p->trace_n = x.trace_n;
@@ -1320,8 +1322,9 @@ int engine_end(mprgp_context *c, int k, mprgp_stats *stats, int *done) {
     if (done) done[i] = finished || err || (!finished && unbounded);
     if ((finished || err || unbounded) && x.code < worst) worst = x.code;
   }
-  if (ctl1.err)
-    return fail(ctl1.err, ctl1.err == kCodeLaunch ? "a kernel was launched with another shape than its own"
+  for (const Ctl &ctl : io.ctl_out)
+    if (ctl.err)
+      return fail(ctl.err, ctl.err == kCodeLaunch ? "a kernel was launched with another shape than its own"
                                                   : "device wait limit reached");
   return worst < MPRGP_NOT_CONVERGED ? worst : MPRGP_OK;
 }

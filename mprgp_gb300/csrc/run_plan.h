@@ -220,4 +220,16 @@ RunPlan plan_run(const std::vector<PlanInst> &insts, const PlanSettings &s, cons
   return R;
 }
 
+// A run's error words: 0 for its waiting launches over the large instances (and
+// whatever joins them), 1 + q for the power loops of cluster class q.  The word
+// of the launch that an instance took part in, or -1: no launch that can give up
+// concerns it, and its result stands whatever becomes of the others.
+constexpr int kErrWords = 1 + kClusterClasses;
+inline int error_word(const RunPlan &R, const PlanInst &p) {
+  if (p.large || R.engine_small) return 0;
+  if (!p.in_power) return -1;
+  if (R.power_sync && R.small_in_plan) return 0;
+  return R.class_units[p.cls] > 0 ? 1 + p.cls : -1;
+}
+
 }  // namespace mprgp

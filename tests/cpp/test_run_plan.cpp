@@ -82,6 +82,28 @@ int main() {
   EXPECT(!waits(plan_run({inst(2, false), inst(3, false, false)}, loops, Cap())));
   R = plan_run({inst(2, false, false)}, loops, Cap());
   EXPECT(R.engine_small && !R.power_sync);
+  // an error concerns the instances of the launch that reports it
+  {
+    const std::vector<PlanInst> r = {inst(900, true), inst(2, true), inst(5, true),
+                                     inst(2, true, false)};
+    R = plan_run(r, settings(true), Cap());
+    EXPECT(R.power_sync && !R.small_in_plan && R.class_units[1] && R.class_units[3]);
+    EXPECT(error_word(R, r[0]) == 0);
+    EXPECT(error_word(R, r[1]) == 2 && error_word(R, r[2]) == 4);
+    EXPECT(error_word(R, r[3]) == -1);  // past its power method: the cluster solver alone
+    const std::vector<PlanInst> t = {inst(198, true), inst(2, true, false), inst(2, false, false)};
+    R = plan_run(t, settings(true), Cap());
+    EXPECT(R.power_sync && error_word(R, t[0]) == 0);
+    EXPECT(error_word(R, t[1]) == -1 && error_word(R, t[2]) == -1);
+    const std::vector<PlanInst> u = {inst(20, true), inst(3, true), inst(3, true, false)};
+    R = plan_run(u, settings(true), Cap());
+    EXPECT(R.small_in_plan && error_word(R, u[1]) == 0 && error_word(R, u[2]) == -1);
+    const std::vector<PlanInst> w = {inst(2, false), inst(3, false, false)};
+    R = plan_run(w, settings(true), Cap());
+    EXPECT(R.engine_small && error_word(R, w[0]) == 0 && error_word(R, w[1]) == 0);
+    R = plan_run(w, settings(false), Cap());
+    EXPECT(error_word(R, w[0]) == -1 && error_word(R, w[1]) == -1);
+  }
   // unit counts and grids agree
   for (const auto &r : runs) {
     R = plan_run(r, settings(true), Cap());
