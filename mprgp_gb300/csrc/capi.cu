@@ -1249,11 +1249,12 @@ int engine_end(mprgp_context *c, int k, mprgp_stats *stats, int *done) {
   Lane &L = c->lane[k];
   LaneRun &R = L.run;
   R.active = false;
-  if (k != 0) lane_taken(coop_gate(c->device), L.e_end);
   nvtx_end(L.nvtx);
   L.nvtx = 0;
   const int n = R.n, n_large = R.n_large;
-  CK(cudaEventSynchronize(L.e_end));
+  const cudaError_t ended = cudaEventSynchronize(L.e_end);
+  if (k != 0) lane_taken(coop_gate(c->device), L.e_end);
+  if (ended != cudaSuccess) return cuda_fail(ended, "cudaEventSynchronize(L.e_end)");
   const HostIO &io = *L.io;
   float ms = 0.f, pms = 0.f;
   CK(cudaEventElapsedTime(&ms, L.e0, L.e1));
