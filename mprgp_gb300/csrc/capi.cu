@@ -965,16 +965,17 @@ int engine_begin(mprgp_context *c, int k, int n, mprgp_problem *const *probs,
   unsigned int in_power = 0;  // large instances in a power phase
   for (int i = 0; i < n; ++i)
     if (R.pos[i] < n_large && engine_in_power(probs[i])) ++in_power;
-  // A synchronous run's kernels may wait for their peers while no lane of any
-  // context has a run in flight; the gate is held until they are issued, so that
-  // none begins meanwhile.  A lane's run begins behind those issued before it.
+  // A synchronous run's kernels may wait for their peers when the gate lets them
+  // in (coop_gate.h); it is held until they are issued.  A lane's run, and a
+  // synchronous one with launch loops in their place, begins behind those issued
+  // before it.
   CoopGate &gate = coop_gate(c->device);
-  LaneStart lane_start(gate, k != 0);
+  LoopRun loop_run(gate);
   std::unique_lock<std::mutex> hold(gate.m);
-  if (k != 0) CK(gate.behind_last(L.stream));
+  const bool loops = gate.loops_in_flight();
   PlanSettings ps;
   ps.nsm = c->nsm;
-  ps.alone = k == 0 && !other_lanes_active(c, k) && gate.lanes_idle();
+  ps.alone = k == 0 && !other_lanes_active(c, k) && !loops;
   ps.quantum = quantum;
   ps.power_launches = power_launches;
   ps.cluster_quantum = cluster_quantum;
@@ -987,8 +988,40 @@ int engine_begin(mprgp_context *c, int k, int n, mprgp_problem *const *probs,
   for (int i = 0; i < n; ++i)
     insts[i] = {R.pos[i] < n_large, cls[i], nitems_of(probs[i]->nv), probs[i]->max_len,
                 desc[R.pos[i]].prec == PREC_MIXED, engine_in_power(probs[i]) != 0};
-  const RunPlan plan = plan_run(insts, ps, Capacity{c});
-  if (!ps.alone) hold.unlock();
+  // What the run waits for its peers in: its own forms, or whole items without
+  // clusters.  (The large instances' phases without the waiting engine: the
+  // cooperative engine, which waits too, or a graph loop; a power method in launch
+  // loops beside it leaves no room for another's run.)
+  RunPlan plan;
+  bool engine_coop = false, waits = false;
+  GateNeed need = {0, false};
+  auto lay_out = [&](bool alone, bool compact) {
+    ps.alone = alone;
+    ps.compact = compact;
+    plan = plan_run(insts, ps, Capacity{c});
+    engine_coop = n_large > 0 && quantum >= 0 && !c->engine_graph && alone && !plan.engine_sync;
+    waits = plan.power_sync || plan.engine_sync || engine_coop;
+    const bool power_loop = c->power_kernel && in_power > 0 && power_launches > 0 && !plan.power_sync;
+    need.sms = engine_coop || power_loop ? c->nsm : std::min(c->nsm, plan_ctas(plan));
+    need.clusters = plan.power.q > 1 || plan.engine.q > 1;
+  };
+  lay_out(ps.alone, false);
+  if (waits) {
+    // (small instances have the cluster solver and wait for no other run)
+    int behind = gate_entry(gate.waiting, c->nsm, need, 0);
+    if (behind < 0 && n_large > 0) {
+      lay_out(true, true);
+      behind = waits ? gate_entry(gate.waiting, c->nsm, need, (int)gate.waiting.size()) : 0;
+    }
+    if (behind < 0) lay_out(false, false);
+    else CK(gate.behind(L.stream, (size_t)behind));
+  }
+  const bool class_waits = std::any_of(plan.class_units, plan.class_units + kClusterClasses,
+                                       [](int u) { return u > 0; });
+  if (!waits) {  // launch loops, or small instances alone
+    if (k != 0 || n_large > 0) CK(loop_run.begin(L.stream));
+    if (!class_waits) hold.unlock();
+  }
   R.power_sync = plan.power_sync;
   R.engine_sync = plan.engine_sync;
   R.engine_small = plan.engine_small;
@@ -1092,12 +1125,10 @@ int engine_begin(mprgp_context *c, int k, int n, mprgp_problem *const *probs,
     CK(cudaMemcpyAsync(L.d_pc, &io.pc_in[0], sizeof(PowCtl), cudaMemcpyHostToDevice, s));
   }
   R.power_graph = pexec != nullptr;
-  // The large instances' remaining phases: the persistent cooperative engine,
-  // or the same phases as a graph loop of the all-phase kernel -- always the
-  // latter while another lane has a run in flight, since a cooperative launch
-  // needs every one of its CTAs resident at once.
-  R.egraph = n_large > 0 && quantum >= 0 &&
-             (c->engine_graph || k != 0 || !ps.alone);
+  // The large instances' remaining phases: the waiting engine, the persistent
+  // cooperative engine, or the same phases as a graph loop of the all-phase
+  // kernel -- always the latter in a run that may not wait.
+  R.egraph = n_large > 0 && quantum >= 0 && (c->engine_graph || !ps.alone);
   cudaGraphExec_t eexec = nullptr;
   const int egrid = power_grid(c, prefix[n_large], 2);
   // Stream form of that loop (with the power loop's stream form, for
@@ -1134,10 +1165,10 @@ int engine_begin(mprgp_context *c, int k, int n, mprgp_problem *const *probs,
     const bool no_clusters = n == n_large || plan.small_in_plan;
     const SyncPlan &pp = plan.power;
     const int per_sm = no_clusters ? (pp.grid + c->nsm - 1) / c->nsm : c->bps_power_pp;
-    CK(gate.launch(s, [&] {
-      return pp.q > 0 ? launch_power_sync(sa, fp32, pp.comps, pp.grid, pp.smem, s)
-                      : launch_power_persistent(sa, fp32, per_sm, pp.grid, s);
-    }));
+    CK(pp.q > 0 ? launch_power_sync(sa, fp32, pp.comps, pp.grid, pp.smem, s)
+                : launch_power_persistent(sa, fp32, per_sm, pp.grid, s));
+    // (small instances go on in the cluster solver)
+    if (!R.engine_sync && !engine_coop && !class_waits) CK(gate.entered(s, need));
     CK(cudaEventRecord(L.e_pow, s));
   }
   if (n - n_large > 0 && plan.small_in_plan) CK(cudaEventRecord(L.fork_ev, s));
@@ -1179,22 +1210,18 @@ int engine_begin(mprgp_context *c, int k, int n, mprgp_problem *const *probs,
     ea.total_ns = args.total_ns;
     ea.ctl = L.ctl;
     const SyncPlan &ep = plan.engine;
-    CK(gate.launch(s, [&] { return launch_engine_sync(ea, ep.groups, ep.grid, ep.smem, s); }));
+    CK(launch_engine_sync(ea, ep.groups, ep.grid, ep.smem, s));
   }
   for (int q = 0; q < kClusterClasses; ++q)
     if (R.class_n[q] && !R.engine_small) CK(cudaStreamWaitEvent(s, L.join_ev[q], 0));
-  for (int q = 0; q < kClusterClasses; ++q)
-    if (R.class_units[q]) {  // their power loops are over by here
-      CK(gate.mark(s));
-      break;
-    }
   if (R.engine_sync) {
     // launched above, beside the cluster classes
   } else if (R.egraph && R.egraph_stream)
     CK(launch_power_direct(egrid, 2, R.egraph_stream, L.d_args, L.d_pc2, s));
   else if (R.egraph) CK(cudaGraphLaunch(eexec, s));
   else if (n_large > 0 && quantum >= 0)
-    CK(gate.launch(s, [&] { return launch_engine(args, grid, s); }));
+    CK(launch_engine(args, grid, s));
+  if (R.engine_sync || engine_coop || class_waits) CK(gate.entered(s, need));
   if (hold.owns_lock()) hold.unlock();
   CK(cudaEventRecord(L.e1, s));
   if (R.power) CK(cudaMemcpyAsync(&io.pc_out[0], L.d_pc, sizeof(PowCtl), cudaMemcpyDeviceToHost, s));
@@ -1210,7 +1237,8 @@ int engine_begin(mprgp_context *c, int k, int n, mprgp_problem *const *probs,
   R.cluster_quantum = cluster_quantum;
   R.power_launches = power_launches;
   R.active = true;
-  lane_start.issued(L.e_end);
+  if (k != 0) loop_run.issued_on_lane(L.e_end);
+  else CK(loop_run.issued(s));
   static const char *kRunNames[kLanes] = {"mprgp run", "mprgp lane small", "mprgp lane large",
                                           "mprgp lane power", "mprgp lane power",
                                           "mprgp lane power", "mprgp lane power"};

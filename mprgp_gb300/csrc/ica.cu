@@ -851,17 +851,20 @@ int mprgp_ica_solve(mprgp_context *ctx, int nv, int nnzb, const int *row_ptr, co
     a.out = (double *)(d + o_out);
     a.wait_ns = 5000000000LL;  // 5 s per barrier wait
     void *params[] = {&a};
-    e = cudaEventRecord(e0, s);
-    if (e == cudaSuccess && clustered) {
+    if (clustered) {
+      e = cudaEventRecord(e0, s);
       IcaClusterArgs ca;
       ca.a = a;
       ca.rows = (const IcaRow *)(d + o_rows);
-      e = cudaLaunchKernelEx(&ccfg, ica_cluster_kernel, ca);
-    } else if (e == cudaSuccess)
-      e = mprgp::gated_launch(s, [&] {
-        return cudaLaunchCooperativeKernel((const void *)ica_kernel, dim3(grid), dim3(kIcaThreads),
-                                           params, 0, s);
+      if (e == cudaSuccess) e = cudaLaunchKernelEx(&ccfg, ica_cluster_kernel, ca);
+    } else {
+      e = mprgp::gated_launch(s, nsm, grid, [&] {
+        const cudaError_t r = cudaEventRecord(e0, s);  // (behind the runs it waits for)
+        return r != cudaSuccess ? r
+                                : cudaLaunchCooperativeKernel((const void *)ica_kernel, dim3(grid),
+                                                              dim3(kIcaThreads), params, 0, s);
       });
+    }
     if (e == cudaSuccess) e = cudaEventRecord(e1, s);
   }
   IcaCtl ctl{};

@@ -314,7 +314,7 @@ extern "C" int mprgp_solve_noalloc(void *stream, int nv, int nnzb, const int *ro
   args.ctl = ctl;
   const int grid = std::max(1, std::min(nitems, dev->nsm * dev->bps));
   const auto t0 = std::chrono::steady_clock::now();
-  NCK(gated_launch(s, [&] { return launch_engine(args, grid, s); }));
+  NCK(gated_launch(s, dev->nsm, grid, [&] { return launch_engine(args, grid, s); }));
   InstState out;
   Ctl c1;
   NCK(cudaMemcpyAsync(&out, d_st, sizeof(out), cudaMemcpyDeviceToHost, s));

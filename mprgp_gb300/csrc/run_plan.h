@@ -26,6 +26,7 @@ struct PlanSettings {
   // The run may hold kernels whose CTAs wait for each other: a synchronous run
   // (lane 0), and nothing of the library beside it that they must not meet.
   bool alone = false;
+  bool compact = false;  // whole items only, no clusters: the fewest SMs a run can do with
   int quantum = 0, power_launches = 0, cluster_quantum = 0;
   bool power_waits = false;   // the tuning leaves the power method to the waiting forms
   bool engine_waits = false;  // ... and the other phases to the waiting engine
@@ -65,7 +66,7 @@ struct RunPlan {
 };
 
 template <typename Cap>
-SyncPlan sync_plan(const Cap &cap, int nsm, int units, int max_slots, int fp32) {
+SyncPlan sync_plan(const Cap &cap, int nsm, int units, int max_slots, int fp32, bool compact) {
   SyncPlan P;
   const int slice = max_slots * kSlice * (9 * (fp32 ? 4 : 8) + 4);
   auto bytes = [&](int q) {  // a CTA's slices, in few distinct sizes
@@ -86,7 +87,7 @@ SyncPlan sync_plan(const Cap &cap, int nsm, int units, int max_slots, int fp32) 
   // 425 vertices: 10.7 -> 7.7 us a phase, 6,720: 12.3 -> 9.3.  (Three quarters
   // of the SMs: clusters do not pack them further, and two CTAs on an SM cost
   // what the split gains: 9,464 vertices 13.2 us, 12.6 with whole rows.)
-  if (!fp32)
+  if (!fp32 && !compact)
     for (int q = 8; q >= 4; q /= 2)
       if (4 * units * q <= 3 * nsm && fits(q, 3)) return P;
   // Else the fewest CTAs an item whose slices fit shared memory, or twice as
@@ -94,7 +95,7 @@ SyncPlan sync_plan(const Cap &cap, int nsm, int units, int max_slots, int fp32) 
   // a phase with q = 1, 5.5 with 2, 4 or 8; 17,856 in FP64: 11.5 with q = 2,
   // 14.2 with 4, 18.3 with 8.
   int tried = 0;
-  for (int q = 1; q <= kThreads / kSlice && tried < 2; q *= 2) {
+  for (int q = 1; q <= (compact ? 1 : kThreads / kSlice) && tried < 2; q *= 2) {
     if (bytes(q) > kSyncStageBytes) continue;
     ++tried;
     if (fits(q, 1)) break;
@@ -118,14 +119,14 @@ inline SyncPlan persistent_plan(const PlanSettings &s, int units) {
 
 // The waiting engine's layout; grid == 0 when it does not apply.
 template <typename Cap>
-SyncPlan engine_plan(const Cap &cap, int nsm, int units, int max_slots, bool fp64, bool beside) {
+SyncPlan engine_plan(const Cap &cap, int nsm, int units, int max_slots, bool split, bool beside) {
   SyncPlan P;
   // FP64 items: eight or four CTAs of three threads a row, with their matrix
   // slices in shared memory, while three quarters of the SMs hold them (the
   // rule of sync_plan); else two CTAs while each has an SM of its own: an
   // item's eight row warps take 135 FP64 FMAs each, two warps a scheduler in
   // one CTA (17,856 vertices 16.6 -> 16.1 ms with two).
-  if (fp64)
+  if (split)
     for (int q = 8; q >= 4; q /= 2) {
       const long long bytes = (long long)max_slots * kSlice * (9 * 8 + 4) * (kThreads / kSlice / q);
       const long long smem = (bytes + 4095) / 4096 * 4096;
@@ -136,7 +137,7 @@ SyncPlan engine_plan(const Cap &cap, int nsm, int units, int max_slots, bool fp6
       P.grid = q * units;
       return P;
     }
-  if (fp64 && 2 * units <= std::min(nsm, cap.engine(2, 0))) {
+  if (split && 2 * units <= std::min(nsm, cap.engine(2, 0))) {
     P.q = 2;
     P.grid = 2 * units;
     return P;
@@ -185,7 +186,7 @@ RunPlan plan_run(const std::vector<PlanInst> &insts, const PlanSettings &s, cons
     }
   }
   if (all.one()) {
-    R.power = sync_plan(cap, s.nsm, all.units, all.slots, all.fp32 ? 1 : 0);
+    R.power = sync_plan(cap, s.nsm, all.units, all.slots, all.fp32 ? 1 : 0, s.compact);
     R.small_in_plan = R.power.grid > 0;
   }
   if (large.one() && R.power.grid == 0) R.power = persistent_plan(s, large.units);
@@ -193,6 +194,7 @@ RunPlan plan_run(const std::vector<PlanInst> &insts, const PlanSettings &s, cons
   R.power_count = R.small_in_plan ? all : large;
   for (int q = 0; q < kClusterClasses; ++q) {
     if (R.small_in_plan || !cl[q].one() || !cl_fits[q] || !s.power_cluster_ok[q]) continue;
+    if (large.n > 0 && !R.power_sync) continue;  // not beside the large ones' launch loop
     R.class_n[q] = cl[q].n;
     R.class_units[q] = cl[q].n << q;
     R.class_fp32[q] = cl[q].fp32 > 0;
@@ -207,18 +209,23 @@ RunPlan plan_run(const std::vector<PlanInst> &insts, const PlanSettings &s, cons
   PlanCount eng;
   for (const PlanInst &p : insts)
     if (n_large == 0 || p.large) eng.add(p);
-  if (n_large == 0 && s.quantum == 0 && s.cluster_quantum == 0 && eng.fp32 == 0 &&
+  if (n_large == 0 && !s.compact && s.quantum == 0 && s.cluster_quantum == 0 && eng.fp32 == 0 &&
       (in_power == 0 || R.small_in_plan)) {
     R.engine = engine_plan(cap, s.nsm, eng.units, eng.slots, true, false);
     if (R.engine.q < 2) R.engine = SyncPlan();
     R.engine_small = R.engine.grid > 0;
   } else if (n_large > 0) {
-    R.engine = engine_plan(cap, s.nsm, eng.units, eng.slots, eng.fp32 == 0, n > n_large);
+    R.engine = engine_plan(cap, s.nsm, eng.units, eng.slots, eng.fp32 == 0 && !s.compact,
+                           n > n_large);
   }
   R.engine_sync = R.engine.grid > 0;
   R.engine_count = eng;
   return R;
 }
+
+// CTAs that the run's waiting launches hold at once, at most (they follow each
+// other; the clusters' power loops wait for nothing outside their cluster).
+inline int plan_ctas(const RunPlan &R) { return std::max(R.power.grid, R.engine.grid); }
 
 // A run's error words: 0 for its waiting launches over the large instances (and
 // whatever joins them), 1 + q for the power loops of cluster class q.  The word

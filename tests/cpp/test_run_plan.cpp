@@ -74,6 +74,9 @@ int main() {
   EXPECT(R.power_sync && !R.small_in_plan && R.power_count.n == 1);
   EXPECT(R.class_units[1] == 2 && R.class_units[3] == 8 && R.class_n[1] == 1 && R.class_fp32[1]);
   EXPECT(R.engine_sync && R.engine_count.n == 1);
+  // items past the persistent loop: the launch loop, and no waiting clusters beside
+  R = plan_run({inst(1360, true), inst(2, true), inst(5, true)}, settings(true), Cap());
+  EXPECT(!R.power_sync && !R.class_units[1] && !R.class_units[3] && R.engine_sync);
   // a tuning with the launch loops keeps a small FP64 instance's power method in
   // the cluster solver; past it, the waiting engine takes it as before
   PlanSettings loops = settings(true);
@@ -82,6 +85,18 @@ int main() {
   EXPECT(!waits(plan_run({inst(2, false), inst(3, false, false)}, loops, Cap())));
   R = plan_run({inst(2, false, false)}, loops, Cap());
   EXPECT(R.engine_small && !R.power_sync);
+  // compact: whole items, no clusters, and no more CTAs than items
+  PlanSettings compact = settings(true);
+  compact.compact = true;
+  for (const auto &r : runs) {
+    R = plan_run(r, compact, Cap());
+    int items = 0;
+    for (const PlanInst &p : r) items += p.items;
+    EXPECT(R.power.q <= 1 && R.engine.q <= 1 && R.power.comps == 1 && plan_ctas(R) <= items);
+    EXPECT(!R.engine_small);
+  }
+  R = plan_run({inst(27, false)}, compact, Cap());
+  EXPECT(R.power_sync && R.power.grid == 27 && R.engine_sync && R.engine.grid == 27);
   // an error concerns the instances of the launch that reports it
   {
     const std::vector<PlanInst> r = {inst(900, true), inst(2, true), inst(5, true),
