@@ -23,6 +23,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/mprgp_gpu.h"
+#include "fem_rule.h"
 
 namespace mprgp {
 void set_last_error(const char *what);
@@ -37,6 +38,7 @@ struct mprgp_fem {
   int *row_ptr = nullptr, *cols = nullptr;
   int *vt_ptr = nullptr, *vt = nullptr;  // incident (tet << 2 | local corner) per vertex
   int max_len = 0;                       // blocks in a row, at most
+  int nsm = 0, sm_smem = 0;              // SMs, and bytes of shared memory in each
   double *geom = nullptr;                // kGeom per tet: V, grad N_0..3, padding
   double *X = nullptr;                   // rest shape
   double *mass = nullptr, *KX = nullptr;
@@ -46,6 +48,11 @@ struct mprgp_fem {
 };
 
 namespace {
+
+using mprgp::kRowPad;
+using mprgp::kRowSmemMax;
+using mprgp::row_smem;
+using mprgp::rows_in_smem;
 
 int fail(int code, const char *what) {
   mprgp::set_last_error(what);
@@ -126,11 +133,6 @@ __device__ __forceinline__ int find_block(const int *__restrict__ cols, int r0, 
 // two moduli applied at the end, upper blocks mirrored: 0.77 ms), but they
 // round differently, and on a small stiff body a last bit of A moves the
 // solution by as much as the solver's tolerance lets it.
-constexpr int kRowPad = 33;
-constexpr int kRowSmemMax = 220 * 1024;  // rows of up to 89 blocks
-__host__ __device__ constexpr int row_smem(int max_len) {
-  return kRowPad * max_len * (9 * 8 + 4);
-}
 __global__ void __launch_bounds__(32)
     assemble_smem_kernel(int nv, int max_len, const int4 *__restrict__ tets,
                          const double *__restrict__ geom, const int *__restrict__ row_ptr,
@@ -194,7 +196,7 @@ __global__ void __launch_bounds__(32)
 }
 
 // The same with the rows in global memory, one thread per vertex, for a mesh
-// with a row too wide for shared memory.
+// whose longest row leaves too few warps in shared memory (fem_rule.h).
 __global__ void assemble_rows_kernel(int nv, const int *__restrict__ tets,
                                      const double *__restrict__ geom,
                                      const int *__restrict__ row_ptr, const int *__restrict__ cols,
@@ -325,6 +327,14 @@ int mprgp_fem_create(mprgp_context *ctx, int nv, int ntet, const int *tets, cons
   f->ntet = ntet;
   f->nnzb = row_ptr[nv];
   f->max_len = max_len;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&f->nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&f->sm_smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) !=
+          cudaSuccess) {
+    delete f;
+    return fail(MPRGP_CUDA_ERROR, "fem_create: device attributes");
+  }
   f->lam = poisson * young / ((1.0 + poisson) * (1.0 - 2.0 * poisson));
   f->mu = young / (2.0 * (1.0 + poisson));
   f->rho = rho;
@@ -381,8 +391,8 @@ int mprgp_fem_assemble(mprgp_fem *f, double h, const double gravity[3], const do
   cudaStream_t s = f->stream;
   const double g[3] = {gravity ? gravity[0] : 0.0, gravity ? gravity[1] : 0.0,
                        gravity ? gravity[2] : 0.0};
-  const int smem = f->max_len < 1024 ? row_smem(f->max_len) : kRowSmemMax + 1;
-  if (smem <= kRowSmemMax) {
+  if (rows_in_smem(f->max_len, f->nv, f->nsm, f->sm_smem)) {
+    const int smem = row_smem(f->max_len);
     FK(cudaFuncSetAttribute(assemble_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                             kRowSmemMax));
     assemble_smem_kernel<<<(f->nv + 31) / 32, 32, smem, s>>>(
