@@ -3653,7 +3653,7 @@ __device__ __noinline__ bool wait_count(const unsigned int *count, unsigned int 
                                         long long wait_ns) {
   long long since = 0;
   int spins = 0;
-  while (ld_acquire(count) < target) {
+  while (!count_reached(ld_acquire(count), target)) {
     const long long now = gtimer();
     if (since == 0) since = now;
     if (now - since > wait_ns) {
@@ -3733,7 +3733,7 @@ __global__ void __launch_bounds__(kStepThreads, kMinBlocks)
     }
     if (threadIdx.x == kThreads && pend) {  // every owned item's instance is done with phase t - 1
       for (int o = 0; o < nown; ++o)
-        if ((pend >> o) & 1u && !wait_count(phase_count(sD[o]), (unsigned int)(t * sD[o].nitems),
+        if ((pend >> o) & 1u && !wait_count(phase_count(sD[o]), phase_target(t - 1, sD[o].nitems),
                                             args.ctl, args.wait_ns))
           sFail = 1;
     }
@@ -4124,7 +4124,7 @@ __global__ void __launch_bounds__(kThr, 1) engine_sync_kernel(EngineSyncArgs arg
     if (threadIdx.x == 0) {
       for (int o = 0; o < nown; ++o)
         if (sSlot[o] == o && sS[o].phase != PH_DONE &&
-            !wait_count(sD[o].cnt, (unsigned int)((t + 1) * sD[o].nitems * q), args.ctl, args.wait_ns))
+            !wait_count(sD[o].cnt, phase_target(t, sD[o].nitems * q), args.ctl, args.wait_ns))
           sFail = 1;
       if (gtimer() - t_start > args.total_ns) {
         atomicCAS(&args.ctl->err, 0, -4);  // MPRGP_TIMEOUT

@@ -52,4 +52,15 @@ __host__ __device__ inline bool split_shape_ok(int q, int units, int rows_thread
          block == rows_threads;
 }
 
+// Whether an instance's phase counter has reached `target`.  Both count modulo
+// 2^32 -- items times phases exceeds it in a long solve -- and never differ by
+// more than the items of one phase, so the sign of the difference tells.
+__host__ __device__ inline bool count_reached(unsigned int count, unsigned int target) {
+  return (int)(count - target) >= 0;
+}
+// The counter at the end of phase `phase` (0, 1, ...) when each counts `per`.
+__host__ __device__ inline unsigned int phase_target(int phase, int per) {
+  return ((unsigned int)phase + 1u) * (unsigned int)per;
+}
+
 }  // namespace mprgp

@@ -1,6 +1,7 @@
 // The launch shape of the kernels whose units take a cluster (split_launch.h):
 // what is asked for, and what a CTA accepts.
 #include <cstdio>
+#include <initializer_list>
 
 #include "split_launch.h"
 
@@ -41,6 +42,19 @@ int main() {
     EXPECT(!split_shape_ok(q, 6, 128, q, 6 * q, 160));
   }
   EXPECT(!split_shape_ok(0, 6, 128, 0, 0, 128));
+  // a phase counter before, at and past its target, also where it wraps
+  for (int per : {1, 2, 16, 70, 1360, 4096})
+    for (long long phase : {0LL, 1LL, 1002LL, (1LL << 31) / per, (1LL << 32) / per - 1,
+                            (1LL << 32) / per, (1LL << 32) / per + 1, 2147483646LL}) {
+      if (phase > 2147483646LL) continue;
+      const unsigned int target = phase_target((int)phase, per);
+      EXPECT(target == (unsigned int)((unsigned long long)(phase + 1) * (unsigned long long)per));
+      for (int missing = 0; missing <= per; missing += per > 8 ? per / 8 : 1)
+        EXPECT(count_reached(target - (unsigned int)missing, target) == (missing == 0));
+      // a peer that is a phase ahead has counted some items more
+      for (int more = 1; more <= per; more += per > 8 ? per / 8 : 1)
+        EXPECT(count_reached(target + (unsigned int)more, target));
+    }
   std::printf(fails ? "FAILED\n" : "OK\n");
   return fails != 0;
 }
