@@ -1094,7 +1094,7 @@ int engine_begin(mprgp_context *c, int k, int n, mprgp_problem *const *probs,
   if (quantum > 0) maxp = std::min<long long>(maxp, quantum);
   args.max_phases = (int)std::min<long long>(maxp, INT_MAX);
   args.wait_ns = (long long)(wait_s * 1e9);
-  args.total_ns = (long long)(std::max(60.0, 20.0 * wait_s) * 1e9);
+  args.total_ns = launch_limit_ns(R.engine_small, wait_s);
   const bool stage = c->stage && c->bps_stage > 0;
   args.stage_bytes = stage ? kStageBytes : 0;
   args.ctl = L.ctl;

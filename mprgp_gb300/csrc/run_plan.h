@@ -5,6 +5,7 @@
 // engine(q, smem)).
 #pragma once
 #include <algorithm>
+#include <climits>
 #include <vector>
 
 #include "engine.h"
@@ -237,6 +238,13 @@ inline int error_word(const RunPlan &R, const PlanInst &p) {
   if (!p.in_power) return -1;
   if (R.power_sync && R.small_in_plan) return 0;
   return R.class_units[p.cls] > 0 ? 1 + p.cls : -1;
+}
+
+// Bound on the time of a whole engine launch: 20 waits, a minute at least.
+// Small instances have none: in the cluster solver, whose phases they take here,
+// only their iterations bound them.
+inline long long launch_limit_ns(bool small, double wait_s) {
+  return small ? LLONG_MAX : (long long)(std::max(60.0, 20.0 * wait_s) * 1e9);
 }
 
 }  // namespace mprgp

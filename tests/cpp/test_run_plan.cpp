@@ -119,6 +119,9 @@ int main() {
     R = plan_run(w, settings(false), Cap());
     EXPECT(error_word(R, w[0]) == -1 && error_word(R, w[1]) == -1);
   }
+  // the waiting engine ends a large instance's launch in time, a small one's never
+  EXPECT(launch_limit_ns(false, 5.0) == 100000000000LL && launch_limit_ns(false, 1e-9) == 60000000000LL);
+  EXPECT(launch_limit_ns(true, 5.0) == LLONG_MAX);
   // unit counts and grids agree
   for (const auto &r : runs) {
     R = plan_run(r, settings(true), Cap());
