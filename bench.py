@@ -185,6 +185,32 @@ def measured_peaks():
     return 6800.0, "fallback"
 
 
+def power_kernel_of(form, launches, nv):
+    """(kernel, label) of the power method of one solve: the loop the tuning
+    names, or the resident launch that takes its place where the items fit, which
+    the few kernels launched per solve show."""
+    if form in ("step", "persistent") and launches < 64:
+        if nv <= 152 * 256:  # up to an item an SM: the slices fit shared memory
+            return "power_sync_kernel", "mprgp::power_sync_kernel (one launch, slices in shared memory)"
+        return "power_persistent_kernel", "mprgp::power_persistent_kernel (one launch, resident CTAs)"
+    if form == "step":
+        return "power_step_kernel", "mprgp::power_step_kernel (power-step loop, CUDA graph)"
+    return "power_kernel", "mprgp::phase_kernel (power phases, CUDA-graph loop)"
+
+
+def engine_kernel_of(tuning, nv, mixed):
+    """The kernel of the MPRGP phases of one solve."""
+    config = (tuning or {}).get("config") or {}
+    bits = (tuning or {}).get("explicit_tuning_bits", 0)
+    if nv <= 16 * 256 and mixed:
+        return "cluster_kernel"
+    if config.get("engine") == "graph" or bits & 16:
+        return "phase_kernel"
+    if config.get("ctas_per_sm") or config.get("stage") or config.get("power") == "engine" or bits & 3:
+        return "engine_kernel"
+    return "engine_sync_kernel"
+
+
 def committed_traffic(name, form, kernel="engine_kernel"):
     """Per-launch DRAM bytes (read + write) of a kernel from the committed ncu
     summary profiles/traffic.json, keyed "<config>:<form>:<kernel>"."""
@@ -400,13 +426,8 @@ def run_gb300(args):
     if power_ms > 0:  # the power loop ran as its own kernel
         pow_launch_ms = power_ms / max(1, passes)
         achieved = pass_bytes / (pow_launch_ms / 1e3) / 1e9
-        form = power_form(tuning)
-        kname = {"step": "power_step_kernel", "persistent": "power_persistent_kernel"}.get(
-            form, "power_kernel")
+        kname, dominant = power_kernel_of(power_form(tuning), launches / max(1, len(stats)), qp.nv)
         traffic = committed_traffic(args.config, args.form, kname)
-        dominant = {"step": "mprgp::power_step_kernel (power-step loop, CUDA graph)",
-                    "persistent": "mprgp::power_persistent_kernel (one cooperative launch)"}.get(
-            form, "mprgp::phase_kernel (power phases, CUDA-graph loop)")
         eng_ms = (solver1 - solver0) - power_ms
     else:  # the tuning put the power phases into the persistent engine
         pow_launch_ms = (solver1 - solver0) / max(1, len(stats))
@@ -442,12 +463,13 @@ def run_gb300(args):
                      "share_of_solve": round(power_ms / max(1e-9, solver1 - solver0), 3)
                      if power_ms > 0 else 1.0,
                      "bytes_rule": "per matrix pass: nnzb*(9*s+2) + (nv+1)*4 + 2*n*s, s = 8 (FP64) or 4 (FP32)"},
-        "roofline_engine": {"kernel": "mprgp::engine_kernel (MPRGP phases)",
+        "roofline_engine": {"kernel": f"mprgp::{engine_kernel_of(tuning, qp.nv, mixed)} (MPRGP phases)",
                             "achieved": None if eng_achieved is None else round(eng_achieved, 2),
                             "frac": None if eng_achieved is None else round(eng_achieved / peak, 4),
                             "bytes": int(eng_bytes + eng_vec), "bytes_matrix": int(eng_bytes),
                             "bytes_vectors": int(eng_vec), "ms": round(eng_ms, 3),
-                            "traffic": committed_traffic(args.config, args.form, "engine_kernel"),
+                            "traffic": committed_traffic(args.config, args.form,
+                                                         engine_kernel_of(tuning, qp.nv, mixed)),
                             "note": "matrix passes plus the estimated vector traffic (VEC_K); "
                                     "the MPRGP phases are FP64-issue bound (ncu)"},
         "gpu_launches": int(launches),
@@ -712,7 +734,8 @@ def run_batch(args):
         "solve": {"iterations_max": max(s.iterations for s in stats),
                   "iterations_mean": round(statistics.mean(s.iterations for s in stats), 1),
                   "phases": max(s.phases for s in stats)},
-        "roofline": {"bound": "hbm", "kernel": "mprgp::engine_kernel", "achieved": round(achieved, 2),
+        "roofline": {"bound": "hbm", "kernel": "all solver kernels of the batch",
+                     "achieved": round(achieved, 2),
                      "peak": peak, "unit": "GB/s", "frac": round(achieved / peak, 4),
                      "peak_source": peak_kind, "traffic": None, "bytes_per_launch": alg,
                      "launch_ms": round(dev_ms, 3)},
@@ -869,8 +892,8 @@ def run_timesteps(args):
                        "p99": round(float(np.percentile(times, 99)), 3)},
         "per_timestep": records,
         "roofline": {"bound": "hbm",
-                     "kernel": "solver kernels of the timestep (engine_kernel; the power loop "
-                               "on the first step)",
+                     "kernel": f"solver kernels of the timestep ({engine_kernel_of(tuning, qp.nv, mixed)}; the "
+                               "power loop on the first step)",
                      "achieved": round(achieved, 2), "peak": peak, "unit": "GB/s",
                      "frac": round(achieved / peak, 4), "peak_source": peak_kind,
                      "traffic": None,

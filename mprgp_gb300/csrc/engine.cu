@@ -3060,7 +3060,7 @@ __global__ void __launch_bounds__(32)
 // all rows, a square root and a reciprocal), not bytes: as graph launches a
 // 70-item phase took 17.1 us and the cluster solver 9.7 (1,760 vertices,
 // mixed) to 16.7 us (425 vertices, FP64: eight row warps' 1,080 FP64 FMAs on
-// one SM alone take 8.6).  This loop takes 13.7, 4.8 and 10.4 us.  Here:
+// one SM alone take 8.6).  This loop takes 11.5, 4.8 and 6.1 us.  Here:
 //  * A unit is one item's rows, in one CTA or split over a cluster of q CTAs,
 //    so that few items still use many SMs' FP64 units.  A row belongs to one
 //    thread for the whole loop: its iterate, the previous one and its matrix
