@@ -66,7 +66,8 @@ using namespace mprgp;
 
 namespace mprgp {
 CoopGate &coop_gate(int device) {
-  static CoopGate gates[64];
+  // (never destroyed: a context owned by a static object may go after this file's)
+  static CoopGate *const gates = new CoopGate[64];
   return gates[device & 63];
 }
 }  // namespace mprgp
