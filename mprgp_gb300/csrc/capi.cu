@@ -741,7 +741,8 @@ int lane_reserve(mprgp_context *c, Lane &L, int n, int items) {
   return MPRGP_OK;
 }
 
-// The same for the units of the power sync loop.
+// The same for the units of the waiting loops, before the run asks the gate:
+// giving back pinned memory waits for the device.
 int lane_reserve_units(mprgp_context *c, Lane &L, int units) {
   if (units <= L.ucap) return MPRGP_OK;
   const int ucap = std::max(1024, std::max(units, 2 * L.ucap));
@@ -966,6 +967,14 @@ int engine_begin(mprgp_context *c, int k, int n, mprgp_problem *const *probs,
   unsigned int in_power = 0;  // large instances in a power phase
   for (int i = 0; i < n; ++i)
     if (R.pos[i] < n_large && engine_in_power(probs[i])) ++in_power;
+  std::vector<PlanInst> insts(n);
+  for (int i = 0; i < n; ++i)
+    insts[i] = {R.pos[i] < n_large, cls[i], nitems_of(probs[i]->nv), probs[i]->max_len,
+                desc[R.pos[i]].prec == PREC_MIXED, engine_in_power(probs[i]) != 0};
+  if (k == 0) {
+    rc = lane_reserve_units(c, L, plan_units_at_most(insts));
+    if (rc) return rc;
+  }
   // A synchronous run's kernels may wait for their peers when the gate lets them
   // in (coop_gate.h); it is held until they are issued.  A lane's run, and a
   // synchronous one with launch loops in their place, begins behind those issued
@@ -985,10 +994,6 @@ int engine_begin(mprgp_context *c, int k, int n, mprgp_problem *const *probs,
   ps.persistent4 = c->power_persistent != 0;
   ps.persistent_per_sm = c->bps_power_pp;
   for (int q = 0; q < kClusterClasses; ++q) ps.power_cluster_ok[q] = c->power_cluster_ok[q] != 0;
-  std::vector<PlanInst> insts(n);
-  for (int i = 0; i < n; ++i)
-    insts[i] = {R.pos[i] < n_large, cls[i], nitems_of(probs[i]->nv), probs[i]->max_len,
-                desc[R.pos[i]].prec == PREC_MIXED, engine_in_power(probs[i]) != 0};
   // What the run waits for its peers in: its own forms, or whole items without
   // clusters.  (The large instances' phases without the waiting engine: the
   // cooperative engine, which waits too, or a graph loop; a power method in launch
@@ -1030,14 +1035,7 @@ int engine_begin(mprgp_context *c, int k, int n, mprgp_problem *const *probs,
   for (int i = 0; i < n; ++i) R.err_word[i] = error_word(plan, insts[i]);
   int nunits = 0, class_unit[kClusterClasses], engine_unit = 0;
   {
-    int want = R.power_sync ? plan.power_count.units : 0;
-    for (int q = 0; q < kClusterClasses; ++q) {
-      R.class_units[q] = plan.class_units[q];
-      want += R.class_units[q];
-    }
-    want += plan.engine.grid > 0 ? plan.engine_count.units : 0;
-    rc = lane_reserve_units(c, L, want);
-    if (rc) return rc;
+    for (int q = 0; q < kClusterClasses; ++q) R.class_units[q] = plan.class_units[q];
     if (R.power_sync)
       for (int i = 0; i < n; ++i) {
         if (!insts[i].in_power || !(insts[i].large || plan.small_in_plan)) continue;

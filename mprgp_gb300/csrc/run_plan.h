@@ -228,6 +228,14 @@ RunPlan plan_run(const std::vector<PlanInst> &insts, const PlanSettings &s, cons
 // other; the clusters' power loops wait for nothing outside their cluster).
 inline int plan_ctas(const RunPlan &R) { return std::max(R.power.grid, R.engine.grid); }
 
+// Entries of the unit list that any plan of these instances can need: every item
+// once for the power method and once for the waiting engine, or a cluster's CTAs.
+inline int plan_units_at_most(const std::vector<PlanInst> &insts) {
+  int n = 0;
+  for (const PlanInst &p : insts) n += p.items + (p.large ? p.items : std::max(p.items, 1 << p.cls));
+  return n;
+}
+
 // A run's error words: 0 for its waiting launches over the large instances (and
 // whatever joins them), 1 + q for the power loops of cluster class q.  The word
 // of the launch that an instance took part in, or -1: no launch that can give up

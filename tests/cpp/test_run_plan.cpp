@@ -124,6 +124,13 @@ int main() {
   EXPECT(launch_limit_ns(true, 5.0) == LLONG_MAX);
   // unit counts and grids agree
   for (const auto &r : runs) {
+    for (bool c : {false, true}) {
+      compact.compact = c;
+      R = plan_run(r, compact, Cap());
+      int units = (R.power_sync ? R.power_count.units : 0) + (R.engine_sync ? R.engine_count.units : 0);
+      for (int u : R.class_units) units += u;
+      EXPECT(units <= plan_units_at_most(r));
+    }
     R = plan_run(r, settings(true), Cap());
     if (R.power_sync && R.power.q > 0) EXPECT(R.power.grid == R.power_count.units * R.power.q);
     if (R.engine_sync && R.engine.q > 1) EXPECT(R.engine.grid == R.engine_count.units * R.engine.q);
